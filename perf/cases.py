@@ -218,6 +218,7 @@ def prepare(case: dict, seed: int):
         w = 0.98 + 0.04 * torch.rand(s["magSf"].shape[0], dtype=torch.float64, device="cuda", generator=s["generator"])
         st["Sf"] = s["Sf"] * w[:, None]
         st["magSf"] = s["magSf"] * w
+        st["n_faces"] = int(w.shape[0])
         return st
     st["mesh"] = _mesh(s)
     st["psi"] = torch.zeros_like(s["source"])
@@ -231,6 +232,15 @@ def prepare(case: dict, seed: int):
     return st
 
 
+def _end_to_end(arrays: list, size: int) -> np.ndarray:
+    out = np.full(size, -1, np.int32)
+    at = 0
+    for a in arrays:
+        out[at:at + a.shape[0]] = a
+        at += a.shape[0]
+    return out
+
+
 def run(st):
     kind = st["kind"]
     if kind == "batch":
@@ -241,7 +251,11 @@ def run(st):
     if kind == "mesh":
         mesh = _mesh(st)
         steps = [mesh.step(i) for i in range(mesh.n_levels)]
-        return [a for s in steps for a in (s["restrict"], s["face_restrict"], s["lower"], s["upper"])]
+        # every level's maps and addressing end to end; the levels' sizes depend on the areas, so the
+        # arrays are as long as they can get
+        return [_end_to_end([s[k] for s in steps], size)
+                for k, size in (("restrict", 3 * st["n"]), ("face_restrict", 3 * st["n_faces"]),
+                                ("lower", 3 * st["n_faces"]), ("upper", 3 * st["n_faces"]))]
     if kind == "smooth":
         st["psi"].copy_(st["psi0"])
         st["matrix"].smooth(0, st["psi"], st["source"], st["sweeps"])
