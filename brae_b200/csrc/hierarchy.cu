@@ -154,86 +154,161 @@ __global__ void kSeedFrontier(int n, const int* __restrict__ ctr, int* __restric
     if (c < n && ctr[c] == 0) frontier[atomicAdd(size, 1)] = c;
 }
 
-__global__ void kPairRound(int n, int fwd, const int* __restrict__ frontier, int fsize,
-                           const int* __restrict__ rowStart, const int* __restrict__ col,
-                           const int* __restrict__ entFace, const double* __restrict__ w,
-                           int* __restrict__ st, int* __restrict__ partner, int* __restrict__ target,
-                           int* __restrict__ ctr, int* __restrict__ next, int* nextSize)
+// A frontier's rounds in ONE cooperative launch: the rounds are separated by a grid-wide barrier on the
+// device, where one launch per round cost the host a size read-back, two copies and a synchronisation each
+// (25-40 us a round; a 260 k-cell box takes some 4,000 rounds over its levels). Every wait is bounded.
+struct FrontierLoop
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= fsize) return;
-    const int c = frontier[t];
-    const int r = rankOf(c, n, fwd);
-    const int rb = rowStart[c];
-    const int re = rowStart[c + 1];
-    if (st[c] != ST_TAKEN)
+    int size[3];       // the frontier's size by round modulo 3: this round's, the next one's, the one after
+    unsigned arrived;  // blocks that have reached a barrier, over all rounds
+    int resolved;      // cells taken off the frontier, and the rounds it took
+    int rounds;
+    int err;           // a barrier gave up
+};
+
+// all blocks of the launch (all resident); false when the wait gave up
+__device__ bool frontierBarrier(FrontierLoop* F, unsigned& target)
+{
+    __shared__ int ok;
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0)
     {
-        // the first face of maximum weight, in cellFaces order, whose other cell is unmatched
-        int best = -1;
-        double bestW = -kGreatAgg;
-        for (int e = rb; e < re; ++e)
-        {
-            const int nb = col[e];
-            const bool avail = rankOf(nb, n, fwd) > r && st[nb] != ST_TAKEN;
-            const double we = w[entFace[e]];
-            if (avail && we > bestW)
+        ok = 1;
+        __threadfence();
+        atomicAdd(&F->arrived, 1u);
+        long long it = 0;
+        while (ldAcquire(&F->arrived) < target)
+            if (++it > k::kSpinLimit || ((it & 4095) == 0 && *reinterpret_cast<volatile int*>(&F->err)))
             {
-                best = e;
-                bestW = we;
+                atomicExch(&F->err, 1);
+                ok = 0;
+                break;
             }
-        }
-        if (best >= 0)
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// visit(cell, lane, round, next, nextSize) for every cell of every frontier, by a warp each (kWarp) or a thread
+// each (lane 0); frontiers in fa and fb by turns, the first in fa. What another block wrote in an earlier round
+// is read past L1 (__ldcg) by the visits.
+template <bool kWarp, class Visit>
+__device__ void frontierRounds(int* fa, int* fb, FrontierLoop* F, Visit&& visit)
+{
+    unsigned target = 0;
+    int resolved = 0, round = 0;
+    constexpr int kPer = kWarp ? 32 : 1;
+    const int t0 = (blockIdx.x * blockDim.x + threadIdx.x) / kPer, stride = gridDim.x * blockDim.x / kPer;
+    for (;; ++round)
+    {
+        const int fsize = __ldcg(&F->size[round % 3]);
+        if (fsize == 0) break;
+        const int* cur = (round & 1) ? fb : fa;
+        int* next = (round & 1) ? fa : fb;
+        // (every block has read this slot's last use, two rounds back, before the barrier in between)
+        if (blockIdx.x == 0 && threadIdx.x == 0) F->size[(round + 2) % 3] = 0;
+        for (int t = t0; t < fsize; t += stride)
+            visit(__ldcg(cur + t), kWarp ? static_cast<int>(threadIdx.x & 31) : 0, round, next, &F->size[(round + 1) % 3]);
+        resolved += fsize;
+        if (!frontierBarrier(F, target)) return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        F->resolved = resolved;
+        F->rounds = round;
+    }
+}
+
+// A warp per cell: a cell's decision and its releases are a few hundred loads and counter updates on the
+// coarse levels (20 entries a row, each with its neighbour's row), which one thread would wait out one after
+// another.
+__global__ void __launch_bounds__(TPB) kPairLoop(int n, int fwd, int* fa, int* fb, const int* __restrict__ rowStart,
+                                                 const int* __restrict__ col, const int* __restrict__ entFace,
+                                                 const double* __restrict__ w, int* st, int* partner, int* target,
+                                                 int* ctr, FrontierLoop* F)
+{
+    frontierRounds<true>(fa, fb, F, [&](int c, int lane, int, int* next, int* nextSize) {
+        const int r = rankOf(c, n, fwd);
+        const int rb = rowStart[c];
+        const int re = rowStart[c + 1];
+        const bool taken = __ldcg(st + c) == ST_TAKEN;
+        if (!taken)
         {
-            const int nb = col[best];
-            partner[c] = nb;
-            partner[nb] = c;
-            st[nb] = ST_TAKEN;
-            st[c] = ST_CREATOR;
-        }
-        else
-        {
-            // no unmatched neighbour: join the cluster across the heaviest face (AGG:239-257)
-            int cbest = -1;
-            double cw = -kGreatAgg;
-            for (int e = rb; e < re; ++e)
+            // the first face of maximum weight, in cellFaces order, whose other cell is unmatched (best), and
+            // among all (the cluster to join across the heaviest face if there is none, AGG:239-257)
+            int best = -1, any = -1;
+            double bestW = -kGreatAgg, anyW = -kGreatAgg;
+            for (int e = rb + lane; e < re; e += 32)
             {
+                const int nb = col[e];
                 const double we = w[entFace[e]];
-                if (we > cw)
+                if (we > anyW)
                 {
-                    cbest = e;
-                    cw = we;
+                    any = e;
+                    anyW = we;
+                }
+                if (we > bestW && rankOf(nb, n, fwd) > r && __ldcg(st + nb) != ST_TAKEN)
+                {
+                    best = e;
+                    bestW = we;
                 }
             }
-            if (cbest >= 0)
+            // the larger weight, of equal ones the earlier entry: a lane's own is its first maximum already
+            for (int o = 16; o > 0; o >>= 1)
             {
-                target[c] = col[cbest];
-                st[c] = ST_JOINER;
+                const int be = __shfl_xor_sync(0xffffffffu, best, o), ae = __shfl_xor_sync(0xffffffffu, any, o);
+                const double bw = __shfl_xor_sync(0xffffffffu, bestW, o), aw = __shfl_xor_sync(0xffffffffu, anyW, o);
+                if (be >= 0 && (best < 0 || bw > bestW || (bw == bestW && be < best)))
+                {
+                    best = be;
+                    bestW = bw;
+                }
+                if (ae >= 0 && (any < 0 || aw > anyW || (aw == anyW && ae < any)))
+                {
+                    any = ae;
+                    anyW = aw;
+                }
             }
-            else
+            if (lane == 0)
             {
-                st[c] = ST_LONE;
+                if (best >= 0)
+                {
+                    const int nb = col[best];
+                    partner[c] = nb;
+                    partner[nb] = c;
+                    st[nb] = ST_TAKEN;
+                    st[c] = ST_CREATOR;
+                }
+                else if (any >= 0)
+                {
+                    target[c] = col[any];
+                    st[c] = ST_JOINER;
+                }
+                else
+                {
+                    st[c] = ST_LONE;
+                }
             }
         }
-    }
-    // release the cells that counted c
-    for (int e = rb; e < re; ++e)
-    {
-        const int m = col[e];
-        const int rm = rankOf(m, n, fwd);
-        if (rm > r)
+        // release the cells that counted c
+        for (int e = rb + lane; e < re; e += 32)
         {
-            if (atomicSub(&ctr[m], 1) == 1) next[atomicAdd(nextSize, 1)] = m;
+            const int m = col[e];
+            if (rankOf(m, n, fwd) > r && atomicSub(&ctr[m], 1) == 1) next[atomicAdd(nextSize, 1)] = m;
         }
-        for (int e2 = rowStart[m]; e2 < rowStart[m + 1]; ++e2)
+        for (int e = rb; e < re; ++e)
         {
-            const int d = col[e2];
-            const int rd = rankOf(d, n, fwd);
-            if (rd > r && rd < rm)
+            const int m = col[e];
+            const int rm = rankOf(m, n, fwd);
+            for (int e2 = rowStart[m] + lane; e2 < rowStart[m + 1]; e2 += 32)
             {
-                if (atomicSub(&ctr[d], 1) == 1) next[atomicAdd(nextSize, 1)] = d;
+                const int d = col[e2];
+                const int rd = rankOf(d, n, fwd);
+                if (rd > r && rd < rm && atomicSub(&ctr[d], 1) == 1) next[atomicAdd(nextSize, 1)] = d;
             }
         }
-    }
+    });
 }
 
 // rank-ordered flags: creators (for pair numbering) and lone cells (singletons)
@@ -396,20 +471,18 @@ __global__ void kIndegree(int n, const int* __restrict__ losortStart, int* __res
     if (d == 0) frontier[atomicAdd(size, 1)] = c;
 }
 
-__global__ void kDepthRound(int round, const int* __restrict__ frontier, int fsize,
-                            const int* __restrict__ ownStart, const int* __restrict__ upper,
-                            int* __restrict__ indeg, int* __restrict__ depth, int* __restrict__ next,
-                            int* nextSize)
+__global__ void __launch_bounds__(TPB) kDepthLoop(int* fa, int* fb, const int* __restrict__ ownStart,
+                                                  const int* __restrict__ upper, int* indeg, int* __restrict__ depth,
+                                                  FrontierLoop* F)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= fsize) return;
-    const int c = frontier[t];
-    depth[c] = round;
-    for (int f = ownStart[c]; f < ownStart[c + 1]; ++f)
-    {
-        const int nb = upper[f];
-        if (atomicSub(&indeg[nb], 1) == 1) next[atomicAdd(nextSize, 1)] = nb;
-    }
+    frontierRounds<false>(fa, fb, F, [&](int c, int, int round, int* next, int* nextSize) {
+        depth[c] = round;
+        for (int f = ownStart[c]; f < ownStart[c + 1]; ++f)
+        {
+            const int nb = upper[f];
+            if (atomicSub(&indeg[nb], 1) == 1) next[atomicAdd(nextSize, 1)] = nb;
+        }
+    });
 }
 
 __global__ void kPartOf(int n, int nParts, const int* __restrict__ partStart, int* __restrict__ partOf)
@@ -825,39 +898,49 @@ void buildLevelLayouts(LevelAddr& L, cudaStream_t s)
 // one pairing pass: gamgPairAgglomerate (AGG:158-284)
 // ---------------------------------------------------------------------------------------------
 
+// One frontier loop (its ctl zeroed, the first frontier seeded) on at most `blocks` blocks, one per SM at most: a
+// frontier is a few per cent of the cells, and more blocks would only lengthen the barrier.
+template <class Launch>
+static FrontierLoop runFrontier(int blocks, DBuf<FrontierLoop>& loop, cudaStream_t s, Launch&& launch)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(std::min(DeviceInfo::get().numSMs, std::max(1, blocks))));
+    cfg.blockDim = dim3(TPB);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B2G_CUDA(launch(cfg));
+    FrontierLoop h;
+    B2G_CUDA(cudaMemcpyAsync(&h, loop.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    B2G_CUDA(cudaStreamSynchronize(s));
+    if (h.err) fail(B2G_ERR_DEVICE_TIMEOUT, "b2g: the hierarchy build's frontier loop gave up waiting.");
+    return h;
+}
+
 static int pairPass(const LevelAddr& L, const double* w, int fwd, DBuf<int>& map, cudaStream_t s)
 {
     const int n = L.nCells;
-    DBuf<int> st, partner, target, ctr, fa, fb, sizes;
+    DBuf<int> st, partner, target, ctr, fa, fb;
+    DBuf<FrontierLoop> loop;
     st.alloc(n, s); st.zero(s);
     partner.alloc(n, s);
     target.alloc(n, s);
     ctr.alloc(n, s);
     fa.alloc(n, s);
     fb.alloc(n, s);
-    sizes.alloc(2, s);
-    sizes.zero(s);
+    loop.alloc(1, s);
+    loop.zero(s);
     kPairCounters<<<grid(n), TPB, 0, s>>>(n, fwd, L.rowStart.p, L.col.p, ctr.p);
-    kSeedFrontier<<<grid(n), TPB, 0, s>>>(n, ctr.p, fa.p, sizes.p);
+    kSeedFrontier<<<grid(n), TPB, 0, s>>>(n, ctr.p, fa.p, loop.p->size);
     B2G_LAUNCH_CHECK();
-    int fsize = readInt(sizes.p, s);
-    int* cur = fa.p;
-    int* nxt = fb.p;
-    int resolved = 0;
-    int pinned[2];
-    while (fsize > 0)
-    {
-        resolved += fsize;
-        B2G_CUDA(cudaMemsetAsync(sizes.p + 1, 0, sizeof(int), s));
-        kPairRound<<<grid(fsize), TPB, 0, s>>>(n, fwd, cur, fsize, L.rowStart.p, L.col.p, L.entFace.p, w,
-                                               st.p, partner.p, target.p, ctr.p, nxt, sizes.p + 1);
-        B2G_LAUNCH_CHECK();
-        B2G_CUDA(cudaMemcpyAsync(pinned, sizes.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-        B2G_CUDA(cudaStreamSynchronize(s));
-        fsize = pinned[1];
-        B2G_CUDA(cudaMemcpyAsync(sizes.p, sizes.p + 1, sizeof(int), cudaMemcpyDeviceToDevice, s));
-        std::swap(cur, nxt);
-    }
+    const int resolved = runFrontier(n / 512, loop, s, [&](const cudaLaunchConfig_t& cfg) {
+        return cudaLaunchKernelEx(&cfg, kPairLoop, n, fwd, fa.p, fb.p, static_cast<const int*>(L.rowStart.p),
+                                  static_cast<const int*>(L.col.p), static_cast<const int*>(L.entFace.p), w, st.p,
+                                  partner.p, target.p, ctr.p, loop.p);
+    }).resolved;
     if (resolved != n)
         fail(B2G_ERR_STATE, "b2g: the agglomeration frontier stopped with " + std::to_string(n - resolved) +
                                 " of " + std::to_string(n) + " cells undecided.");
@@ -1077,33 +1160,20 @@ void buildGsSchedule(LevelAddr& L, cudaStream_t s)
     if (n == 0) return;
     // depths by Kahn's frontier: a cell's depth is one more than its deepest owner-side neighbour
     {
-        DBuf<int> indeg, fa, fb, sizes;
+        DBuf<int> indeg, fa, fb;
+        DBuf<FrontierLoop> loop;
         indeg.alloc(n, s);
         fa.alloc(n, s);
         fb.alloc(n, s);
-        sizes.alloc(2, s);
-        sizes.zero(s);
-        kIndegree<<<grid(n), TPB, 0, s>>>(n, L.losortStart.p, indeg.p, fa.p, sizes.p);
+        loop.alloc(1, s);
+        loop.zero(s);
+        kIndegree<<<grid(n), TPB, 0, s>>>(n, L.losortStart.p, indeg.p, fa.p, loop.p->size);
         B2G_LAUNCH_CHECK();
-        int fsize = readInt(sizes.p, s);
-        int round = 0;
-        int done = 0;
-        int* cur = fa.p;
-        int* nxt = fb.p;
-        int hsz[2];
-        while (fsize > 0)
-        {
-            done += fsize;
-            B2G_CUDA(cudaMemsetAsync(sizes.p + 1, 0, sizeof(int), s));
-            kDepthRound<<<grid(fsize), TPB, 0, s>>>(round, cur, fsize, L.ownStart.p, L.upper.p, indeg.p,
-                                                    G.depth.p, nxt, sizes.p + 1);
-            B2G_LAUNCH_CHECK();
-            B2G_CUDA(cudaMemcpyAsync(hsz, sizes.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-            B2G_CUDA(cudaStreamSynchronize(s));
-            fsize = hsz[1];
-            std::swap(cur, nxt);
-            ++round;
-        }
+        const FrontierLoop h = runFrontier(n / 2048, loop, s, [&](const cudaLaunchConfig_t& cfg) {
+            return cudaLaunchKernelEx(&cfg, kDepthLoop, fa.p, fb.p, static_cast<const int*>(L.ownStart.p),
+                                      static_cast<const int*>(L.upper.p), indeg.p, G.depth.p, loop.p);
+        });
+        const int done = h.resolved, round = h.rounds;
         if (done != n) fail(B2G_ERR_STATE, "b2g: the Gauss-Seidel dependency graph has a cycle.");
         G.maxDepth = round - 1;
     }
