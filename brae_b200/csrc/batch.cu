@@ -7,7 +7,7 @@
 //
 // Reference: GAMG = src/matrices/lduMatrix/solvers/GAMG/gamg_solver_cpp.cu
 #include "batch.cuh"
-#include "pipe_kernels.cuh"
+#include "flow.cuh"
 #include "capi_internal.cuh"
 
 #include <algorithm>
@@ -21,6 +21,8 @@ namespace {
 
 constexpr int BT = 256;       // threads per tile block
 constexpr int kTile = 2048;   // cells per tile
+constexpr int kFlowBatchCells = 300000;   // the largest level whose batched sweeps are data-flow launches
+constexpr int kFlowBatchShare = 1600;     // its cells per CTA, while the CTAs fit the SMs
 constexpr int kWarpsPerBlock = BT / 32;
 
 int warpGrid(int n) { return std::max(1, ceilDiv(n, kWarpsPerBlock)); }
@@ -1037,6 +1039,7 @@ unsigned long long Batch::layoutFingerprint() const
             mix(kv.second.table.p);
             mix(kv.second.caseOf.p);
             mix(kv.second.partsBig.p);
+            for (const auto& f : kv.second.flow) mix(f.blocks.p);
         }
         for (const TileList& L : B.mc) mix(L.tiles.p);
     }
@@ -1190,13 +1193,15 @@ void Batch::smooth(int lv, int nSweeps)
     auto pit = B.pipe.find(nSweeps * 16 + static_cast<int>(sizeof(T)));
     if (pipeOn && pit != B.pipe.end() && pit->second.use)
     {
-        // the cases whose level fits one CTA: every sweep in one pipelined launch; the rest below
+        // every sweep of the cases with a data-flow schedule in one launch (two when the cases with one CTA
+        // each do not fit beside the others); the rest below
         const BatchLevel::Pipe& P = pit->second;
-        if (P.nSmall)
-        {
-            launchPipeBatch<T>(P.table.p, P.caseOf.p, P.nSmall, P.smem, active.p, stream);
-            ++launches;
-        }
+        for (const BatchLevel::FlowBlocks& F : P.flow)
+            if (F.n)
+            {
+                launchFlowBatch<T>(P.table.p, F.blocks.p, F.n, F.remote, P.caseOf.p, active.p, stream);
+                ++launches;
+            }
         parts = P.partsBig.p;
         nParts = P.nPartsBig;
     }
@@ -1211,28 +1216,70 @@ void Batch::smooth(int lv, int nSweeps)
     }
 }
 
-// The batched pipelined sweeps of level lv for nSweeps sweeps in T: per case whose level fits one
-// CTA's shared memory, the one-CTA schedule (on its mesh, built once) with that case's vectors; the
-// other cases' parts for the sweep-by-sweep launch. Outside any capture.
+// The batched sweeps of level lv for nSweeps sweeps in T as data-flow launches (flow_kernels.cuh): each case's
+// level on a share of the SMs by its size, a power of two of CTAs (so a mesh keeps few schedules). All in one
+// cooperative launch while the CTAs fit the SMs; the cases with one CTA, which wait for nobody, in a launch of
+// their own when not. Levels above kFlowBatchCells keep the sweep-by-sweep launch: they would hold the GPU's
+// SMs anyway, and their schedules would weigh on every resident case's memory. Outside any capture.
 template <class T>
 void Batch::preparePipe(int lv, int nSweeps)
 {
     BatchLevel& B = lev[lv];
     const int key = nSweeps * 16 + static_cast<int>(sizeof(T));
     if (B.nParts == 0) return;
-    if (B.pipe.count(key)) return;
+    if (B.pipe.count(key))
+    {
+        // the values for the current coefficients (into the same buffers)
+        for (const auto& f : B.pipe[key].flows)
+        {
+            Matrix& A = *cases[f.first];
+            if (A.data<T>().flows[f.second->id].gen == A.coefGen) continue;
+            A.flowValuesOf<T>(lv, *f.second);
+            B2G_CUDA(cudaStreamSynchronize(A.stream));
+        }
+        return;
+    }
     BatchLevel::Pipe& P = B.pipe[key];
     const int K = static_cast<int>(cases.size());
-    std::vector<k::PipeArgs<T>> table;
+    std::vector<k::FlowArgs<T>> table;
     std::vector<int> caseOf;
     std::vector<char> small(K, 0);
+    std::vector<int> ranks(K, 0);
+    const int sms = DeviceInfo::get().numSMs;
+    {
+        // a CTA per kFlowBatchShare cells, fewer for all when that is more than the SMs
+        double share = kFlowBatchShare;
+        for (bool fits = false; !fits; share *= 1.1)
+        {
+            int remote = 0, single = 0;
+            for (int c = 0; c < K; ++c)
+            {
+                if (nLevelsOf[c] < lv + 1) continue;
+                const int n = cases[c]->mesh->lev[lv].nCells;
+                if (n == 0 || n > kFlowBatchCells) continue;
+                int r = 1;
+                while (2 * r * share <= n && 2 * r <= sms) r *= 2;
+                ranks[c] = r;
+                if (r > 1) remote += r;
+                else ++single;
+            }
+            fits = remote == 0 || remote + std::min(single, sms / 2) <= sms;
+        }
+    }
+    std::vector<FlowJob> jobs;
+    std::vector<int> jobCase;
     for (int c = 0; c < K; ++c)
     {
-        if (nLevelsOf[c] < lv + 1 || lv > nLevelsOf[c]) continue;
+        if (ranks[c] == 0) continue;
+        jobs.push_back({&cases[c]->mesh->lev[lv], ranks[c], nullptr});
+        jobCase.push_back(c);
+    }
+    flowsForBatch(jobs, nSweeps, sizeof(T), stream);
+    for (size_t i = 0; i < jobs.size(); ++i)
+    {
+        const int c = jobCase[i];
         Matrix& A = *cases[c];
-        LevelAddr& L = A.mesh->lev[lv];
-        if (L.nCells == 0) continue;
-        const PipeSchedule* S = pipeOneCta(L, nSweeps, sizeof(T), stream);
+        const FlowSchedule* S = jobs[i].flow;
         if (!S) continue;
         const T* b;
         T* psi;
@@ -1246,10 +1293,11 @@ void Batch::preparePipe(int lv, int nSweeps)
             b = reinterpret_cast<const T*>(lv == 0 ? A.r32.p : A.v32.src[lv - 1].p);
             psi = reinterpret_cast<T*>(lv == 0 ? A.w32.p : A.v32.corr[lv - 1].p);
         }
-        table.push_back(A.pipeArgs<T>(lv, *S, psi, b));
+        table.push_back(A.flowArgs<T>(lv, *S, psi, b));
+        B2G_CUDA(cudaStreamSynchronize(A.stream));  // its values were filled there
         caseOf.push_back(c);
         small[c] = 1;
-        P.smem = std::max(P.smem, pipeSmemBytes(*S, sizeof(T)));
+        P.flows.push_back({c, S});
     }
     std::vector<int4> big;
     for (const int4& q : B.hostParts)
@@ -1258,9 +1306,29 @@ void Batch::preparePipe(int lv, int nSweeps)
     P.nPartsBig = static_cast<int>(big.size());
     if (P.nSmall)
     {
-        P.table.upload(reinterpret_cast<const unsigned char*>(table.data()), sizeof(k::PipeArgs<T>) * table.size(),
+        std::vector<int2> many, one;
+        for (int i = 0; i < P.nSmall; ++i)
+            for (int r = 0; r < table[i].ranks; ++r) (table[i].ranks > 1 ? many : one).push_back(make_int2(i, r));
+        // (one launch when every CTA fits; the one-CTA cases first else, the largest first)
+        if (!many.empty() && many.size() + one.size() <= static_cast<size_t>(sms))
+        {
+            many.insert(many.end(), one.begin(), one.end());
+            one.clear();
+        }
+        std::stable_sort(one.begin(), one.end(), [&](const int2& x, const int2& y) {
+            return cases[caseOf[x.x]]->mesh->lev[lv].nCells > cases[caseOf[y.x]]->mesh->lev[lv].nCells;
+        });
+        for (int i = 0; i < 2; ++i)
+        {
+            const std::vector<int2>& v = i == 0 ? many : one;
+            P.flow[i].n = static_cast<int>(v.size());
+            P.flow[i].remote = i == 0;
+            if (!v.empty()) P.flow[i].blocks.upload(v.data(), v.size(), stream);
+        }
+        P.table.upload(reinterpret_cast<const unsigned char*>(table.data()), sizeof(k::FlowArgs<T>) * table.size(),
                        stream);
         P.caseOf.upload(caseOf.data(), caseOf.size(), stream);
+        B2G_CUDA(cudaStreamSynchronize(stream));  // the host lists go out of scope
     }
     if (P.nPartsBig) P.partsBig.upload(big.data(), big.size(), stream);
     B2G_CUDA(cudaStreamSynchronize(stream));

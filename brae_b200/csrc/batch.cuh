@@ -101,13 +101,20 @@ struct BatchLevel
     DBuf<unsigned> progress;
     size_t ticketAt = 0;  // the sweep launch's ticket counter: the word after the parts' progress lines
     std::vector<int4> hostParts;  // the parts table on the host
-    // the exact form's smoothing calls by sweeps * 16 + value size: the cases whose level fits one CTA
-    // run all their sweeps in one pipelined launch (pipe_kernels.cuh), the others the sweep above
+    // the exact form's smoothing calls by sweeps * 16 + value size: the cases whose level has a schedule
+    // run all their sweeps in data-flow launches (flow_kernels.cuh), the others the sweep above
+    struct FlowBlocks
+    {
+        DBuf<int2> blocks;           // {entry of the table, rank}
+        int n = 0;
+        bool remote = false;         // some entry has more than one rank
+    };
     struct Pipe
     {
         int nSmall = 0;
-        size_t smem = 0;
-        DBuf<unsigned char> table;   // k::PipeArgs<T>[nSmall]
+        DBuf<unsigned char> table;   // k::FlowArgs<T>[nSmall]
+        FlowBlocks flow[2];          // the launches: with more than one rank, and one CTA each
+        std::vector<std::pair<int, const FlowSchedule*>> flows;  // {case, its schedule}
         DBuf<int> caseOf;            // [nSmall]
         DBuf<int4> partsBig;         // the parts of the cases that do not fit
         int nPartsBig = 0;

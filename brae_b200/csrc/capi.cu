@@ -902,6 +902,40 @@ b2g_status b2g_level_smooth_pipelined(b2g_matrix* m, int level, double* psi, con
     });
 }
 
+b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const double* source, int nSweeps, int symmetric,
+                                 int ranks, int weight, long long stallLimit, float* ms)
+{
+    return guarded([&] {
+        need(m && psi && source, "b2g_level_smooth_flow: null argument");
+        need(level >= 0 && level <= m->mat->nLevels(), "b2g_level_smooth_flow: level out of range");
+        need(nSweeps >= 1, "b2g_level_smooth_flow: nSweeps must be positive");
+        need(ranks >= 1 && weight >= 1 && weight <= 64, "b2g_level_smooth_flow: ranks and weight must be positive, weight at most 64");
+        need(stallLimit >= 0 && stallLimit <= b2g::k::kSpinLimit, "b2g_level_smooth_flow: stallLimit out of range");
+        b2g::Matrix& A = *m->mat;
+        need(!A.coupled, "b2g_level_smooth_flow: not for a coupled matrix");
+        A.toPos(level, static_cast<const double*>(psi), A.ioBuf(0));
+        A.toPos(level, source, A.ioBuf(1));
+        struct Waits
+        {
+            b2g::Matrix& A;
+            ~Waits()
+            {
+                A.spinLimit = b2g::k::kSpinLimit;
+                A.publish = 1;
+            }
+        } waits{A};
+        if (stallLimit > 0)
+        {
+            A.spinLimit = stallLimit;
+            A.publish = 0;
+        }
+        if (!A.flowForced<double>(level, A.ioBuf(0), A.ioBuf(1), nSweeps, symmetric != 0, ranks, weight, ms))
+            b2g::fail(B2G_ERR_ARGUMENT, "b2g_level_smooth_flow: the level does not fit that many CTAs");
+        A.fromPos(level, static_cast<const double*>(A.ioBuf(0)), psi);
+        B2G_CUDA(cudaStreamSynchronize(A.stream));
+    });
+}
+
 b2g_status b2g_coarsest_dense_solve(b2g_matrix* m, double* psi, const double* source)
 {
     return guarded([&] {
@@ -935,12 +969,13 @@ b2g_status b2g_level_pipe_shape(const b2g_mesh* mesh, int level, int nSweeps, in
         const auto it = pipe.find(nSweeps * 16 + valueBytes);
         const bool have = it != pipe.end();
         const int mode = have ? it->second.mode : 0;
-        if (ranks) *ranks = mode == 1 ? it->second.sched->ranks : mode == 2 ? -it->second.items->nParts : 0;
+        if (ranks)
+            *ranks = mode == 1 ? it->second.sched->ranks : mode == 2 ? -it->second.items->nParts : mode == 3 ? it->second.flow->ranks : 0;
         if (nSteps)
-            *nSteps = mode == 1 ? it->second.sched->nSteps : mode == 2 ? it->second.items->maxDepth + 1 : 0;
+            *nSteps = mode == 1 ? it->second.sched->nSteps : mode == 2 ? it->second.items->maxDepth + 1 : mode == 3 ? it->second.flow->nSteps : 0;
         const bool grid = mode == 1 && it->second.sched->grid;
         if (msPipe)
-            *msPipe = !have ? 0.f : mode == 2 ? it->second.msItems : grid ? it->second.msGrid : it->second.msPipe;
+            *msPipe = !have ? 0.f : mode == 3 ? it->second.msFlow : mode == 2 ? it->second.msItems : grid ? it->second.msGrid : it->second.msPipe;
         if (msGrid) *msGrid = have ? it->second.msGrid : 0.f;
         if (gridForm) *gridForm = grid ? 1 : 0;
         if (msSweeps) *msSweeps = have ? it->second.msSweeps : 0.f;
@@ -1000,7 +1035,7 @@ b2g_status b2g_level_mc_pipe(const b2g_mesh* mesh, int level, int nSweeps, int s
         const b2g::Colouring& C = mesh->m.lev[level].mc;
         const auto it = C.pipe.find(nSweeps * 2 + (symmetric ? 1 : 0));
         const bool have = it != C.pipe.end();
-        if (ranks) *ranks = have && it->second.use ? it->second.sched->ranks : 0;
+        if (ranks) *ranks = have && it->second.use ? it->second.flow->ranks : 0;
         if (msPipe) *msPipe = have ? it->second.msPipe : 0.f;
         if (msColours) *msColours = have ? it->second.msColours : 0.f;
     });

@@ -1,0 +1,401 @@
+// flow.cu -- the data-flow launch of a smoothing call (flow_kernels.cuh): its schedule on the device, its
+// values per matrix, and its launch.
+
+#include "flow.cuh"
+#include "solver.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <vector>
+
+namespace b2g {
+namespace {
+
+template <class T>
+void allowFlowSmem()
+{
+    static std::atomic<unsigned long long> done{0};  // one bit per device
+    int dev = 0;
+    B2G_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (done.load() & bit) return;
+    auto allow = [](const void* f) {
+        B2G_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFlowSmem)));
+    };
+    allow(reinterpret_cast<const void*>(&k::gsFlow<T, false, false>));
+    allow(reinterpret_cast<const void*>(&k::gsFlow<T, false, true>));
+    allow(reinterpret_cast<const void*>(&k::gsFlowBatch<T, false>));
+    allow(reinterpret_cast<const void*>(&k::gsFlowBatch<T, true>));
+    if constexpr (sizeof(T) == 4)
+    {
+        allow(reinterpret_cast<const void*>(&k::gsFlow<T, true, false>));
+        allow(reinterpret_cast<const void*>(&k::gsFlow<T, true, true>));
+    }
+    done.fetch_or(bit);
+}
+
+}  // namespace
+
+FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s)
+{
+    FlowLevel H;
+    H.n = L.nCells;
+    H.nF = L.nFaces;
+    H.lower = L.lower.download(s);
+    H.upper = L.upper.download(s);
+    H.depth = L.gs.depth.download(s);
+    H.posCell = L.gs.posCell.download(s);
+    H.posRow = L.gs.posRow.download(s);
+    H.entColPos = L.gs.entColPos.download(s);
+    H.lower.resize(H.nF);
+    H.upper.resize(H.nF);
+    H.posCell.resize(H.n);
+    H.posRow.resize(static_cast<size_t>(H.n) + 1);
+    H.cellPos.resize(H.n);
+    for (int p = 0; p < H.n; ++p) H.cellPos[H.posCell[p]] = p;
+    return H;
+}
+
+static std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int S, int nSteps, int R, cudaStream_t s);
+
+std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb,
+                                        cudaStream_t s)
+{
+    FlowProgram G;
+    if (!buildFlowProgram(H, T, S, nSteps, R, vb, G)) return nullptr;
+    return uploadFlow(G, S, nSteps, R, s);
+}
+
+std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int S, int nSteps, int R, cudaStream_t s)
+{
+    auto F = std::make_unique<FlowSchedule>();
+    static std::atomic<long long> nextId{1};
+    F->id = nextId++;
+    F->sweeps = S;
+    F->ranks = R;
+    F->nSteps = nSteps;
+    F->slots = G.slots;
+    F->nVal = static_cast<long long>(G.nVal);
+    F->meta.alloc(std::max<size_t>(G.metaBytes, 16), s);
+    F->src.alloc(std::max<size_t>(G.nVal, 1), s);
+    size_t metaAt = 0, valAt = 0;
+    for (const RankProgram& P : G.prog)
+    {
+        if (!P.meta.empty())
+            B2G_CUDA(cudaMemcpyAsync(F->meta.p + metaAt, P.meta.data(), P.meta.size(), cudaMemcpyHostToDevice, s));
+        if (!P.src.empty())
+            B2G_CUDA(cudaMemcpyAsync(F->src.p + valAt, P.src.data(), sizeof(int) * P.src.size(), cudaMemcpyHostToDevice, s));
+        metaAt += P.meta.size();
+        valAt += P.src.size();
+    }
+    F->chunkStart.upload(G.chunkStart.data(), G.chunkStart.size(), s);
+    F->rec.upload(reinterpret_cast<const int4*>(G.rec.data()), 3 * G.rec.size(), s);
+    B2G_CUDA(cudaStreamSynchronize(s));  // the host arrays go out of scope
+    return F;
+}
+
+// Measured per smoothing call (FP64, graded boxes of 24 k and 1 M cells, all levels; 1 to 148 CTAs, weights 2
+// and 4): a hand-over through L2 takes about four steps, so 4 beats 2 nearly everywhere; one CTA per SM is the
+// fastest above 700 k cells, that or half as many down to 200 k, then about one per 1,000 to 4,000 cells.
+std::vector<FlowShape> flowShapes(int n)
+{
+    const int sms = DeviceInfo::get().numSMs;
+    std::vector<FlowShape> out;
+    auto add = [&](int R, int w) {
+        R = std::min(R, sms);
+        if (R < 1 || R > n) return;
+        if (R == 1) w = 1;
+        for (const FlowShape& f : out)
+            if (f.ranks == R && f.weight == w) return;
+        out.push_back({R, w});
+    };
+    if (n >= 700000)
+        add(sms, 4);
+    else if (n >= 200000)
+    {
+        add(sms, 4);
+        add(sms / 2, 4);
+    }
+    else
+    {
+        int r = 1;
+        while (2 * r * 2000 <= n) r *= 2;
+        add(r, 4);
+        if (n >= 6000) add(2 * r, 4);
+    }
+    return out;
+}
+
+bool flowFits(int ranks)
+{
+    return ranks <= DeviceInfo::get().numSMs;
+}
+
+// A schedule's values on this matrix, refilled when the coefficients changed since (outside any capture).
+template <class T>
+const T* Matrix::flowValuesOf(int level, const FlowSchedule& F)
+{
+    VCycleData<T>& D = data<T>();
+    auto& B = D.flows[F.id];
+    if (B.gen != coefGen)
+    {
+        if (capturing) fail(B2G_ERR_STATE, "b2g: a smoothing schedule's values were not filled before the capture");
+        B.val.ensure(static_cast<size_t>(std::max<long long>(F.nVal, 1)), stream);
+        if (F.nVal)
+            k::flowValues<T><<<std::min(ceilDiv(F.nVal, 256), 8192), 256, 0, stream>>>(
+                F.nVal, F.src.p, D.coef[level].rowVal.p, D.coef[level].gsDiag.p, B.val.p);
+        B2G_LAUNCH_CHECK();
+        if (F.ranks > 1 && !B.mail.p)
+        {
+            B.mail.alloc(2 * sizeof(T) * static_cast<size_t>(mesh->lev[level].nCells), stream);
+            B.mail.zero(stream);
+            const unsigned first[2] = {1, 0};
+            B.ctl.upload(first, 2, stream);
+            B2G_CUDA(cudaStreamSynchronize(stream));  // first is on this frame
+        }
+        B.gen = coefGen;
+    }
+    return B.val.p;
+}
+
+template <class T>
+k::FlowArgs<T> Matrix::flowArgs(int level, const FlowSchedule& F, T* psiL, const T* src)
+{
+    k::FlowArgs<T> a;
+    a.chunkStart = F.chunkStart.p;
+    a.rec = F.rec.p;
+    a.meta = F.meta.p;
+    a.val = flowValuesOf<T>(level, F);
+    a.b = src;
+    a.psi = psiL;
+    const auto& B = data<T>().flows[F.id];
+    a.mail = B.mail.p;
+    a.ctl = B.ctl.p;
+    a.ranks = F.ranks;
+    a.slots = F.slots;
+    a.spinLimit = spinLimit;
+    a.err = err.p;
+    a.publish = publish;
+    return a;
+}
+
+template <class T>
+void Matrix::flowLaunch(int level, const FlowSchedule& F, T* psiL, const T* src, bool fma)
+{
+    allowFlowSmem<T>();
+    const k::FlowArgs<T> a = flowArgs<T>(level, F, psiL, src);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(F.ranks));
+    cfg.blockDim = dim3(static_cast<unsigned>(k::flowThreads(F.ranks > 1)));
+    cfg.dynamicSmemBytes = kFlowSmem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = F.ranks > 1 ? 1 : 0;
+    if constexpr (sizeof(T) == 4)
+    {
+        if (fma)
+        {
+            B2G_CUDA(F.ranks > 1 ? cudaLaunchKernelEx(&cfg, k::gsFlow<T, true, true>, a)
+                                 : cudaLaunchKernelEx(&cfg, k::gsFlow<T, true, false>, a));
+            ++launches;
+            return;
+        }
+    }
+    if (fma) fail(B2G_ERR_STATE, "b2g: the multicolour smoothing schedule is FP32 only");
+    B2G_CUDA(F.ranks > 1 ? cudaLaunchKernelEx(&cfg, k::gsFlow<T, false, true>, a)
+                         : cudaLaunchKernelEx(&cfg, k::gsFlow<T, false, false>, a));
+    ++launches;
+}
+
+// The mean milliseconds of a few calls, after one that fills the values.
+template <class T>
+float Matrix::flowTime(int level, const FlowSchedule& F, T* psiL, const T* src, bool fma)
+{
+    constexpr int kCalls = 3;
+    flowLaunch<T>(level, F, psiL, src, fma);
+    cudaEvent_t e0, e1;
+    B2G_CUDA(cudaEventCreate(&e0));
+    B2G_CUDA(cudaEventCreate(&e1));
+    B2G_CUDA(cudaEventRecord(e0, stream));
+    for (int i = 0; i < kCalls; ++i) flowLaunch<T>(level, F, psiL, src, fma);
+    B2G_CUDA(cudaEventRecord(e1, stream));
+    B2G_CUDA(cudaEventSynchronize(e1));
+    float ms = 0.f;
+    B2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    checkDeviceError();
+    return ms / kCalls;
+}
+
+// nSweeps sweeps of `level` as one data-flow launch on `ranks` CTAs, whatever the tuned choice (for
+// tests and tuning); false when the level has no such schedule. ms (may be null): a call's mean time.
+template <class T>
+bool Matrix::flowForced(int level, T* psiL, const T* src, int nSweeps, bool symmetric, int ranks, int weight, float* ms)
+{
+    if (ranks < 1 || weight < 1 || !flowFits(ranks)) return false;
+    FlowLevel H = flowDownload(mesh->lev[level], stream);
+    int nSteps = 0;
+    const std::vector<int> steps = flowSteps(H, nSweeps, symmetric, ranks, weight, nSteps);
+    std::unique_ptr<FlowSchedule> F = buildFlow(H, steps, symmetric ? 2 * nSweeps : nSweeps, nSteps, ranks, sizeof(T), stream);
+    if (!F) return false;
+    struct Drop
+    {
+        VCycleData<T>& D;
+        long long id;
+        ~Drop() { D.flows.erase(id); }
+    } drop{data<T>(), F->id};
+    flowLaunch<T>(level, *F, psiL, src, false);
+    if (ms) *ms = flowTime<T>(level, *F, psiL, src);
+    B2G_CUDA(cudaStreamSynchronize(stream));  // F is released on return
+    checkDeviceError();
+    return true;
+}
+
+// The symmetric sweeps' launch of `level` (null: the level has no such schedule). Not timed against the sweeps' own launches, two and two
+// vector moves a sweep: on a 61 x 47 x 53 box those took 0.17 (33 cells) to 1.5 ms (19 k cells) a call of
+// four sweeps. Outside any capture.
+template <class T>
+void Matrix::ensureSymFlow(int level, int nSweeps)
+{
+    LevelAddr& L = mesh->lev[level];
+    const int key = nSweeps * 16 + static_cast<int>(sizeof(T));
+    if (L.flowSym.count(key)) return;
+    std::unique_ptr<FlowSchedule>& kept = L.flowSym[key];
+    if (nSweeps < 1 || L.nCells == 0) return;
+    DBuf<T> x, b;
+    x.alloc(nAlloc(level), stream);
+    b.alloc(nAlloc(level), stream);
+    x.zero(stream);
+    b.zero(stream);
+    FlowLevel H = flowDownload(L, stream);
+    float best = 0.f;
+    const long long l0 = launches;
+    // (the walks of a symmetric call follow one another, so a step has a share of the items it has in a forward
+    // call of as many sweeps: half the CTAs)
+    for (const FlowShape& f : {FlowShape{std::max(1, flowShapes(L.nCells).front().ranks / 2), 4}})
+    {
+        int nSteps = 0;
+        const std::vector<int> steps = flowSteps(H, nSweeps, true, f.ranks, f.weight, nSteps);
+        std::unique_ptr<FlowSchedule> F = buildFlow(H, steps, 2 * nSweeps, nSteps, f.ranks, sizeof(T), stream);
+        if (!F) continue;
+        const float ms = flowTime<T>(level, *F, x.p, b.p);
+        if (!kept || ms < best)
+        {
+            best = ms;
+            if (kept) data<T>().flows.erase(kept->id);
+            kept = std::move(F);
+        }
+        else
+            data<T>().flows.erase(F->id);
+    }
+    launches = l0;
+    B2G_CUDA(cudaStreamSynchronize(stream));
+}
+
+// nSweeps symmetric sweeps of `level` in one launch; false when they run as launches of their own
+template <class T>
+bool Matrix::symFlowSweeps(int level, T* psiL, const T* src, int nSweeps)
+{
+    if (!g_pipeline) return false;
+    LevelAddr& L = mesh->lev[level];
+    const int key = nSweeps * 16 + static_cast<int>(sizeof(T));
+    auto it = L.flowSym.find(key);
+    if (it == L.flowSym.end())
+    {
+        if (capturing) return false;
+        ensureSymFlow<T>(level, nSweeps);
+        it = L.flowSym.find(key);
+    }
+    if (!it->second) return false;
+    flowLaunch<T>(level, *it->second, psiL, src);
+    return true;
+}
+
+// Before a capture: the values of every symmetric launch, for the current coefficients.
+template <class T>
+void Matrix::refreshSymFlows()
+{
+    for (int lv = 0; lv <= nLevels(); ++lv)
+        for (auto& kv : mesh->lev[lv].flowSym)
+            if (kv.second && kv.first % 16 == static_cast<int>(sizeof(T))) flowValuesOf<T>(lv, *kv.second);
+}
+
+void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStream_t s)
+{
+    auto keyOf = [&](const FlowJob& j) { return std::pair<int, int>{nSweeps * 16 + static_cast<int>(vb), j.ranks}; };
+    struct Work
+    {
+        size_t job;
+        FlowLevel H;
+        FlowProgram G;
+        int nSteps = 0;
+        bool ok = false;
+    };
+    std::vector<Work> work;
+    for (size_t i = 0; i < jobs.size(); ++i)
+    {
+        auto known = jobs[i].level->flowBatch.find(keyOf(jobs[i]));
+        if (known != jobs[i].level->flowBatch.end()) continue;
+        jobs[i].level->flowBatch[keyOf(jobs[i])];  // (a level listed twice is built once)
+        work.emplace_back();
+        work.back().job = i;
+        work.back().H = flowDownload(*jobs[i].level, s);
+    }
+    flowParallel(static_cast<int>(work.size()), [&](int i, int) {
+        Work& w = work[i];
+        const int R = jobs[w.job].ranks;
+        const std::vector<int> steps = flowSteps(w.H, nSweeps, false, R, 4, w.nSteps);
+        w.ok = buildFlowProgram(w.H, steps, nSweeps, w.nSteps, R, vb, w.G);
+    });
+    for (Work& w : work)
+    {
+        const FlowJob& j = jobs[w.job];
+        if (w.ok) j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, nSweeps, w.nSteps, j.ranks, s);
+    }
+    for (FlowJob& j : jobs) j.flow = j.level->flowBatch[keyOf(j)].get();
+}
+
+template <class T>
+void launchFlowBatch(const void* table, const int2* blocks, int nBlocks, bool remote, const int* caseOf, const int* active,
+                     cudaStream_t s)
+{
+    allowFlowSmem<T>();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(nBlocks));
+    cfg.blockDim = dim3(static_cast<unsigned>(k::flowThreads(remote)));
+    cfg.dynamicSmemBytes = kFlowSmem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = remote ? 1 : 0;
+    const auto* t = static_cast<const k::FlowArgs<T>*>(table);
+    B2G_CUDA(remote ? cudaLaunchKernelEx(&cfg, k::gsFlowBatch<T, true>, t, blocks, caseOf, active)
+                    : cudaLaunchKernelEx(&cfg, k::gsFlowBatch<T, false>, t, blocks, caseOf, active));
+}
+template void launchFlowBatch<double>(const void*, const int2*, int, bool, const int*, const int*, cudaStream_t);
+template void launchFlowBatch<float>(const void*, const int2*, int, bool, const int*, const int*, cudaStream_t);
+template k::FlowArgs<double> Matrix::flowArgs<double>(int, const FlowSchedule&, double*, const double*);
+template k::FlowArgs<float> Matrix::flowArgs<float>(int, const FlowSchedule&, float*, const float*);
+
+template bool Matrix::flowForced<double>(int, double*, const double*, int, bool, int, int, float*);
+template bool Matrix::flowForced<float>(int, float*, const float*, int, bool, int, int, float*);
+template void Matrix::ensureSymFlow<double>(int, int);
+template void Matrix::ensureSymFlow<float>(int, int);
+template bool Matrix::symFlowSweeps<double>(int, double*, const double*, int);
+template bool Matrix::symFlowSweeps<float>(int, float*, const float*, int);
+template void Matrix::refreshSymFlows<double>();
+template void Matrix::refreshSymFlows<float>();
+template float Matrix::flowTime<double>(int, const FlowSchedule&, double*, const double*, bool);
+template float Matrix::flowTime<float>(int, const FlowSchedule&, float*, const float*, bool);
+template void Matrix::flowLaunch<double>(int, const FlowSchedule&, double*, const double*, bool);
+template void Matrix::flowLaunch<float>(int, const FlowSchedule&, float*, const float*, bool);
+template const double* Matrix::flowValuesOf<double>(int, const FlowSchedule&);
+template const float* Matrix::flowValuesOf<float>(int, const FlowSchedule&);
+
+}  // namespace b2g

@@ -1,0 +1,82 @@
+// flow.cuh -- the schedule of the data-flow launch of a smoothing call (flow_kernels.cuh) and its builder.
+#pragma once
+
+#include "flow_kernels.cuh"
+#include "hierarchy.cuh"
+
+#include <functional>
+#include <memory>
+#include <vector>
+
+namespace b2g {
+
+// The level's addressing on the host, as the schedule builder reads it.
+struct FlowLevel
+{
+    int n = 0, nF = 0;
+    std::vector<int> lower, upper, depth, posCell, posRow, entColPos, cellPos;
+    bool crosses = false;  // more than one rank
+};
+
+// rank r's cells are [flowBegin(r), flowBegin(r + 1))
+inline int flowBegin(int r, int n, int R) { return static_cast<int>((static_cast<long long>(r) * n + R - 1) / R); }
+inline int flowRank(int c, int n, int R) { return static_cast<int>(static_cast<long long>(c) * R / n); }
+
+constexpr size_t kFlowSmem = 220 * 1024;  // dynamic shared memory of a CTA: value slots and ring
+
+// One rank's program .
+struct RankProgram
+{
+    std::vector<k::FlowRec> rec;
+    std::vector<unsigned char> meta;
+    std::vector<int> src;     // per value (flowValues)
+    int slots = 1;            // value slots used (slot 0 is the zero)
+    bool ok = true;
+};
+
+// A whole launch's program, ranks in order (the ranks' blobs and values follow one another).
+struct FlowProgram
+{
+    std::vector<RankProgram> prog;
+    std::vector<int> chunkStart;   // [ranks + 1]
+    std::vector<k::FlowRec> rec;
+    int slots = 1;
+    size_t metaBytes = 0, nVal = 0;
+};
+
+FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s);
+std::vector<int> flowSteps(const FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps);
+// The program for R ranks of items (visit q, cell c) at steps T[q * n + c], values of vb bytes; false when
+// a rank's live values or chunks do not fit its shared memory, or a row is too long.
+bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb, FlowProgram& F);
+// The same on the device, or null.
+std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb,
+                                        cudaStream_t s);
+// The batched form's launches of nSweeps sweeps: per job its level on `ranks` CTAs, built once and kept on the
+// level, the missing ones side by side on the host's cores; job.flow is null when the level has none.
+struct FlowJob
+{
+    LevelAddr* level;
+    int ranks;
+    const FlowSchedule* flow;
+};
+void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStream_t s);
+// The batched launch (flow.cu): table = k::FlowArgs<T>[entries] on the device, blocks[i] = {entry, rank},
+// caseOf[entry] its case. `remote`: some entry has more than one rank (a cooperative launch).
+template <class T>
+void launchFlowBatch(const void* table, const int2* blocks, int nBlocks, bool remote, const int* caseOf, const int* active,
+                     cudaStream_t s);
+// Runs body(i, worker) for i in [0, n) on the host's cores, worker < kFlowThreads; the first exception is
+// rethrown. Nested calls run on the calling thread.
+constexpr int kFlowThreads = 16;
+void flowParallel(int n, const std::function<void(int, int)>& body);
+// The launches worth timing on a level of n cells.
+struct FlowShape
+{
+    int ranks, weight;
+};
+std::vector<FlowShape> flowShapes(int n);
+// whether a launch of that many ranks can be resident (one CTA per SM)
+bool flowFits(int ranks);
+
+}  // namespace b2g

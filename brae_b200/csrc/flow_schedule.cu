@@ -1,0 +1,433 @@
+// flow_schedule.cu -- the schedule of the data-flow launch of a smoothing call (flow_kernels.cuh), built
+// once per (level, sweep count, value type) on the host from the level's addressing. Host code only.
+//
+// Reference: the sweeps it reproduces are gaussSeidelSweeps, src/OpenFOAM/matrices/
+// smooth_solver_cpp.cu:87-166 (forward only for GaussSeidel, :144), called nSweeps times per
+// smoothing call by GaussSeidelSmoother::smooth (gamg_solver_cpp.cu:234-317).
+
+#include "flow.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <exception>
+#include <thread>
+#include <vector>
+
+namespace b2g {
+namespace {
+
+constexpr int kFlowChunkItems = 32 * k::kFlowTeam;      // items of a chunk, at most (the team's threads)
+constexpr size_t kFlowChunkBytes = 28 * 1024;           // and its place in the ring
+
+// scratch of one builder thread
+struct RankScratch
+{
+    std::vector<int> localOf;  // cell -> ghost index of the rank at work, -1
+};
+
+struct ItemRef
+{
+    int p, q, w;  // position, visit, row width
+    bool out;     // another rank reads it
+};
+
+void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int c0, int c1, size_t vb,
+               RankScratch& X, RankProgram& P)
+{
+    const size_t n = static_cast<size_t>(H.n);
+    const int nOwn = c1 - c0;
+    if (X.localOf.size() != n) X.localOf.assign(n, -1);
+    // cells another rank reads: those with a neighbour there
+    std::vector<char> exported(nOwn, 0);
+    if (H.crosses)
+        for (int c = c0; c < c1; ++c)
+        {
+            const int p = H.cellPos[c];
+            for (int e = H.posRow[p]; e < H.posRow[p + 1] && !exported[c - c0]; ++e)
+            {
+                const int cn = H.posCell[H.entColPos[e]];
+                exported[c - c0] = cn < c0 || cn >= c1;
+            }
+        }
+    // items by step; of a step of several chunks those that another rank reads first, so that their way there
+    // overlaps the step's other chunks; then the longest rows first, so that the slices of a chunk pad little
+    std::vector<int> start(static_cast<size_t>(nSteps) + 1, 0);
+    for (int q = 0; q < S; ++q)
+        for (int c = c0; c < c1; ++c) ++start[T[q * n + c] + 1];
+    for (int i = 0; i < nSteps; ++i) start[i + 1] += start[i];
+    std::vector<ItemRef> items(static_cast<size_t>(S) * nOwn);
+    {
+        std::vector<int> cur(start.begin(), start.end() - 1);
+        for (int q = 0; q < S; ++q)
+            for (int c = c0; c < c1; ++c)
+            {
+                const int p = H.cellPos[c];
+                items[cur[T[q * n + c]]++] = ItemRef{p, q, H.posRow[p + 1] - H.posRow[p], exported[c - c0] != 0};
+            }
+    }
+    struct Span
+    {
+        int a, b;
+    };
+    std::vector<Span> chunks;
+    for (int st = 0; st < nSteps; ++st)
+    {
+        const int a = start[st], b = start[st + 1];
+        if (a == b) continue;
+        const bool several = b - a > kFlowChunkItems;
+        std::sort(items.begin() + a, items.begin() + b, [several](const ItemRef& x, const ItemRef& y) {
+            if (several && x.out != y.out) return x.out;
+            return x.w != y.w ? x.w > y.w : x.p != y.p ? x.p < y.p : x.q < y.q;
+        });
+        // cut where the chunk is full: whole slices, its blobs and source within its share of the ring
+        int from = a;
+        size_t bytes = 64;
+        for (int i = a; i < b; i += 32)
+        {
+            int w = 0;
+            for (int x = i; x < std::min(b, i + 32); ++x) w = std::max(w, items[x].w);
+            if (w > 252)
+            {
+                P.ok = false;
+                return;
+            }
+            // slice: descriptors, diagonal, source, entries; about half of them a fetch or a ghost
+            const size_t sl = 16 + 32 * (8 + 3 * vb) + static_cast<size_t>(32) * ((w + 3) & ~3) * (vb + 2 + 4);
+            if (i > from && (i - from >= kFlowChunkItems || bytes + sl > kFlowChunkBytes))
+            {
+                chunks.push_back({from, i});
+                from = i;
+                bytes = 64;
+            }
+            bytes += sl;
+        }
+        chunks.push_back({from, b});
+    }
+    const int nCh = static_cast<int>(chunks.size());
+    // first pass: each local value's last use. Own cells are 0..nOwn-1, ghosts follow as they are met.
+    std::vector<int> last(nOwn, -1), ghostCell;
+    auto localId = [&](int cell) {
+        if (cell >= c0 && cell < c1) return cell - c0;
+        int g = X.localOf[cell];
+        if (g < 0)
+        {
+            g = static_cast<int>(ghostCell.size());
+            X.localOf[cell] = g;
+            ghostCell.push_back(cell);
+            last.push_back(-1);
+        }
+        return nOwn + g;
+    };
+    for (int j = 0; j < nCh; ++j)
+        for (int i = chunks[j].a; i < chunks[j].b; ++i)
+        {
+            const int p = items[i].p;
+            last[H.posCell[p] - c0] = j;
+            for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e) last[localId(H.posCell[H.entColPos[e]])] = j;
+        }
+    // second pass: slots (a value's from its first use to kFlowDepth chunks after its last), the
+    // fetches of initial values, the ghosts' arrivals, the chunks' blobs
+    const int nLoc = static_cast<int>(last.size());
+    std::vector<int> slot(nLoc, 0), visit(nLoc, -2);
+    std::vector<int> head(nCh, -1), nextOf(nLoc, -1);
+    for (int v = 0; v < nLoc; ++v)
+        if (last[v] >= 0)
+        {
+            nextOf[v] = head[last[v]];
+            head[last[v]] = v;
+        }
+    std::vector<int> freeSlots;
+    P.rec.resize(nCh);
+    struct Pair
+    {
+        unsigned a, b;
+    };
+    std::vector<Pair> fetch, halo;
+    std::vector<unsigned short> codes;
+    int width[kFlowChunkItems / 32 + 1], first[kFlowChunkItems / 32 + 1];
+    long long valAt = 0;
+    for (int j = 0; j < nCh; ++j)
+    {
+        if (j - k::kFlowDepth >= 0)
+            for (int v = head[j - k::kFlowDepth]; v >= 0; v = nextOf[v]) freeSlots.push_back(slot[v]);
+        auto give = [&](int v) {
+            if (slot[v]) return;
+            if (!freeSlots.empty())
+            {
+                slot[v] = freeSlots.back();
+                freeSlots.pop_back();
+            }
+            else
+                slot[v] = P.slots++;
+        };
+        const int a = chunks[j].a, b = chunks[j].b, m = b - a, nSl = (m + 31) / 32;
+        int nEnt = 0;
+        for (int s = 0; s < nSl; ++s)
+        {
+            // a multiple of 4 (the kernels' straight-line widths), at least 4
+            int longest = 0;
+            for (int i = 32 * s; i < std::min(m, 32 * s + 32); ++i) longest = std::max(longest, items[a + i].w);
+            width[s] = std::max(4, (longest + 3) & ~3);
+            first[s] = nEnt;
+            nEnt += k::flowStride(m, s) * width[s];
+        }
+        fetch.clear();
+        halo.clear();
+        codes.assign(nEnt, 0);
+        const size_t srcAt = P.src.size();
+        P.src.resize(srcAt + 64 * static_cast<size_t>(nSl) + nEnt, -1);
+        int* diagSrc = P.src.data() + srcAt;
+        int* entSrc = diagSrc + 64 * nSl;
+        for (int i = 0; i < m; ++i)
+        {
+            diagSrc[2 * i] = -(2 * items[a + i].p + 2);
+            diagSrc[2 * i + 1] = -(2 * items[a + i].p + 3);
+        }
+        // (a chunk's values are read before its items write: every read first, then the writes)
+        for (int i = 0; i < m; ++i)
+        {
+            const ItemRef& it = items[a + i];
+            const int c = H.posCell[it.p];
+            const int step = T[it.q * n + c];
+            const int st = k::flowStride(m, i / 32);
+            const int at0 = first[i / 32], l = i % 32, vg = vb == 8 ? 2 : 4;
+            for (int e = H.posRow[it.p], q = 0; e < H.posRow[it.p + 1]; ++e, ++q)
+            {
+                const int pn = H.entColPos[e];
+                const int cn = H.posCell[pn];
+                const int v = localId(cn);
+                // the neighbour's latest visit before this item (-1: its initial value)
+                int ver = it.q;
+                while (ver >= 0 && T[ver * n + cn] >= step) --ver;
+                if (v < nOwn)
+                {
+                    if (!slot[v])
+                    {
+                        give(v);
+                        fetch.push_back({static_cast<unsigned>(pn), static_cast<unsigned>(slot[v])});
+                    }
+                }
+                else if (ver > visit[v])
+                {
+                    give(v);
+                    if (ver < 0)
+                        fetch.push_back({static_cast<unsigned>(pn), static_cast<unsigned>(slot[v])});
+                    else
+                        halo.push_back({static_cast<unsigned>(pn), static_cast<unsigned>(slot[v]) | static_cast<unsigned>(ver) << 16});
+                    visit[v] = ver;
+                }
+                codes[at0 + 4 * (st * (q / 4) + l) + q % 4] = static_cast<unsigned short>(slot[v]);
+                entSrc[at0 + vg * (st * (q / vg) + l) + q % vg] = e;
+            }
+        }
+        for (int i = 0; i < m; ++i) give(H.posCell[items[a + i].p] - c0);
+        const size_t itemsAt = 16 * static_cast<size_t>(nSl), fetchAt = itemsAt + 256 * static_cast<size_t>(nSl);
+        const size_t haloAt = fetchAt + (fetch.size() + 1) / 2 * 16, codesAt = haloAt + (halo.size() + 1) / 2 * 16;
+        const size_t metaBytes = codesAt + (2 * static_cast<size_t>(nEnt) + 15) / 16 * 16;
+        const size_t valsAt = metaBytes + 64 * static_cast<size_t>(nSl) * vb, srcBytesAt = valsAt + nEnt * vb;
+        // (offsets within a chunk count 8 bytes in 16 bits)
+        if (P.slots > k::kFlowMaxSlots || srcBytesAt + 32 * static_cast<size_t>(nSl) * vb > 8 * 65535u ||
+            fetch.size() > 65535u || halo.size() > 65535u)
+        {
+            P.ok = false;
+            break;
+        }
+        const size_t at = P.meta.size();
+        P.meta.resize(at + metaBytes, 0);
+        unsigned char* M = P.meta.data() + at;
+        for (int s = 0; s < nSl; ++s)
+        {
+            k::FlowSlice h{};
+            h.items8 = static_cast<unsigned short>((itemsAt + 256 * static_cast<size_t>(s)) / 8);
+            h.codes8 = static_cast<unsigned short>((codesAt + 2 * static_cast<size_t>(first[s])) / 8);
+            h.vals8 = static_cast<unsigned short>((valsAt + vb * static_cast<size_t>(first[s])) / 8);
+            h.diag8 = static_cast<unsigned short>((metaBytes + 64 * static_cast<size_t>(s) * vb) / 8);
+            h.src8 = static_cast<unsigned short>((srcBytesAt + 32 * static_cast<size_t>(s) * vb) / 8);
+            h.width = static_cast<unsigned char>(width[s]);
+            h.stride = static_cast<unsigned char>(k::flowStride(m, s));
+            h.count = static_cast<unsigned char>(std::min(32, m - 32 * s));
+            std::memcpy(M + 16 * static_cast<size_t>(s), &h, sizeof(h));
+        }
+        for (int i = 0; i < m; ++i)
+        {
+            const ItemRef& it = items[a + i];
+            const int c = H.posCell[it.p];
+            const Pair w{static_cast<unsigned>(it.p),
+                         static_cast<unsigned>(slot[c - c0]) | static_cast<unsigned>(it.q) << 16 |
+                             (it.out ? 0x40000000u : 0u) | (it.q == S - 1 ? 0x80000000u : 0u)};
+            std::memcpy(M + itemsAt + 8 * static_cast<size_t>(i), &w, 8);
+        }
+        if (!fetch.empty()) std::memcpy(M + fetchAt, fetch.data(), 8 * fetch.size());
+        if (!halo.empty()) std::memcpy(M + haloAt, halo.data(), 8 * halo.size());
+        if (nEnt) std::memcpy(M + codesAt, codes.data(), 2 * static_cast<size_t>(nEnt));
+        k::FlowRec& r = P.rec[j];
+        r.meta16 = static_cast<int>(at / 16);
+        r.metaBytes = static_cast<int>(metaBytes);
+        const long long nVal = 64LL * nSl + nEnt;
+        r.val16 = static_cast<int>(valAt * static_cast<long long>(vb) / 16);
+        r.valBytes = static_cast<int>(nVal * static_cast<long long>(vb));
+        r.m = m;
+        r.nSlices = nSl;
+        r.items8 = static_cast<int>(itemsAt / 8);
+        r.fetch8 = static_cast<int>(fetchAt / 8);
+        r.halo8 = static_cast<int>(haloAt / 8);
+        r.counts = static_cast<int>(static_cast<unsigned>(fetch.size()) | static_cast<unsigned>(halo.size()) << 16);
+        valAt += nVal;
+    }
+    for (int g : ghostCell) X.localOf[g] = -1;
+}
+
+// Places a rank's chunks in a ring of `ring` bytes; false when two chunks do not fit together.
+bool placeInRing(std::vector<k::FlowRec>& rec, size_t ring, size_t vb)
+{
+    std::vector<std::pair<size_t, size_t>> at(rec.size());
+    size_t headAt = 0;
+    for (size_t j = 0; j < rec.size(); ++j)
+    {
+        k::FlowRec& r = rec[j];
+        const size_t need = static_cast<size_t>(r.metaBytes) + r.valBytes + 32 * static_cast<size_t>(r.nSlices) * vb;
+        if (need > ring) return false;
+        if (headAt + need > ring) headAt = 0;
+        at[j] = {headAt, headAt + need};
+        int freeAfter = static_cast<int>(j) - k::kFlowDepth;
+        for (int i = static_cast<int>(j) - 1; i > freeAfter && i >= 0; --i)
+            if (at[i].first < at[j].second && at[j].first < at[i].second)
+            {
+                freeAfter = i;
+                break;
+            }
+        // chunk j is staged while chunk j - 1 is computed
+        if (freeAfter > static_cast<int>(j) - 2) return false;
+        r.ringOff = static_cast<int>(headAt);
+        r.freeAfter = freeAfter;
+        headAt += need;
+    }
+    return true;
+}
+
+}  // namespace
+
+void flowParallel(int n, const std::function<void(int, int)>& body)
+{
+    // a loop within a loop runs on its own thread: the outer one has the cores
+    static thread_local bool inside = false;
+    const int hw = static_cast<int>(std::max(1u, std::thread::hardware_concurrency()));
+    const int nt = inside ? 1 : std::min(n, std::min(hw, kFlowThreads));
+    std::atomic<int> next{0};
+    std::vector<std::exception_ptr> bad(std::max(nt, 1));
+    auto work = [&](int w) {
+        const bool was = inside;
+        inside = true;
+        try
+        {
+            for (int i = next++; i < n; i = next++) body(i, w);
+        }
+        catch (...)
+        {
+            bad[w] = std::current_exception();
+            next = n;
+        }
+        inside = was;
+    };
+    std::vector<std::thread> th;
+    try
+    {
+        for (int w = 1; w < nt; ++w) th.emplace_back(work, w);
+    }
+    catch (...)
+    {
+        // no more threads to be had: the ones that started, and this one, do the work
+    }
+    work(0);
+    for (auto& x : th) x.join();
+    for (auto& e : bad)
+        if (e) std::rethrow_exception(e);
+}
+
+// T_s(c) of every item (flow_kernels.cuh): the combined DAG of pipe_kernels.cuh with `weight` steps
+// across a face between two ranks.
+//
+// Symmetric sweeps (gaussSeidelSweeps' symmetric variant) visit a cell twice a sweep, forward then back.
+// The backward walk's bPrime is the source less the terms of the faces the cell is the neighbour of, in face
+// order, with the forward values, and the walk subtracts its own faces' terms ascending: the row's terms in
+// the row's order again. So a backward visit q is the same row reading its lower neighbours at visit q - 1
+// and its upper ones at visit q.
+std::vector<int> flowSteps(const FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps)
+{
+    const int S = symmetric ? 2 * nSweeps : nSweeps;
+    const size_t n = static_cast<size_t>(H.n);
+    std::vector<int> T(static_cast<size_t>(S) * n, 0);
+    std::vector<unsigned char> cross(R > 1 ? H.nF : 0);
+    if (R > 1)
+        for (int f = 0; f < H.nF; ++f) cross[f] = flowRank(H.lower[f], H.n, R) != flowRank(H.upper[f], H.n, R);
+    const int extra = weight - 1;
+    auto at = [&](int f) { return 1 + (R > 1 && cross[f] ? extra : 0); };
+    for (int s = 0; s < S; ++s)
+    {
+        int* cur = T.data() + s * n;
+        const int* prev = s > 0 ? T.data() + (s - 1) * n : nullptr;
+        const bool back = symmetric && (s & 1);
+        // the cell itself and the neighbours the walk has not reached: their previous visit
+        if (prev)
+        {
+            for (size_t c = 0; c < n; ++c) cur[c] = prev[c] + 1;
+            for (int f = 0; f < H.nF; ++f)
+            {
+                const int c = back ? H.upper[f] : H.lower[f], o = back ? H.lower[f] : H.upper[f];
+                cur[c] = std::max(cur[c], prev[o] + at(f));
+            }
+        }
+        // those it has: this visit (faces are sorted by owner, so in this order each is final when read)
+        if (!back)
+            for (int f = 0; f < H.nF; ++f) cur[H.upper[f]] = std::max(cur[H.upper[f]], cur[H.lower[f]] + at(f));
+        else
+            for (int f = H.nF - 1; f >= 0; --f) cur[H.lower[f]] = std::max(cur[H.lower[f]], cur[H.upper[f]] + at(f));
+    }
+    nSteps = T.empty() ? 0 : *std::max_element(T.begin(), T.end()) + 1;
+    return T;
+}
+
+bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb, FlowProgram& F)
+{
+    if (H.n == 0 || R < 1 || R > H.n || S < 1 || S > k::kFlowMaxVisits) return false;
+    H.crosses = R > 1;
+    F.prog.clear();
+    F.prog.resize(R);
+    std::vector<RankScratch> scratch(kFlowThreads);
+    flowParallel(R, [&](int r, int w) {
+        buildRank(H, T, S, nSteps, flowBegin(r, H.n, R), flowBegin(r + 1, H.n, R), vb, scratch[w], F.prog[r]);
+    });
+    F.slots = 1;
+    F.metaBytes = F.nVal = 0;
+    for (const RankProgram& P : F.prog)
+    {
+        if (!P.ok) return false;
+        F.slots = std::max(F.slots, P.slots);
+        F.metaBytes += P.meta.size();
+        F.nVal += P.src.size();
+    }
+    const size_t ringAt = k::flowRingAt(F.slots, vb);
+    if (ringAt + 3 * kFlowChunkBytes > kFlowSmem) return false;
+    if (F.metaBytes / 16 > 0x7fffffffull || F.nVal * vb / 16 > 0x7fffffffull) return false;
+    F.chunkStart.assign(static_cast<size_t>(R) + 1, 0);
+    F.rec.clear();
+    size_t metaAt = 0, valAt = 0;
+    for (int r = 0; r < R; ++r)
+    {
+        RankProgram& P = F.prog[r];
+        if (!placeInRing(P.rec, kFlowSmem - ringAt, vb)) return false;
+        for (k::FlowRec x : P.rec)
+        {
+            x.meta16 += static_cast<int>(metaAt / 16);
+            x.val16 += static_cast<int>(valAt * vb / 16);
+            F.rec.push_back(x);
+        }
+        F.chunkStart[r + 1] = static_cast<int>(F.rec.size());
+        metaAt += P.meta.size();
+        valAt += P.src.size();
+    }
+    return true;
+}
+
+}  // namespace b2g

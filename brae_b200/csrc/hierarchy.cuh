@@ -94,6 +94,23 @@ struct PipeSchedule
     DBuf<unsigned> progress;    // [ranks][kProgressStride]
 };
 
+// One smoothing call's sweeps of a level as a data flow between `ranks` CTAs (flow_kernels.cuh), for
+// values of one size: every rank's chunks with their place in the shared-memory ring, and where each
+// chunk's values come from. A matrix keeps the values themselves (VCycleData::flows).
+struct FlowSchedule
+{
+    long long id = 0;             // names the schedule in the matrices' value buffers
+    int sweeps = 0;
+    int ranks = 0;
+    int nSteps = 0;
+    int slots = 0;                // value slots of a CTA
+    long long nVal = 0;
+    DBuf<int> chunkStart;         // [ranks + 1]
+    DBuf<int4> rec;               // [chunks][3] k::FlowRec
+    DBuf<unsigned char> meta;     // the chunks' meta blobs
+    DBuf<int> src;                // [nVal] row entry or diagonal of each value (k::flowValues)
+};
+
 // The dynamic shared memory of a pipelined launch in values of valueBytes (pipe.cu): the rank's
 // slots in the shared-memory forms, the rank's step table in the grid form.
 size_t pipeSmemBytes(const PipeSchedule& P, size_t valueBytes);
@@ -104,9 +121,11 @@ size_t pipeSmemBytes(const PipeSchedule& P, size_t valueBytes);
 // schedule, or the sweep-by-sweep launches when those are faster.
 struct PipeChoice
 {
-    int mode = 0;                        // 0 sweep by sweep, 1 the pipelined launch, 2 items
+    int mode = 0;                        // 0 sweep by sweep, 1 the pipelined launch, 2 items, 3 the data flow
     std::unique_ptr<PipeSchedule> sched; // mode 1 (shared memory, or the grid form)
     std::unique_ptr<GsSchedule> items;   // mode 2: the multi-part sweep over (sweep, cell) items
+    std::unique_ptr<FlowSchedule> flow;  // mode 3
+    float msFlow = 0.f;   // per smoothing call, the best data-flow launch (0: not tried)
     float msPipe = 0.f;   // per smoothing call, the best shared-memory shape (0: none fits)
     float msItems = 0.f;  // per smoothing call, the item schedule (0: not built)
     float msSweeps = 0.f; // per smoothing call, sweep by sweep
@@ -145,11 +164,11 @@ struct Colouring
     int cluster = 0;
     int block = 256;
     float msPerSweep = 0.f;
-    // per smoothing call of nSweeps sweeps (key nSweeps * 2 + symmetric): the pipelined shared-memory
-    // launch (pipe.cu) whose steps are the colours, kept where it measured faster than the shape above
+    // per smoothing call of nSweeps sweeps (key nSweeps * 2 + symmetric): the data-flow launch
+    // (flow_kernels.cuh) whose steps are the colours, kept where it measured faster than the shape above
     struct Pipe
     {
-        std::unique_ptr<PipeSchedule> sched;
+        std::unique_ptr<FlowSchedule> flow;
         bool use = false;
         float msPipe = 0.f, msColours = 0.f;  // per smoothing call, as measured
     };
@@ -204,6 +223,10 @@ struct LevelAddr
     PairLevel pair;         // the coupled pair, if the mesh carries one (nFaces 0 otherwise)
     // pipelined smoothing calls, keyed by sweeps * 16 + the value size (built on first use)
     std::map<int, PipeChoice> pipe;
+    // the batched form's launches of this level, by {key above, ranks}
+    std::map<std::pair<int, int>, std::unique_ptr<FlowSchedule>> flowBatch;
+    // symmetric smoothing calls as one data-flow launch, by the same key (null: none for the level)
+    std::map<int, std::unique_ptr<FlowSchedule>> flowSym;
     // the one-CTA pipelined schedule by the same key (the batched form's; null: the level does not fit)
     std::map<int, std::unique_ptr<PipeSchedule>> pipeOne;
     // The one-block resident Gauss-Seidel sweep of a small one-part level (solver.cu gsResident),

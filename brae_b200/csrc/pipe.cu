@@ -9,6 +9,7 @@
 // smooth_solver_cpp.cu:87-166 (forward only for GaussSeidel, :144), called nSweeps times per
 // smoothing call by GaussSeidelSmoother::smooth (gamg_solver_cpp.cu:234-317).
 
+#include "flow.cuh"
 #include "pipe_kernels.cuh"
 #include "solver.cuh"
 
@@ -19,6 +20,7 @@
 namespace b2g {
 namespace {
 
+constexpr int kMcFlowCells = 600000;  // the largest level whose colours are tried as a data flow
 constexpr size_t kPipeSmemCap = 220 * 1024;  // dynamic shared memory of one rank: its psi slots and step table
 
 // The level's addressing on the host, as the schedule builder reads it.
@@ -166,12 +168,12 @@ std::unique_ptr<PipeSchedule> assemble(const LevelHost& H, const std::vector<int
     return P;
 }
 
-// The multicolour smoother's sweeps as a pipelined schedule: item (sweep s, cell c) runs at step
-// s * stepsPerSweep + k for a cell of colour k; symmetric sweeps visit the colours forward then back,
-// each cell twice a sweep. No two cells of a colour share a face, so a step's items are independent,
-// and each row reads the values the colour-by-colour sweep gives it. Null when a cell has no colour.
-std::unique_ptr<PipeSchedule> colourSchedule(const LevelHost& H, const Colouring& C, const std::vector<int>& rowPos,
-                                             int nSweeps, bool symmetric, int R, cudaStream_t s)
+// The multicolour smoother's sweeps as steps: item (sweep s, cell c) runs at step s * stepsPerSweep + k for a
+// cell of colour k; symmetric sweeps visit the colours forward then back, each cell twice a sweep. No two cells
+// of a colour share a face, so a step's items are independent, and each row reads the values the
+// colour-by-colour sweep gives it. Empty when a cell has no colour.
+std::vector<int> colourSteps(const FlowLevel& H, const Colouring& C, const std::vector<int>& rowPos, int nSweeps,
+                             bool symmetric, int& visits, int& nSteps)
 {
     const int n = H.n;
     std::vector<int> colourOf(n, -1);
@@ -179,11 +181,12 @@ std::unique_ptr<PipeSchedule> colourSchedule(const LevelHost& H, const Colouring
         for (int r = C.colourStart[k]; r < C.colourStart[k + 1]; ++r)
             if (rowPos[r] >= 0) colourOf[H.posCell[rowPos[r]]] = k;
     for (int c = 0; c < n; ++c)
-        if (colourOf[c] < 0) return nullptr;
+        if (colourOf[c] < 0) return {};
     const int per = symmetric ? 2 : 1;
     const int stepsPerSweep = per * C.nColours;
-    const int S = nSweeps * per;
-    std::vector<int> T(static_cast<size_t>(S) * n);
+    visits = nSweeps * per;
+    nSteps = nSweeps * stepsPerSweep;
+    std::vector<int> T(static_cast<size_t>(visits) * n);
     for (int sw = 0; sw < nSweeps; ++sw)
         for (int c = 0; c < n; ++c)
         {
@@ -191,7 +194,7 @@ std::unique_ptr<PipeSchedule> colourSchedule(const LevelHost& H, const Colouring
             T[static_cast<size_t>(sw * per) * n + c] = sw * stepsPerSweep + k;
             if (symmetric) T[static_cast<size_t>(sw * per + 1) * n + c] = sw * stepsPerSweep + 2 * C.nColours - 1 - k;
         }
-    return assemble(H, T, S, nSweeps * stepsPerSweep, R, sizeof(float), s);
+    return T;
 }
 
 template <class T>
@@ -504,7 +507,30 @@ void Matrix::ensurePipe(int level, int nSweeps)
     });
     checkDeviceError();
     float best = C.msSweeps;
-    if (L.nCells <= k::kPipeMaxRanks * static_cast<int>(kPipeSmemCap / sizeof(T)))
+    {
+        // the data-flow launch on a few CTA counts
+        FlowLevel H = flowDownload(L, stream);
+        for (const FlowShape& f : flowShapes(L.nCells))
+        {
+            int nSteps = 0;
+            const std::vector<int> steps = flowSteps(H, nSweeps, false, f.ranks, f.weight, nSteps);
+            std::unique_ptr<FlowSchedule> F = buildFlow(H, steps, nSweeps, nSteps, f.ranks, sizeof(T), stream);
+            if (!F) continue;
+            const long long id = F->id;
+            const float ms = timeIt([&] { flowLaunch<T>(level, *F, x.p, b.p); });
+            checkDeviceError();
+            if (C.mode != 3 || ms < C.msFlow)
+            {
+                C.msFlow = ms;
+                if (C.flow) data<T>().flows.erase(C.flow->id);
+                C.flow = std::move(F);
+                C.mode = 3;
+            }
+            else
+                data<T>().flows.erase(id);
+        }
+    }
+    if (C.mode != 3 && L.nCells <= k::kPipeMaxRanks * static_cast<int>(kPipeSmemCap / sizeof(T)))
     {
         const LevelHost H = download(L, stream);
         int nSteps = 0;
@@ -524,7 +550,7 @@ void Matrix::ensurePipe(int level, int nSweeps)
             }
         }
     }
-    if (L.gs.nParts > 1)
+    if (C.mode != 3 && L.gs.nParts > 1)
     {
         // the grid form: one CTA per SM, or per two
         const LevelHost H = download(L, stream);
@@ -596,20 +622,25 @@ void Matrix::ensurePipe(int level, int nSweeps)
     B2G_CUDA(cudaStreamSynchronize(stream));
 }
 
-// The multicolour smoothing call of nSweeps sweeps on `level` as one pipelined launch over the colours
-// (colourSchedule), on one CTA or a cluster of 2-16, against the tuned colour-by-colour shape
-// (Matrix::tuneMulticolour): the faster is kept. Both compute every row with the same fused
-// multiply-adds in the same order on the same values, so the choice changes the time only.
+// The multicolour smoothing call of nSweeps sweeps on `level` as one data-flow launch whose steps are the
+// colours (colourSteps), against the tuned colour-by-colour shape (Matrix::tuneMulticolour): the faster is
+// kept. Both compute every row with the same fused multiply-adds in the same order on the same values, so the
+// choice changes the time only. Tried with a CTA per chunk of a colour's rows (k::kFlowTeam warps), where a step
+// is one chunk and a hand-over, and with twice as many. Above kMcFlowCells the colours are bound by bandwidth and
+// the launch per colour, which reads each value once from L2, wins.
 void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
 {
     LevelAddr& L = mesh->lev[level];
     Colouring& C = L.mc;
     const int key = nSweeps * 2 + (symmetric ? 1 : 0);
-    if (C.pipe.count(key)) return;
+    auto known = C.pipe.find(key);
+    if (known != C.pipe.end())
+    {
+        if (known->second.use) flowValuesOf<float>(level, *known->second.flow);
+        return;
+    }
     Colouring::Pipe& M = C.pipe[key];
-    if (nSweeps < 1 || L.nCells == 0 || C.nColours == 0 || !C.tuned) return;
-    if (L.nCells > k::kPipeMaxRanks * static_cast<int>(kPipeSmemCap / sizeof(float))) return;
-    allowPipeSmem<float>();
+    if (nSweeps < 1 || L.nCells == 0 || C.nColours == 0 || !C.tuned || L.nCells > kMcFlowCells) return;
     float* x = level == 0 ? w32.p : v32.corr[level - 1].p;
     float* b = level == 0 ? r32.p : v32.src[level - 1].p;
     // scratch vectors of the level (the times do not depend on the values)
@@ -619,38 +650,40 @@ void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
     B2G_CUDA(cudaEventCreate(&e0));
     B2G_CUDA(cudaEventCreate(&e1));
     const long long l0 = launches;
-    auto timeIt = [&](auto&& launch) {
-        launch();  // warm
-        B2G_CUDA(cudaEventRecord(e0, stream));
-        for (int i = 0; i < 3; ++i) launch();
-        B2G_CUDA(cudaEventRecord(e1, stream));
-        B2G_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        B2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        return ms / 3.f;
-    };
-    M.msColours = timeIt([&] { mcLaunch(level, C.fused, C.cluster, C.block, x, b, nSweeps, false, symmetric); });
-    checkDeviceError();
-    const LevelHost H = download(L, stream);
-    const std::vector<int> rowPos = C.pos.download(stream);
+    mcLaunch(level, C.fused, C.cluster, C.block, x, b, nSweeps, false, symmetric);  // warm
+    B2G_CUDA(cudaEventRecord(e0, stream));
+    for (int i = 0; i < 3; ++i) mcLaunch(level, C.fused, C.cluster, C.block, x, b, nSweeps, false, symmetric);
+    B2G_CUDA(cudaEventRecord(e1, stream));
+    B2G_CUDA(cudaEventSynchronize(e1));
+    B2G_CUDA(cudaEventElapsedTime(&M.msColours, e0, e1));
+    M.msColours /= 3.f;
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    FlowLevel H = flowDownload(L, stream);
+    int visits = 0, nSteps = 0;
+    const std::vector<int> T = colourSteps(H, C, C.pos.download(stream), nSweeps, symmetric, visits, nSteps);
     float best = M.msColours;
-    for (int R : {1, 2, 4, 8, 16})
+    const int per = 32 * k::kFlowTeam * C.nColours;
+    const int sms = DeviceInfo::get().numSMs, one = std::min(sms, (L.nCells + per - 1) / per);
+    for (int R : {one, std::min(sms, 2 * one)})
     {
-        std::unique_ptr<PipeSchedule> P = colourSchedule(H, C, rowPos, nSweeps, symmetric, R, stream);
-        if (!P) continue;
-        if (R > 1 && !pipeClusterFits<float>(R, pipeSmemBytes(*P, sizeof(float)), stream, true)) continue;
-        const float ms = timeIt([&] { pipeLaunch<float>(level, *P, x, b, true); });
+        if (T.empty()) break;
+        std::unique_ptr<FlowSchedule> F = buildFlow(H, T, visits, nSteps, R, sizeof(float), stream);
+        if (!F) continue;
+        const float ms = flowTime<float>(level, *F, x, b, true);
         if (M.msPipe == 0.f || ms < M.msPipe) M.msPipe = ms;
         if (ms < best)
         {
             best = ms;
-            M.sched = std::move(P);
+            if (M.flow) v32.flows.erase(M.flow->id);
+            M.flow = std::move(F);
             M.use = true;
         }
+        else
+            v32.flows.erase(F->id);
+        if (one == 1 || one == sms) break;
     }
     launches = l0;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     B2G_CUDA(cudaStreamSynchronize(stream));
     checkDeviceError();
 }
@@ -665,6 +698,7 @@ void Matrix::refreshItems()
         {
             if (kv.first % 16 != static_cast<int>(sizeof(T))) continue;
             if (kv.second.mode == 2) itemBuffers<T>(lv, *kv.second.items);
+            if (kv.second.mode == 3) flowValuesOf<T>(lv, *kv.second.flow);
         }
 }
 
@@ -691,6 +725,11 @@ bool Matrix::pipeSweeps(int level, T* psiL, const T* src, int nSweeps)
     if (C.mode == 2)
     {
         itemsLaunch<T>(level, *C.items, psiL, src);
+        return true;
+    }
+    if (C.mode == 3)
+    {
+        flowLaunch<T>(level, *C.flow, psiL, src);
         return true;
     }
     return false;

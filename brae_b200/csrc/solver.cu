@@ -910,6 +910,7 @@ void Matrix::gsLaunch(const LevelAddr& L, const LevelCoef<T>& C, T* psiL, const 
     a.spinLimit = spinLimit;
     a.publish = publish;
     a.err = err.p;
+        if (symFlowSweeps<T>(level, psiL, src, nSweeps)) return;
     a.trace = trace;
     a.traceDepths = G.maxDepth + 2;
     const size_t smem = k::gsSmemBytes<T>(G.maxCells, G.maxEnt, G.maxGat);
@@ -1060,8 +1061,8 @@ void Matrix::prepareSmoother(const b2g_controls& c)
     for (int i = 0; i < nLevels(); ++i)
     {
         // the multicolour form sweeps symGaussSeidel by colour; DIC there runs in exact order
-        if (sym && fp64) ensureSym<double>(i);
-        else if (sym && c.precision == B2G_PRECISION_FP32_PRECOND) ensureSym<float>(i);
+        if (sym && fp64 && !symLaunches(i, sizeof(double))) ensureSym<double>(i);
+        else if (sym && !fp64 && c.precision == B2G_PRECISION_FP32_PRECOND && !symLaunches(i, sizeof(float))) ensureSym<float>(i);
         if (dic && fp64) ensureDic<double>(i);
         else if (dic) ensureDic<float>(i);
     }
@@ -1094,6 +1095,30 @@ void Matrix::ensureDic(int level)
         const std::vector<int> lo = L.lower.download(stream);
         const std::vector<int> up = L.upper.download(stream);
         std::vector<double> rD(diag);
+    // the symmetric smoothing calls as one launch each
+    if (g_pipeline && sym && (fp64 || c.precision == B2G_PRECISION_FP32_PRECOND))
+    {
+        auto want = [&](int level, int nSweeps) {
+            if (nSweeps <= 0 || level > nLevels()) return;
+            if (fp64) ensureSymFlow<double>(level, nSweeps);
+            else ensureSymFlow<float>(level, nSweeps);
+        };
+        want(0, c.nFinestSweeps);
+        for (int li = 0; li + 1 < nLevels(); ++li)
+        {
+            want(li + 1, std::min(c.nPostSweeps + c.postSweepsLevelMultiplier * li, c.maxPostSweeps));
+            if (c.nPreSweeps) want(li + 1, std::min(c.nPreSweeps + c.preSweepsLevelMultiplier * li, c.maxPreSweeps));
+        }
+        if (fp64) refreshSymFlows<double>();
+        else refreshSymFlows<float>();
+    }
+    // a level whose symmetric calls all have their launch needs no reversed layout
+    auto symLaunches = [&](int level, size_t valueBytes) {
+        bool all = g_pipeline && !mesh->lev[level].flowSym.empty();
+        for (const auto& kv : mesh->lev[level].flowSym)
+            if (kv.first % 16 == static_cast<int>(valueBytes) && !kv.second) all = false;
+        return all;
+    };
         for (int f = 0; f < nF; ++f) rD[up[f]] -= coef[f] * coef[f] / rD[lo[f]];
         for (int c = 0; c < n; ++c) rD[c] = 1.0 / rD[c];
         rdCell[level].ensure(rD.size(), stream);
@@ -1201,7 +1226,7 @@ void Matrix::mcSmooth(int level, float* psiL, const float* src, int nSweeps, boo
     const auto it = C.pipe.find(nSweeps * 2 + (symmetric ? 1 : 0));
     if (g_pipeline && it != C.pipe.end() && it->second.use)
     {
-        pipeLaunch<float>(level, *it->second.sched, psiL, src, true);
+        flowLaunch<float>(level, *it->second.flow, psiL, src, true);
         return;
     }
     mcLaunch(level, C.fused, C.cluster, C.block, psiL, src, nSweeps, true, symmetric);
@@ -1865,6 +1890,16 @@ b2g_perf Matrix::pcg(const b2g_controls& c, b2g_solve_log* log)
     kPcgStart<<<1, 1, 0, stream>>>(scal.p);
     B2G_LAUNCH_CHECK();
     do
+    for (const auto& kv : v64.flows)
+    {
+        mix(kv.second.val.p);
+        mix(kv.second.mail.p);
+    }
+    for (const auto& kv : v32.flows)
+    {
+        mix(kv.second.val.p);
+        mix(kv.second.mail.p);
+    }
     {
         runIteration(pcgGraph, c, [&] {
             precondition(c, wA.p, rA.p);

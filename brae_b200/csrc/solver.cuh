@@ -2,6 +2,7 @@
 #pragma once
 
 #include "coarsest_kernels.cuh"
+#include "flow_kernels.cuh"
 #include "gs_kernels.cuh"
 #include "hierarchy.cuh"
 #include "ldu_kernels.cuh"
@@ -66,6 +67,16 @@ struct VCycleData
         long long gen = -1;
     };
     std::map<std::pair<int, int>, ItemBuffers> items;
+    // data-flow schedules (flow.cu), by their id: this matrix's values with the coefficient generation
+    // they were filled for, and its mailboxes
+    struct FlowBuffers
+    {
+        DBuf<T> val;
+        DBuf<unsigned char> mail;   // {value, tag} by position, and the launch counter with the ranks that
+        DBuf<unsigned> ctl;         // have finished (more than one rank)
+        long long gen = -1;
+    };
+    std::map<long long, FlowBuffers> flows;
     // FP32 form only: dense Cholesky of the coarsest level
     bool built = false;
 };
@@ -194,6 +205,15 @@ struct Matrix
     template <class T> typename VCycleData<T>::ItemBuffers& itemBuffers(int level, const GsSchedule& G);
     template <class T> void itemsLaunch(int level, const GsSchedule& G, T* psi, const T* source);
     template <class T> void refreshItems();
+    // the data-flow launch of a smoothing call (flow.cu)
+    template <class T> const T* flowValuesOf(int level, const FlowSchedule& F);
+    template <class T> k::FlowArgs<T> flowArgs(int level, const FlowSchedule& F, T* psi, const T* source);
+    template <class T> void flowLaunch(int level, const FlowSchedule& F, T* psi, const T* source, bool fma = false);
+    template <class T> bool flowForced(int level, T* psi, const T* source, int nSweeps, bool symmetric, int ranks, int weight, float* ms);
+    template <class T> float flowTime(int level, const FlowSchedule& F, T* psi, const T* source, bool fma = false);
+    template <class T> void ensureSymFlow(int level, int nSweeps);
+    template <class T> bool symFlowSweeps(int level, T* psi, const T* source, int nSweeps);
+    template <class T> void refreshSymFlows();
     // the coarsest level's dense Cholesky factor (FP32-preconditioned forms, coarsestDirect), made for
     // the current coefficients by ensureDense outside any capture
     DBuf<double> denseL;

@@ -76,6 +76,7 @@ def _load():
         "b2g_set_part_cells": (ip, [ip]),
         "b2g_level_grid_stall": (ip, [vp, ip, vp, vp, ip, ip, C.c_longlong]),
         "b2g_level_smooth_pipelined": (ip, [vp, ip, vp, vp, ip, ip]),
+        "b2g_level_smooth_flow": (ip, [vp, ip, vp, vp, ip, ip, ip, ip, C.c_longlong, C.POINTER(C.c_float)]),
         "b2g_level_pipe_shape": (ip, [vp, ip, ip, ip, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_float),
                                       C.POINTER(C.c_float), C.POINTER(C.c_float), C.POINTER(C.c_float),
                                       C.POINTER(C.c_float), C.POINTER(C.c_int)]),
@@ -157,7 +158,7 @@ EXPORTED = [
     "b2g_batch_launches", "b2g_batch_destroy", "b2g_mesh_set_pair", "b2g_mesh_level_pair",
     "b2g_gamg_solve_coupled", "b2g_matrix_create_coupled", "b2g_matrix_level_pair_coeffs", "b2g_matrix_gamg_solve",
     "b2g_matrix_set_coeffs", "b2g_matrix_level_timings", "b2g_level_smooth_stall", "b2g_set_sweep_pipeline",
-    "b2g_level_smooth_pipelined", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
+    "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
 ]
 
 
@@ -438,6 +439,15 @@ class Matrix:
     def smooth_pipelined(self, level, psi, source, n_sweeps, ranks):
         """n_sweeps sweeps in one pipelined launch on `ranks` CTAs (b2g_level_smooth_pipelined)."""
         _check(lib.b2g_level_smooth_pipelined(self.handle, level, _ptr(psi), _ptr(source), n_sweeps, ranks))
+
+    def smooth_flow(self, level, psi, source, n_sweeps, ranks, weight=1, stall_limit=0, timed=False,
+                    symmetric=False):
+        """n_sweeps sweeps in one data-flow launch on `ranks` CTAs (b2g_level_smooth_flow): the mean
+        milliseconds of a call if `timed`."""
+        ms = C.c_float()
+        _check(lib.b2g_level_smooth_flow(self.handle, level, _ptr(psi), _ptr(source), n_sweeps, int(symmetric), ranks, weight,
+                                         int(stall_limit), C.byref(ms) if timed else None))
+        return ms.value
 
     def grid_stall(self, level, psi, source, n_sweeps, ranks, spin_limit):
         """The grid form with no rank publishing its progress (b2g_level_grid_stall): the status name."""

@@ -398,6 +398,18 @@ B2G_API b2g_status b2g_level_grid_stall(b2g_matrix* m, int level, double* psi, c
  * when a grid-form wait gave up. For tests and tuning. */
 B2G_API b2g_status b2g_level_smooth_pipelined(b2g_matrix* m, int level, double* psi, const double* source,
                                               int nSweeps, int ranks);
+/* nSweeps exact Gauss-Seidel sweeps (symmetric 1: symGaussSeidel's) of `level` (device pointers, natural cell
+ * order) in ONE data-flow
+ * launch on `ranks` CTAs, whatever form the level's tuned choice would take: each CTA runs the items
+ * of one contiguous cell range in the combined order of the sweeps and takes the values of other ranges
+ * as they are handed over, which gives bit for bit the result of nSweeps sequential sweeps. `weight`:
+ * the steps a face between two CTAs counts in that order (the hand-over's time in steps). stallLimit
+ * above 0 (a test of the waits' limit): no CTA hands its values over and every wait gives up after that
+ * many polls; B2G_ERR_DEVICE_TIMEOUT then, with psi unspecified and the context still usable, where one
+ * CTA waits for another. *ms (may be NULL): after the call's own sweeps, the mean time of 3 of 4 more calls
+ * (psi then holds 5 * nSweeps sweeps). B2G_ERR_ARGUMENT when the level has no such schedule. For tests and tuning. */
+B2G_API b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const double* source, int nSweeps,
+                                         int symmetric, int ranks, int weight, long long stallLimit, float* ms);
 /* psi = A^-1 source on the coarsest level by its dense Cholesky factor (device pointers, natural
  * cell order): the direct coarsest solve the FP32-preconditioned forms take (coarsestDirect).
  * B2G_ERR_ARGUMENT when the level has more than 96 cells or is not positive definite. The factor of
