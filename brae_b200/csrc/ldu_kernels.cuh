@@ -8,6 +8,8 @@
 
 #include "b2g_common.cuh"
 
+#include <cooperative_groups.h>
+
 namespace b2g {
 namespace k {
 
@@ -260,6 +262,187 @@ __global__ void scaleUpdateAddProlong(int n, const T* __restrict__ sfp, const in
         const T corr = addRn(mulRn(sf, coarse[prolongP[c]]), divRn(subRn(source[c], mulRn(sf, Acf[c])), diag[c]));
         psi[c] = addRn(psi[c], corr);
     }
+}
+
+// THE WAY UP ONTO A SMALL LEVEL, IN ONE LAUNCH: prolong, Amul with the scaling's dots, the factor and the
+// update (prolongField, amulScaleDots, scaleFactor, scaleUpdate) on one thread-block cluster of C CTAs. The
+// four launches are bound by their latency on such a level (about 3 us each), not by bytes. A thread keeps
+// its cells' correction and product in registers between the two halves, so neither is stored; partial sums
+// go to CTA 0's shared memory. The sums have the shape of the separate kernels' -- a block sum per 256
+// cells, then one over those -- so the result is theirs bit for bit. Grid = the cluster; n <= C * kUpThreads *
+// kUpCells.
+constexpr int kUpThreads = 1024;
+constexpr int kUpCells = 2;
+constexpr int kUpMaxCtas = 16;
+template <class T>
+__global__ void __launch_bounds__(kUpThreads, 1) scaleProlongCluster(Rows<T> A, const int* __restrict__ prolongP,
+                                                                     const T* __restrict__ coarse,
+                                                                     const T* __restrict__ source, T* __restrict__ field)
+{
+    constexpr int kBlocks = kUpMaxCtas * kUpCells * (kUpThreads / 256);  // partial sums, at most
+    static_assert(kBlocks <= 256, "the final sum takes one partial a thread");
+    __shared__ T part[2 * kBlocks];    // CTA 0's: every 256 cells' sums
+    __shared__ T sh[2 * (kUpThreads / 32)];
+    __shared__ T sfS;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int rank = static_cast<int>(cluster.block_rank()), C = static_cast<int>(cluster.num_blocks());
+    const int nPart = (A.n + 255) / 256;
+    T fc[kUpCells], ac[kUpCells];
+#pragma unroll
+    for (int i = 0; i < kUpCells; ++i)
+    {
+        const int c = (i * C + rank) * kUpThreads + t;
+        T num = T(0), den = T(0);
+        if (c < A.n)
+        {
+            const T f = coarse[prolongP[c]];
+            T acc = mulRn(A.diag[c], f);
+            const int e1 = A.rowStart[c + 1];
+            // eight entries' loads in flight together; the sum in the row's order
+            for (int e = A.rowStart[c]; e < e1; e += 8)
+            {
+                int p[8];
+                T v[8], x[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (e + j < e1)
+                    {
+                        p[j] = A.col[e + j];
+                        v[j] = A.val[e + j];
+                    }
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (e + j < e1) p[j] = prolongP[p[j]];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (e + j < e1) x[j] = coarse[p[j]];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (e + j < e1) acc = addRn(acc, mulRn(v[j], x[j]));
+            }
+            if (A.pairStart)
+            {
+                const int k1 = A.pairStart[c + 1];
+                for (int k = A.pairStart[c]; k < k1; ++k)
+                    acc = subRn(acc, mulRn(A.pairVal[k], coarse[prolongP[A.pairCol[k]]]));
+            }
+            fc[i] = f;
+            ac[i] = acc;
+            num = addRn(num, mulRn(f, source[c]));
+            den = addRn(den, mulRn(f, acc));
+        }
+        // blockSum over 256 threads, two sums side by side
+        for (int o = 16; o > 0; o >>= 1)
+        {
+            num = addRn(num, __shfl_down_sync(0xffffffffu, num, o));
+            den = addRn(den, __shfl_down_sync(0xffffffffu, den, o));
+        }
+        if (lane == 0)
+        {
+            sh[2 * warp] = num;
+            sh[2 * warp + 1] = den;
+        }
+        __syncthreads();
+        if ((warp & 7) == 0)
+        {
+            T a = lane < 8 ? sh[2 * (warp + lane)] : T(0), b = lane < 8 ? sh[2 * (warp + lane) + 1] : T(0);
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                a = addRn(a, __shfl_down_sync(0xffffffffu, a, o));
+                b = addRn(b, __shfl_down_sync(0xffffffffu, b, o));
+            }
+            const int q = (i * C + rank) * (kUpThreads / 256) + warp / 8;
+            if (lane == 0 && q < nPart)
+            {
+                T* p0 = cluster.map_shared_rank(part, 0);
+                p0[2 * q] = a;
+                p0[2 * q + 1] = b;
+            }
+        }
+        __syncthreads();
+    }
+    cluster.sync();
+    if (rank == 0)
+    {
+        // scaleFactor's sum over the partials, one a thread of 256
+        T num = T(0), den = T(0);
+        if (t < nPart)
+        {
+            num = addRn(num, part[2 * t]);
+            den = addRn(den, part[2 * t + 1]);
+        }
+        if (t < 256)
+        {
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                num = addRn(num, __shfl_down_sync(0xffffffffu, num, o));
+                den = addRn(den, __shfl_down_sync(0xffffffffu, den, o));
+            }
+            if (lane == 0)
+            {
+                sh[2 * warp] = num;
+                sh[2 * warp + 1] = den;
+            }
+        }
+        __syncthreads();
+        if (warp == 0)
+        {
+            num = lane < 8 ? sh[2 * lane] : T(0);
+            den = lane < 8 ? sh[2 * lane + 1] : T(0);
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                num = addRn(num, __shfl_down_sync(0xffffffffu, num, o));
+                den = addRn(den, __shfl_down_sync(0xffffffffu, den, o));
+            }
+            num = __shfl_sync(0xffffffffu, num, 0);
+            den = __shfl_sync(0xffffffffu, den, 0);
+            const T v = Small<T>::vsmall;
+            const T sf = divRn(num, den >= T(0) ? addRn(den, v) : subRn(den, v));
+            if (lane < C) *cluster.map_shared_rank(&sfS, lane) = sf;
+        }
+    }
+    cluster.sync();
+    const T sf = sfS;
+#pragma unroll
+    for (int i = 0; i < kUpCells; ++i)
+    {
+        const int c = (i * C + rank) * kUpThreads + t;
+        if (c < A.n) field[c] = addRn(mulRn(sf, fc[i]), divRn(subRn(source[c], mulRn(sf, ac[i])), A.diag[c]));
+    }
+}
+
+// THE WAY DOWN THROUGH THE SMALL LEVELS, IN ONE LAUNCH: restrictField step after step by one block, which
+// waits out three dependent loads a step instead of a launch; the last level's correction is zeroed.
+constexpr int kChainSteps = 16;
+template <class T>
+struct RestrictChain
+{
+    int n;
+    const T* first;                       // the first step's fine field
+    const int* start[kChainSteps];        // per step: its coarse positions' fine positions
+    const int* list[kChainSteps];
+    T* coarse[kChainSteps];               // and the coarse field
+    int nCoarse[kChainSteps];
+    T* zero;                              // set to zero over the last level's cells
+};
+template <class T>
+__global__ void __launch_bounds__(1024) restrictChain(RestrictChain<T> a)
+{
+    const T* ff = a.first;
+    for (int i = 0; i < a.n; ++i)
+    {
+        for (int c = threadIdx.x; c < a.nCoarse[i]; c += 1024)
+        {
+            T acc = T(0);
+            const int e1 = a.start[i][c + 1];
+            for (int e = a.start[i][c]; e < e1; ++e) acc = addRn(acc, ff[a.list[i][e]]);
+            a.coarse[i][c] = acc;
+        }
+        __syncthreads();
+        ff = a.coarse[i];
+    }
+    for (int c = threadIdx.x; c < a.nCoarse[a.n - 1]; c += 1024) a.zero[c] = T(0);
 }
 
 // The residual between V-cycles, FUSED: Apsi = A*psi (Amul's order) and r = source - Apsi in one pass,

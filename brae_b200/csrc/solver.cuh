@@ -244,6 +244,8 @@ struct Matrix
                                    unsigned long long* trace = nullptr);
     template <class T> void smoothCall(int level, int smoother, T* psi, const T* source, int nSweeps,
                                        unsigned long long* trace);
+    int upCtas = 0;                           // the largest cluster scaleProlongCluster may take
+    template <class T> bool scaleProlonged(int level, const T* coarse, T* field, const T* source);
     template <class T> void scale(int level, T* field, T* Acf, const T* source);
     template <class T> void restrictTo(int step, const T* fine, T* coarse);
     template <class T> void prolongFrom(int step, const T* coarse, T* fine);
