@@ -1742,8 +1742,8 @@ void Batch::solve(const b2g_controls& c, const double* const* source, double* co
 
 namespace {
 
-// Batch streams are never destroyed. A batch builds layouts that its meshes keep (the one-CTA
-// pipelined schedules of pipeOneCta) on its own stream, and a mesh frees them on that stream when it
+// Batch streams are never destroyed. A batch builds layouts that its meshes keep (the data-flow
+// schedules of flowsForBatch) on its own stream, and a mesh frees them on that stream when it
 // goes, which may be long after the batch: a destroyed batch hands its stream back here, idle, for
 // the next batch on the same device.
 std::mutex g_batchStreamMu;

@@ -1,9 +1,9 @@
 // pipe.cu -- the pipelined multi-sweep Gauss-Seidel launch (pipe_kernels.cuh): its schedule, built
 // once per (level, sweep count, shape) on the host from the level's addressing, and the choice, by
 // measurement on the device, between its shapes (one CTA; a cluster of 2..16 CTAs; the grid form on
-// 148 or 74 resident CTAs), the item schedule (items.cu) and the sweep-by-sweep launches. The same
-// launch also runs the multicolour FP32 smoother's calls, with the colours as its steps
-// (colourSchedule, Matrix::ensureMcPipe).
+// 148 or 74 resident CTAs), the item schedule (items.cu), the sweep-by-sweep launches and the data-flow
+// launch (flow.cu), which nearly every level takes. Also the choice for the multicolour FP32 smoother's
+// calls, whose data-flow launch has the colours as its steps (colourSteps, Matrix::ensureMcPipe).
 //
 // Reference: the sweeps it reproduces are gaussSeidelSweeps, src/OpenFOAM/matrices/
 // smooth_solver_cpp.cu:87-166 (forward only for GaussSeidel, :144), called nSweeps times per
@@ -213,17 +213,6 @@ void allowPipeSmem()
     // then finds no such shape resident)
     if (cudaFuncSetAttribute(k::gsPipe<T, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         cudaGetLastError();
-    if constexpr (sizeof(T) == 4)
-    {
-        // the multicolour smoother's launches (the colours as steps)
-        B2G_CUDA(cudaFuncSetAttribute(k::gsPipe<T, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kPipeSmemCap)));
-        B2G_CUDA(cudaFuncSetAttribute(k::gsPipe<T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kPipeSmemCap)));
-        if (cudaFuncSetAttribute(k::gsPipe<T, true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess)
-            cudaGetLastError();
-    }
     done.fetch_or(bit);
 }
 
@@ -249,16 +238,11 @@ struct PipeLaunch
 };
 
 template <class T>
-bool pipeClusterFits(int ranks, size_t smem, cudaStream_t s, bool fma = false)
+bool pipeClusterFits(int ranks, size_t smem, cudaStream_t s)
 {
     PipeLaunch L(ranks, smem, s);
     int n = 0;
-    cudaError_t e;
-    if constexpr (sizeof(T) == 4)
-        e = fma ? cudaOccupancyMaxActiveClusters(&n, k::gsPipe<T, true, true>, &L.cfg)
-                : cudaOccupancyMaxActiveClusters(&n, k::gsPipe<T, true>, &L.cfg);
-    else
-        e = cudaOccupancyMaxActiveClusters(&n, k::gsPipe<T, true>, &L.cfg);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k::gsPipe<T, true>, &L.cfg);
     if (e != cudaSuccess)
     {
         cudaGetLastError();
@@ -319,7 +303,7 @@ k::PipeArgs<T> Matrix::pipeArgs(int level, const PipeSchedule& P, T* psiL, const
 }
 
 template <class T>
-void Matrix::pipeLaunch(int level, const PipeSchedule& P, T* psiL, const T* src, bool fma)
+void Matrix::pipeLaunch(int level, const PipeSchedule& P, T* psiL, const T* src)
 {
     const k::PipeArgs<T> a = pipeArgs<T>(level, P, psiL, src);
     const size_t smem = pipeSmemBytes(P, sizeof(T));
@@ -347,24 +331,6 @@ void Matrix::pipeLaunch(int level, const PipeSchedule& P, T* psiL, const T* src,
         launches += 2;
         return;
     }
-    if constexpr (sizeof(T) == 4)
-        if (fma)
-        {
-            // the multicolour smoother's arithmetic
-            if (P.ranks == 1)
-            {
-                k::gsPipe<T, false, true><<<1, k::kPipeBlock, smem, stream>>>(a);
-                B2G_LAUNCH_CHECK();
-            }
-            else
-            {
-                PipeLaunch C(P.ranks, smem, stream);
-                B2G_CUDA(cudaLaunchKernelEx(&C.cfg, k::gsPipe<T, true, true>, a));
-            }
-            ++launches;
-            return;
-        }
-    if (fma) fail(B2G_ERR_STATE, "b2g: the multicolour pipelined launch is FP32 only");
     if (P.ranks == 1)
     {
         k::gsPipe<T, false><<<1, k::kPipeBlock, smem, stream>>>(a);
@@ -770,53 +736,14 @@ bool Matrix::pipeForced(int level, T* psiL, const T* src, int nSweeps, int ranks
     return true;
 }
 
-const PipeSchedule* pipeOneCta(LevelAddr& L, int S, size_t valueBytes, cudaStream_t s)
-{
-    const int key = pipeKey(S, valueBytes);
-    auto it = L.pipeOne.find(key);
-    if (it != L.pipeOne.end()) return it->second.get();
-    std::unique_ptr<PipeSchedule>& P = L.pipeOne[key];
-    if (S < 1 || L.nCells == 0 || static_cast<size_t>(L.nCells) * valueBytes > kPipeSmemCap) return nullptr;
-    const LevelHost H = download(L, s);
-    int nSteps = 0;
-    const std::vector<int> Tsteps = combinedSteps(H, S, nSteps);
-    P = assemble(H, Tsteps, S, nSteps, 1, valueBytes, s);
-    return P.get();
-}
-
-// The batched one-CTA launch's shared-memory ceiling, once per device and value type.
-template <class T>
-static void allowPipeBatchSmem()
-{
-    static std::atomic<unsigned long long> done{0};
-    int dev = 0;
-    B2G_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done.load() & bit) return;
-    B2G_CUDA(cudaFuncSetAttribute(k::gsPipeBatch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(kPipeSmemCap)));
-    done.fetch_or(bit);
-}
-template <class T>
-void launchPipeBatch(const void* table, const int* caseOf, int n, size_t smem, const int* active, cudaStream_t s)
-{
-    allowPipeBatchSmem<T>();
-    k::gsPipeBatch<T><<<n, k::kPipeBlock, smem, s>>>(static_cast<const k::PipeArgs<T>*>(table), caseOf, active);
-    B2G_LAUNCH_CHECK();
-}
-template void launchPipeBatch<double>(const void*, const int*, int, size_t, const int*, cudaStream_t);
-template void launchPipeBatch<float>(const void*, const int*, int, size_t, const int*, cudaStream_t);
-
 template void Matrix::ensurePipe<double>(int, int);
 template bool Matrix::pipeForced<double>(int, double*, const double*, int, int);
 template void Matrix::ensurePipe<float>(int, int);
 template bool Matrix::pipeSweeps<double>(int, double*, const double*, int);
 template bool Matrix::pipeSweeps<float>(int, float*, const float*, int);
-template void Matrix::pipeLaunch<double>(int, const PipeSchedule&, double*, const double*, bool);
-template void Matrix::pipeLaunch<float>(int, const PipeSchedule&, float*, const float*, bool);
+template void Matrix::pipeLaunch<double>(int, const PipeSchedule&, double*, const double*);
+template void Matrix::pipeLaunch<float>(int, const PipeSchedule&, float*, const float*);
 template void Matrix::refreshItems<double>();
-template k::PipeArgs<double> Matrix::pipeArgs<double>(int, const PipeSchedule&, double*, const double*);
-template k::PipeArgs<float> Matrix::pipeArgs<float>(int, const PipeSchedule&, float*, const float*);
 template void Matrix::refreshItems<float>();
 template void Matrix::itemsLaunch<double>(int, const GsSchedule&, double*, const double*);
 

@@ -123,10 +123,6 @@ k::Rows<T> rowsOf(const LevelAddr& L, const LevelCoef<T>& C)
 
 // Whether smoothing calls may take the pipelined multi-sweep launch (pipe.cu; b2g_set_sweep_pipeline).
 extern bool g_pipeline;
-// The batched one-CTA pipelined launch (pipe.cu): n cases' levels, table = k::PipeArgs<T>[n] on the
-// device, caseOf[n] each entry's case (its `active` flag; active may be null).
-template <class T>
-void launchPipeBatch(const void* table, const int* caseOf, int n, size_t smem, const int* active, cudaStream_t s);
 
 struct Matrix
 {
@@ -198,7 +194,7 @@ struct Matrix
     // the pipelined multi-sweep launch (pipe.cu): the level's tuned choice, built on first use
     template <class T> void ensurePipe(int level, int nSweeps);
     template <class T> bool pipeSweeps(int level, T* psi, const T* source, int nSweeps);
-    template <class T> void pipeLaunch(int level, const PipeSchedule& P, T* psi, const T* source, bool fma = false);
+    template <class T> void pipeLaunch(int level, const PipeSchedule& P, T* psi, const T* source);
     template <class T> k::PipeArgs<T> pipeArgs(int level, const PipeSchedule& P, T* psi, const T* source);
     template <class T> bool pipeForced(int level, T* psi, const T* source, int nSweeps, int ranks);
     // an item schedule's launch (items.cu): its blobs filled for the current coefficients first
