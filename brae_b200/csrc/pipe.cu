@@ -168,32 +168,64 @@ std::unique_ptr<PipeSchedule> assemble(const LevelHost& H, const std::vector<int
     return P;
 }
 
-// The multicolour smoother's sweeps as steps: item (sweep s, cell c) runs at step s * stepsPerSweep + k for a
-// cell of colour k; symmetric sweeps visit the colours forward then back, each cell twice a sweep. No two cells
-// of a colour share a face, so a step's items are independent, and each row reads the values the
-// colour-by-colour sweep gives it. Empty when a cell has no colour.
+// The multicolour smoother's sweeps as steps on R ranks. The colours are an order of visits like the exact
+// sweeps' cell order, so an item runs one step after the last visit it reads, `weight` steps after one of another
+// rank: only the cells near a rank's border wait for a hand-over, the others run ahead into the next colours.
+// Every row still reads its neighbours of earlier colours at this visit and the others at the one before, as the
+// colour-by-colour sweep does. Symmetric sweeps visit the colours forward then back, each cell twice a sweep.
+// Empty when a cell has no colour.
 std::vector<int> colourSteps(const FlowLevel& H, const Colouring& C, const std::vector<int>& rowPos, int nSweeps,
-                             bool symmetric, int& visits, int& nSteps)
+                             bool symmetric, int R, int weight, int& visits, int& nSteps)
 {
     const int n = H.n;
-    std::vector<int> colourOf(n, -1);
+    std::vector<int> colourOf(n, -1), byColour, start(1, 0);
+    byColour.reserve(n);
     for (int k = 0; k < C.nColours; ++k)
+    {
         for (int r = C.colourStart[k]; r < C.colourStart[k + 1]; ++r)
-            if (rowPos[r] >= 0) colourOf[H.posCell[rowPos[r]]] = k;
+            if (rowPos[r] >= 0)
+            {
+                byColour.push_back(H.posCell[rowPos[r]]);
+                colourOf[byColour.back()] = k;
+            }
+        start.push_back(static_cast<int>(byColour.size()));
+    }
     for (int c = 0; c < n; ++c)
         if (colourOf[c] < 0) return {};
-    const int per = symmetric ? 2 : 1;
-    const int stepsPerSweep = per * C.nColours;
-    visits = nSweeps * per;
-    nSteps = nSweeps * stepsPerSweep;
+    visits = symmetric ? 2 * nSweeps : nSweeps;
+    std::vector<int> rank(R > 1 ? n : 0);
+    for (size_t c = 0; c < rank.size(); ++c) rank[c] = flowRank(static_cast<int>(c), n, R);
     std::vector<int> T(static_cast<size_t>(visits) * n);
-    for (int sw = 0; sw < nSweeps; ++sw)
-        for (int c = 0; c < n; ++c)
+    for (int v = 0; v < visits; ++v)
+    {
+        int* cur = T.data() + static_cast<size_t>(v) * n;
+        const int* prev = v > 0 ? cur - n : nullptr;
+        const bool back = symmetric && (v & 1);
+        for (int i = 0; i < C.nColours; ++i)
         {
-            const int k = colourOf[c];
-            T[static_cast<size_t>(sw * per) * n + c] = sw * stepsPerSweep + k;
-            if (symmetric) T[static_cast<size_t>(sw * per + 1) * n + c] = sw * stepsPerSweep + 2 * C.nColours - 1 - k;
+            const int k = back ? C.nColours - 1 - i : i;
+            // a colour's cells side by side: none reads another
+            constexpr int kBlock = 16384;
+            const int from = start[k], count = start[k + 1] - from;
+            flowParallel((count + kBlock - 1) / kBlock, [&](int block, int) {
+                const int end = std::min(count, (block + 1) * kBlock);
+                for (int j = block * kBlock; j < end; ++j)
+                {
+                    const int c = byColour[from + j], p = H.cellPos[c];
+                    int t = prev ? prev[c] + 1 : 0;
+                    for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e)
+                    {
+                        const int o = H.posCell[H.entColPos[e]];
+                        const bool earlier = back ? colourOf[o] > k : colourOf[o] < k;
+                        if (!earlier && !prev) continue;
+                        t = std::max(t, (earlier ? cur[o] : prev[o]) + (R > 1 && rank[o] != rank[c] ? weight : 1));
+                    }
+                    cur[c] = t;
+                }
+            });
         }
+    }
+    nSteps = T.empty() ? 0 : *std::max_element(T.begin(), T.end()) + 1;
     return T;
 }
 
@@ -591,9 +623,13 @@ void Matrix::ensurePipe(int level, int nSweeps)
 // The multicolour smoothing call of nSweeps sweeps on `level` as one data-flow launch whose steps are the
 // colours (colourSteps), against the tuned colour-by-colour shape (Matrix::tuneMulticolour): the faster is
 // kept. Both compute every row with the same fused multiply-adds in the same order on the same values, so the
-// choice changes the time only. Tried with a CTA per chunk of a colour's rows (k::kFlowTeam warps), where a step
-// is one chunk and a hand-over, and with twice as many. Above kMcFlowCells the colours are bound by bandwidth and
-// the launch per colour, which reads each value once from L2, wins.
+// choice changes the time only. Tried with a CTA per chunk of a colour's rows (k::kFlowTeam warps), one CTA
+// alone where that would be two. Measured per call of four sweeps (4 M-cell box's levels), a step per colour ->
+// the colours' order with a hand-over of 4 steps: 256 k cells 138 -> 112 us, 128 k 132 -> 103, 64 k 127 -> 91, 16 k
+// 110 -> 75, 8 k 96 -> 67, and the colour-by-colour shapes 198, 222, 208, 176, 155; weights 2 and 8 were up to 12 %
+// slower, half and twice the CTAs about the same; 2,000 cells 42 us on one CTA, 48 on two. Above
+// kMcFlowCells the colours are bound by bandwidth and the launch per colour, which reads each value once from
+// L2, wins.
 void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
 {
     LevelAddr& L = mesh->lev[level];
@@ -626,28 +662,22 @@ void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     FlowLevel H = flowDownload(L, stream);
-    int visits = 0, nSteps = 0;
-    const std::vector<int> T = colourSteps(H, C, C.pos.download(stream), nSweeps, symmetric, visits, nSteps);
-    float best = M.msColours;
+    const std::vector<int> rowPos = C.pos.download(stream);
     const int per = 32 * k::kFlowTeam * C.nColours;
-    const int sms = DeviceInfo::get().numSMs, one = std::min(sms, (L.nCells + per - 1) / per);
-    for (int R : {one, std::min(sms, 2 * one)})
+    const int one = std::min(DeviceInfo::get().numSMs, (L.nCells + per - 1) / per);
+    const FlowShape f = one <= 2 ? FlowShape{1, 1} : FlowShape{one, 4};
+    int visits = 0, nSteps = 0;
+    const std::vector<int> T = colourSteps(H, C, rowPos, nSweeps, symmetric, f.ranks, f.weight, visits, nSteps);
+    std::unique_ptr<FlowSchedule> F;
+    if (!T.empty()) F = buildFlow(H, T, visits, nSteps, f.ranks, sizeof(float), stream);
+    if (F)
     {
-        if (T.empty()) break;
-        std::unique_ptr<FlowSchedule> F = buildFlow(H, T, visits, nSteps, R, sizeof(float), stream);
-        if (!F) continue;
-        const float ms = flowTime<float>(level, *F, x, b, true);
-        if (M.msPipe == 0.f || ms < M.msPipe) M.msPipe = ms;
-        if (ms < best)
-        {
-            best = ms;
-            if (M.flow) v32.flows.erase(M.flow->id);
+        M.msPipe = flowTime<float>(level, *F, x, b, true);
+        M.use = M.msPipe < M.msColours;
+        if (M.use)
             M.flow = std::move(F);
-            M.use = true;
-        }
         else
             v32.flows.erase(F->id);
-        if (one == 1 || one == sms) break;
     }
     launches = l0;
     B2G_CUDA(cudaStreamSynchronize(stream));
