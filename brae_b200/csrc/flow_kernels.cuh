@@ -52,7 +52,7 @@ constexpr int kFlowHalo = 4;      // NH: halo warps of a launch with more than o
 // row entries a thread holds in registers (the rest come from the ring, four at a time): as many as fit
 // beside the gathered values without spilling at the launch's register count
 constexpr int kFlowK = 16;
-constexpr int kFlowMaxSlots = 16384;
+constexpr int kFlowMaxSlots = 65535;  // a slot's number has 16 bits
 constexpr int kFlowMaxVisits = 63;  // visits of a cell in one call (the tag's low 6 bits)
 
 // A chunk's record, three int4. Offsets within a chunk count 8 bytes from its place in the ring.

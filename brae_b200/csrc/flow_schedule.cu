@@ -227,7 +227,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         const size_t metaBytes = codesAt + (2 * static_cast<size_t>(nEnt) + 15) / 16 * 16;
         const size_t valsAt = metaBytes + 64 * static_cast<size_t>(nSl) * vb, srcBytesAt = valsAt + nEnt * vb;
         // (offsets within a chunk count 8 bytes in 16 bits)
-        if (P.slots > k::kFlowMaxSlots || srcBytesAt + 32 * static_cast<size_t>(nSl) * vb > 8 * 65535u ||
+        if (P.slots > k::kFlowMaxSlots || vb * P.slots > kFlowSmem || srcBytesAt + 32 * static_cast<size_t>(nSl) * vb > 8 * 65535u ||
             fetch.size() > 65535u || halo.size() > 65535u)
         {
             P.ok = false;
@@ -407,8 +407,13 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
         F.metaBytes += P.meta.size();
         F.nVal += P.src.size();
     }
+    // the ring holds three chunks at least: one computed, one loaded by the other team, one on its way
     const size_t ringAt = k::flowRingAt(F.slots, vb);
-    if (ringAt + 3 * kFlowChunkBytes > kFlowSmem) return false;
+    size_t chunk = 0;
+    for (const RankProgram& P : F.prog)
+        for (const k::FlowRec& r : P.rec)
+            chunk = std::max(chunk, static_cast<size_t>(r.metaBytes) + r.valBytes + 32 * static_cast<size_t>(r.nSlices) * vb);
+    if (ringAt + 3 * chunk > kFlowSmem) return false;
     if (F.metaBytes / 16 > 0x7fffffffull || F.nVal * vb / 16 > 0x7fffffffull) return false;
     F.chunkStart.assign(static_cast<size_t>(R) + 1, 0);
     F.rec.clear();
