@@ -33,7 +33,14 @@
 // more is several chunks. A producer warp keeps bulk copies of the
 // chunks ahead in flight into a shared-memory ring (placed by the schedule). A gather warp brings each
 // chunk's source values and initial values (cp.async). Halo warps, chunk j by warp j mod NH, poll the
-// mailboxes.
+// mailboxes. What these warps bring is told by one mbarrier per chunk in flight and kind, the copies of the
+// gather warp arriving on it themselves.
+//
+// BOUND. Neither bytes nor arithmetic: the chain of chunks. About 850 cycles a chunk (clock stamps, FP64 levels
+// of 88 to 24 k cells): a team's row 440-580, its barrier to the other 300 with the slowest warp's lag; and a
+// team's own loop (barrier, row, stores 150, the next chunk's wait and load 700) is about two of those. With a
+// release-acquire counter in place of the mbarriers and the gather warp waiting for its copies: 24 k cells
+// 9.38 -> 8.97 ms a solve, 1 M 42.6 -> 41.7, 4 M (two iterations) 14.7 -> 13.8, a batch of 24 48.1 -> 44.4.
 //
 // LIMITS. Every wait has an iteration limit; when one runs out the error word is set, every role
 // stops taking work, the copies in flight are waited for, and the launch ends with an error. All CTAs
@@ -194,12 +201,12 @@ __device__ __forceinline__ float flowTerm(float acc, float v, float x)
 // the launch's shared control words
 struct FlowShared
 {
-    unsigned long long full[kFlowDepth];   // a chunk's bulk copies have landed
+    unsigned long long full[kFlowDepth];    // a chunk's bulk copies have landed
+    unsigned long long staged[kFlowDepth];  // and its source and initial values (the gather warp's lanes)
+    unsigned long long halo[kFlowDepth];    // and the values of other ranks (its halo warp)
     int4 rec[kFlowDepth][3];
     uint2 place[kFlowDepth];               // a chunk's shared address and its slices
     unsigned consumed;                     // chunks consumed
-    unsigned staged;                       // chunks whose source and initial values have landed, too
-    unsigned halo[kFlowHalo];              // per halo warp: the last chunk it completed, plus one
     unsigned stop;                         // a wait gave up
 };
 
@@ -225,6 +232,17 @@ __device__ __forceinline__ bool flowWait(FlowShared& S, int* err, long long limi
         }
     }
     return true;
+}
+
+// mbarTryWait without its wait: asked again by the caller
+__device__ __forceinline__ bool mbarTestWait(unsigned long long* bar, unsigned parity)
+{
+    unsigned ok;
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok)
+                 : "r"(smemAddr(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
 }
 
 __device__ __forceinline__ int4 lds128(unsigned a)
@@ -381,16 +399,24 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
     const unsigned tagOut = a.publish ? tag0 : 0u;  // epochs start at 1: no tag is met when not publishing
     if (t == 0)
     {
-        for (int i = 0; i < kD; ++i) mbarInit(&S.full[i], 1);
-        for (int i = 0; i < kFlowHalo; ++i) S.halo[i] = 0;
+        for (int i = 0; i < kD; ++i)
+        {
+            mbarInit(&S.full[i], 1);
+            mbarInit(&S.staged[i], 32);
+            mbarInit(&S.halo[i], 1);
+        }
         S.consumed = 0;
-        S.staged = 0;
         S.stop = 0;
         stsT(xA, T(0));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    // A chunk's place in these barriers is taken again kFlowDepth chunks later, once the chunk is consumed; a warp
+    // that waits for chunk j has waited for chunk j - kFlowDepth before, so the parity tells the two apart.
+    static_assert(kD % 2 == 0 && kD % kFlowHalo == 0, "a team and a halo warp meet a barrier in every phase");
     auto isFull = [&](int j) { return mbarTryWait(&S.full[j % kD], (j / kD) & 1u); };
+    auto isStaged = [&](int j) { return mbarTestWait(&S.staged[j % kD], (j / kD) & 1u); };
+    auto hasHalo = [&](int j) { return mbarTestWait(&S.halo[j % kD], (j / kD) & 1u); };
     if (warp < 2 * kTeamWarps)
     {
         // Team j mod 2 computes chunk j. A team waits for the other's last chunk only (a named barrier per
@@ -402,12 +428,12 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
         bool ok = true;   // no wait of this warp has given up
         bool haloOk = true;
         auto preload = [&](int j) {
-            if (ok) ok = flowWait(S, a.err, a.spinLimit, [&] { return ldAcquireCta(&S.staged) > static_cast<unsigned>(j); });
+            if (ok) ok = flowWait(S, a.err, a.spinLimit, [&] { return isFull(j) && isStaged(j); });
             R.w = -1;
             if (!ok) return;
             const uint2 p = lds64(smemAddr(&S.place[j % kD]));
             if (wi < static_cast<int>(p.y)) flowLoad(p.x, wi, lane, xA, R);
-            if (kRemote) haloOk = ldAcquireCta(&S.halo[j % kFlowHalo]) > static_cast<unsigned>(j);
+            if (kRemote) haloOk = hasHalo(j);
         };
         if (team < nCh) preload(team);
         for (int j = team; j < nCh; j += 2)
@@ -420,7 +446,7 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
                 if (wi == 0 && lane == 0) *reinterpret_cast<volatile unsigned*>(&S.consumed) = static_cast<unsigned>(j);
             }
             if (kRemote && ok && !haloOk)
-                ok = flowWait(S, a.err, a.spinLimit, [&] { return ldAcquireCta(&S.halo[j % kFlowHalo]) > static_cast<unsigned>(j); });
+                ok = flowWait(S, a.err, a.spinLimit, [&] { return hasHalo(j); });
             T x = T(0);
             if (ok && R.w >= 0) x = flowRow<T, kFma>(R, xA);
             if (j + 1 < nCh) asm volatile("bar.arrive %0, %1;" ::"r"(1 + (j & 1)), "n"(64 * kTeamWarps) : "memory");
@@ -436,7 +462,7 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
     else if (warp == 2 * kTeamWarps)
     {
         // the producer: chunk j's blobs into its place in the ring once that place is free
-        int issued = 0;
+        int issued = 0, consumed = 0;
         int4 q0{}, q1{}, q2{};
         for (int j = 0; j < nCh; ++j)
         {
@@ -455,9 +481,16 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
             r1.z = __shfl_sync(~0u, q1.z, from); r1.w = __shfl_sync(~0u, q1.w, from);
             r2.x = __shfl_sync(~0u, q2.x, from); r2.y = __shfl_sync(~0u, q2.y, from);
             r2.z = __shfl_sync(~0u, q2.z, from); r2.w = __shfl_sync(~0u, q2.w, from);
-            const bool go = flowWait(S, a.err, a.spinLimit,
-                                     [&] { return static_cast<int>(ldAcquireCta(&S.consumed)) > r0.w; });
-            if (!__all_sync(~0u, go)) break;
+            if (consumed <= r0.w)
+            {
+                const bool go = flowWait(S, a.err, a.spinLimit, [&] {
+                    consumed = static_cast<int>(ldAcquireCta(&S.consumed));
+                    return consumed > r0.w;
+                });
+                if (!go) consumed = -1;
+            }
+            consumed = __reduce_min_sync(~0u, consumed);
+            if (consumed < 0) break;
             if (lane == 0)
             {
                 unsigned long long* bar = &S.full[j % kD];
@@ -483,25 +516,12 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
     }
     else if (warp == 2 * kTeamWarps + 1)
     {
-        // the gather warp: each chunk's source values and the initial values first used there. They are
-        // published (S.staged) kAhead chunks behind their issue, so that the copies of a few chunks overlap,
-        // and all of them before the warp waits for a chunk that has not arrived yet.
-        constexpr int kAhead = 2;
-        auto publish = [&](int upTo) {
-            __syncwarp();
-            if (lane == 0) stReleaseCta(&S.staged, static_cast<unsigned>(upTo));
-        };
-        bool all = true;
+        // the gather warp: each chunk's source values and the initial values first used there. The copies tell
+        // the chunk's barrier themselves when they have landed, so any number of chunks are under way.
         for (int j = 0; j < nCh; ++j)
         {
-            if (!__shfl_sync(~0u, static_cast<int>(isFull(j)), 0))
-            {
-                asm volatile("cp.async.wait_all;" ::: "memory");
-                publish(j);
-            }
             const bool go = flowWait(S, a.err, a.spinLimit, [&] { return isFull(j); });
-            all = __all_sync(~0u, go);
-            if (!all) break;
+            if (!__all_sync(~0u, go)) break;
             const int4 r0 = S.rec[j % kD][0], r1 = S.rec[j % kD][1], r2 = S.rec[j % kD][2];
             const unsigned chunkA = ringA + static_cast<unsigned>(r0.z);
             const unsigned bA = chunkA + static_cast<unsigned>(r0.y + r1.y);
@@ -512,15 +532,9 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
                 const uint2 f = lds64(chunkA + 8u * (r2.y + i));
                 cpAsync(xA + static_cast<unsigned>(sizeof(T)) * f.y, a.psi + f.x);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if (j >= kAhead)
-            {
-                asm volatile("cp.async.wait_group %0;" ::"n"(kAhead) : "memory");
-                publish(j + 1 - kAhead);
-            }
+            mbarArriveCpAsync(&S.staged[j % kD]);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        if (all) publish(nCh);
     }
     else if (kRemote)
     {
@@ -556,7 +570,7 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
             }
             if (!__all_sync(~0u, go)) break;
             __syncwarp();
-            if (lane == 0) stReleaseCta(&S.halo[h], static_cast<unsigned>(j + 1));
+            if (lane == 0) mbarArrive(&S.halo[j % kD]);
         }
     }
     if (kRemote && a.ctl)
