@@ -26,11 +26,23 @@ struct RankScratch
     std::vector<int> localOf;  // cell -> ghost index of the rank at work, -1
 };
 
+// An item as a sort key: [first: its step's other chunks go before it][65535 - row width][position][visit][out:
+// another rank reads it]
 struct ItemRef
 {
-    int p, q, w;  // position, visit, row width
-    bool out;     // another rank reads it
+    unsigned long long key;
+    int p() const { return static_cast<int>(key >> 7 & 0x7fffffffu); }
+    int q() const { return static_cast<int>(key >> 1 & 0x3fu); }
+    int w() const { return 65535 - static_cast<int>(key >> 38 & 0xffffu); }
+    bool out() const { return key & 1u; }
 };
+static_assert(k::kFlowMaxVisits < 64, "a visit has 6 bits of the key");
+ItemRef itemRef(int p, int q, int w, bool out)
+{
+    return {static_cast<unsigned long long>(65535 - std::min(w, 65535)) << 38 | static_cast<unsigned long long>(p) << 7 |
+            static_cast<unsigned long long>(q) << 1 | (out ? 1u : 0u)};
+}
+constexpr unsigned long long kItemLater = 1ull << 62;
 
 void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int c0, int c1, size_t vb,
                RankScratch& X, RankProgram& P)
@@ -63,7 +75,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
             for (int c = c0; c < c1; ++c)
             {
                 const int p = H.cellPos[c];
-                items[cur[T[q * n + c]]++] = ItemRef{p, q, H.posRow[p + 1] - H.posRow[p], exported[c - c0] != 0};
+                items[cur[T[q * n + c]]++] = itemRef(p, q, H.posRow[p + 1] - H.posRow[p], exported[c - c0] != 0);
             }
     }
     struct Span
@@ -76,17 +88,17 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         const int a = start[st], b = start[st + 1];
         if (a == b) continue;
         const bool several = b - a > kFlowChunkItems;
-        std::sort(items.begin() + a, items.begin() + b, [several](const ItemRef& x, const ItemRef& y) {
-            if (several && x.out != y.out) return x.out;
-            return x.w != y.w ? x.w > y.w : x.p != y.p ? x.p < y.p : x.q < y.q;
-        });
+        if (several)
+            for (int i = a; i < b; ++i)
+                if (!items[i].out()) items[i].key |= kItemLater;
+        std::sort(items.begin() + a, items.begin() + b, [](const ItemRef& x, const ItemRef& y) { return x.key < y.key; });
         // cut where the chunk is full: whole slices, its blobs and source within its share of the ring
         int from = a;
         size_t bytes = 64;
         for (int i = a; i < b; i += 32)
         {
             int w = 0;
-            for (int x = i; x < std::min(b, i + 32); ++x) w = std::max(w, items[x].w);
+            for (int x = i; x < std::min(b, i + 32); ++x) w = std::max(w, items[x].w());
             if (w > 252)
             {
                 P.ok = false;
@@ -122,7 +134,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
     for (int j = 0; j < nCh; ++j)
         for (int i = chunks[j].a; i < chunks[j].b; ++i)
         {
-            const int p = items[i].p;
+            const int p = items[i].p();
             last[H.posCell[p] - c0] = j;
             for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e) last[localId(H.posCell[H.entColPos[e]])] = j;
         }
@@ -143,6 +155,11 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
     {
         unsigned a, b;
     };
+    // (about what the items take: records, sources and rows padded by a quarter)
+    size_t rowEntries = 0;
+    for (const ItemRef& it : items) rowEntries += static_cast<size_t>((it.w() + 3) & ~3);
+    P.src.reserve(2 * items.size() + rowEntries * 5 / 4 + 128 * static_cast<size_t>(nCh));
+    P.meta.reserve(16 * items.size() + rowEntries * 5 / 2 + 1024 * static_cast<size_t>(nCh));
     std::vector<Pair> fetch, halo;
     std::vector<unsigned short> codes;
     int width[kFlowChunkItems / 32 + 1], first[kFlowChunkItems / 32 + 1];
@@ -167,7 +184,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         {
             // a multiple of 4 (the kernels' straight-line widths), at least 4
             int longest = 0;
-            for (int i = 32 * s; i < std::min(m, 32 * s + 32); ++i) longest = std::max(longest, items[a + i].w);
+            for (int i = 32 * s; i < std::min(m, 32 * s + 32); ++i) longest = std::max(longest, items[a + i].w());
             width[s] = std::max(4, (longest + 3) & ~3);
             first[s] = nEnt;
             nEnt += k::flowStride(m, s) * width[s];
@@ -181,24 +198,24 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         int* entSrc = diagSrc + 64 * nSl;
         for (int i = 0; i < m; ++i)
         {
-            diagSrc[2 * i] = -(2 * items[a + i].p + 2);
-            diagSrc[2 * i + 1] = -(2 * items[a + i].p + 3);
+            diagSrc[2 * i] = -(2 * items[a + i].p() + 2);
+            diagSrc[2 * i + 1] = -(2 * items[a + i].p() + 3);
         }
         // (a chunk's values are read before its items write: every read first, then the writes)
         for (int i = 0; i < m; ++i)
         {
-            const ItemRef& it = items[a + i];
-            const int c = H.posCell[it.p];
-            const int step = T[it.q * n + c];
+            const int p = items[a + i].p(), visitOf = items[a + i].q();
+            const int c = H.posCell[p];
+            const int step = T[visitOf * n + c];
             const int st = k::flowStride(m, i / 32);
             const int at0 = first[i / 32], l = i % 32, vg = vb == 8 ? 2 : 4;
-            for (int e = H.posRow[it.p], q = 0; e < H.posRow[it.p + 1]; ++e, ++q)
+            for (int e = H.posRow[p], q = 0; e < H.posRow[p + 1]; ++e, ++q)
             {
                 const int pn = H.entColPos[e];
                 const int cn = H.posCell[pn];
                 const int v = localId(cn);
                 // the neighbour's latest visit before this item (-1: its initial value)
-                int ver = it.q;
+                int ver = visitOf;
                 while (ver >= 0 && T[ver * n + cn] >= step) --ver;
                 if (v < nOwn)
                 {
@@ -221,7 +238,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
                 entSrc[at0 + vg * (st * (q / vg) + l) + q % vg] = e;
             }
         }
-        for (int i = 0; i < m; ++i) give(H.posCell[items[a + i].p] - c0);
+        for (int i = 0; i < m; ++i) give(H.posCell[items[a + i].p()] - c0);
         const size_t itemsAt = 16 * static_cast<size_t>(nSl), fetchAt = itemsAt + 256 * static_cast<size_t>(nSl);
         const size_t haloAt = fetchAt + (fetch.size() + 1) / 2 * 16, codesAt = haloAt + (halo.size() + 1) / 2 * 16;
         const size_t metaBytes = codesAt + (2 * static_cast<size_t>(nEnt) + 15) / 16 * 16;
@@ -252,10 +269,10 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         for (int i = 0; i < m; ++i)
         {
             const ItemRef& it = items[a + i];
-            const int c = H.posCell[it.p];
-            const Pair w{static_cast<unsigned>(it.p),
-                         static_cast<unsigned>(slot[c - c0]) | static_cast<unsigned>(it.q) << 16 |
-                             (it.out ? 0x40000000u : 0u) | (it.q == S - 1 ? 0x80000000u : 0u)};
+            const int c = H.posCell[it.p()];
+            const Pair w{static_cast<unsigned>(it.p()),
+                         static_cast<unsigned>(slot[c - c0]) | static_cast<unsigned>(it.q()) << 16 |
+                             (it.out() ? 0x40000000u : 0u) | (it.q() == S - 1 ? 0x80000000u : 0u)};
             std::memcpy(M + itemsAt + 8 * static_cast<size_t>(i), &w, 8);
         }
         if (!fetch.empty()) std::memcpy(M + fetchAt, fetch.data(), 8 * fetch.size());
