@@ -42,9 +42,13 @@
 // release-acquire counter in place of the mbarriers and the gather warp waiting for its copies: 24 k cells
 // 9.38 -> 8.97 ms a solve, 1 M 42.6 -> 41.7, 4 M (two iterations) 14.7 -> 13.8, a batch of 24 48.1 -> 44.4.
 //
-// LIMITS. Every wait has an iteration limit; when one runs out the error word is set, every role
-// stops taking work, the copies in flight are waited for, and the launch ends with an error. All CTAs
-// of a launch with ranks are resident together (a cooperative launch).
+// LIMITS. Every wait has an iteration limit; when one runs out the error word and the CTA's stop word are
+// set and the launch ends with an error. From then on no chunk counts as consumed (a chunk counts only while
+// the stop word is clear, behind the barrier that every warp of its team has passed: so every wait for it,
+// the gather warp's and the halo warp's parts included, ended well). Nothing in the ring is staged over what
+// any role may still read, at most the chunks already allowed are issued, and the producer waits for every
+// copy it has issued before the CTA ends. All CTAs of a launch with ranks are resident together (a
+// cooperative launch).
 #pragma once
 
 #include "b2g_common.cuh"
@@ -441,9 +445,10 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
             if (j > 0)
             {
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + ((j - 1) & 1)), "n"(64 * kTeamWarps) : "memory");
-                // (the barrier has ordered the chunk's reads; a plain store, since a release would wait for this
-                // thread's mailbox stores to land, on the chain of every step)
-                if (wi == 0 && lane == 0) *reinterpret_cast<volatile unsigned*>(&S.consumed) = static_cast<unsigned>(j);
+                // (never after a stop: the chunks that a stopped warp skipped may still be read by the other
+                // roles, see LIMITS. The last warp publishes, since it has no row in a chunk of fewer slices)
+                if (wi == kTeamWarps - 1 && lane == 0 && *reinterpret_cast<volatile unsigned*>(&S.stop) == 0)
+                    *reinterpret_cast<volatile unsigned*>(&S.consumed) = static_cast<unsigned>(j);
             }
             if (kRemote && ok && !haloOk)
                 ok = flowWait(S, a.err, a.spinLimit, [&] { return hasHalo(j); });
@@ -509,10 +514,9 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
             __syncwarp();
             issued = j + 1;
         }
-        // the CTA leaves only once the copies issued have landed
-        if (issued < nCh)
-            for (int j = max(0, issued - kD); j < issued; ++j)
-                for (long long it = 0; it < (1 << 20) && !isFull(j); ++it) {}
+        // the CTA leaves only once the copies issued have landed, whether a wait gave up before or does after this
+        for (int j = max(0, issued - kD); j < issued; ++j)
+            for (long long it = 0; it < (1 << 20) && !isFull(j); ++it) {}
     }
     else if (warp == 2 * kTeamWarps + 1)
     {

@@ -103,23 +103,32 @@ def test_quotient_edges(b2g, oracle, scale):
                 assert np.array_equal(np.signbit(got[finite]), np.signbit(want[finite]))
 
 
-def test_wait_gives_up(b2g, oracle):
+# CTA counts and limits that make waits run out at different places of a launch: at the first hand-over, with the
+# ring full of chunks under way, on levels of few and of many chunks a CTA
+@pytest.mark.parametrize("ranks,limit", [(2, 1 << 10), (7, 1 << 12), (16, 1 << 14), (0, 1 << 12)])
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_wait_gives_up(b2g, oracle, ranks, limit, symmetric):
     # no rank hands its values over: every rank's wait runs out after a short limit, the launch ends and the
     # call reports a device time-out; the next call on the same matrix is the oracle's
     c = cases.box_case(40, 40, 40, (2.0, 1.0, 1.0), 20.0)
+    ranks = ranks or torch.cuda.get_device_properties(0).multi_processor_count
     mesh, A = _build(b2g, c)
-    lo, up, d, u = _level_system(mesh, A, c, 0)
     rng = np.random.default_rng(5)
-    x0, b = rng.uniform(-1.0, 1.0, d.shape[0]), rng.uniform(-1.0, 1.0, d.shape[0])
-    status = "OK"
-    try:
-        A.smooth_flow(0, dev(x0), dev(b), 2, 16, 4, stall_limit=1 << 14)
-    except b2g.GamgError as e:
-        status = e.status
-    assert status == "DEVICE_TIMEOUT"
-    x = dev(x0)
-    A.smooth_flow(0, x, dev(b), 2, 16, 4)
-    assert np.array_equal(x.cpu().numpy(), oracle.smooth(lo, up, d, u, x0, b, 2))
+    for lv in (0, 2):
+        lo, up, d, u = _level_system(mesh, A, c, lv)
+        x0, b = rng.uniform(-1.0, 1.0, d.shape[0]), rng.uniform(-1.0, 1.0, d.shape[0])
+        want = oracle.smooth(lo, up, d, u, x0, b, 3, "symGaussSeidel" if symmetric else "GaussSeidel")
+        for sweeps in (1, 3):
+            status = "OK"
+            try:
+                A.smooth_flow(lv, dev(x0), dev(b), sweeps, ranks, 4, stall_limit=limit, symmetric=symmetric)
+            except b2g.GamgError as e:
+                status = e.status
+            assert status in ("DEVICE_TIMEOUT", "ARGUMENT"), (lv, sweeps)
+            assert status == "DEVICE_TIMEOUT" or d.shape[0] / ranks > 10000  # (ARGUMENT: too many cells for so few)
+        x = dev(x0)
+        A.smooth_flow(lv, x, dev(b), 3, max(ranks, 7), 4, symmetric=symmetric)
+        assert np.array_equal(x.cpu().numpy(), want)
 
 
 def test_smoothing_calls_on_streams_and_threads(b2g, oracle):
