@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from typing import NamedTuple
 
 import numpy as np
@@ -225,7 +226,41 @@ def _as_host(a, dtype):
     return np.ascontiguousarray(a, dtype=dtype)
 
 
-class Mesh:
+class _Handle:
+    """A library handle and those it is built on: destroyed when its object and every handle built on it
+    are gone. The garbage collector may finalise a mesh and its matrices, freed in one cycle, in any order."""
+
+    __slots__ = ("value", "destroy", "needs", "users")
+    lock = threading.RLock()  # (a collection within a release may release others)
+
+    def __init__(self, value, destroy, needs=()):
+        self.value, self.destroy, self.needs, self.users = value, destroy, tuple(needs), 1
+        with self.lock:
+            for h in self.needs:
+                h.users += 1
+
+    def release(self):
+        with self.lock:
+            self.users -= 1
+            if self.users:
+                return
+            self.destroy(self.value)
+            for h in self.needs:
+                h.release()
+
+
+class _Owner:
+    """An object with a _Handle."""
+    _owned = None
+
+    def __del__(self):
+        o, self._owned = self._owned, None
+        if o is not None and lib is not None:
+            o.release()
+            self.handle = None
+
+
+class Mesh(_Owner):
     """The mesh's GAMG hierarchy (GamgAgglomerationCache): built once, on the device."""
 
     def __init__(self, lower, upper, Sf, magSf, n_cells: int, n_coarsest: int = 10,
@@ -251,15 +286,10 @@ class Mesh:
                                               str(cache_path).encode(), C.byref(h), C.byref(hit)))
             self.from_cache = bool(hit.value)
         self.handle = h
+        self._owned = _Handle(h, lib.b2g_mesh_destroy)
         self.forward = bool(fw.value)
         self.n_cells = int(n_cells)
         self.n_faces = nF
-
-    def __del__(self):
-        h = getattr(self, "handle", None)
-        if h is not None and h.value and lib is not None:
-            lib.b2g_mesh_destroy(h)
-            self.handle = None
 
     @property
     def n_levels(self) -> int:
@@ -364,7 +394,7 @@ class _LogBuf:
                  self.coarse[i].nIterations) for i in range(n)]
 
 
-class Matrix:
+class Matrix(_Owner):
     """One folded matrix on a mesh's hierarchy (GamgHierarchy): Galerkin levels on the device."""
 
     def __init__(self, mesh: Mesh, diag, upper, pair_coeffs=None):
@@ -381,6 +411,7 @@ class Matrix:
             _check(lib.b2g_matrix_create_coupled(mesh.handle, _ptr(diag), _ptr(upper), _ptr(pair_coeffs), ms,
                                                  _stream(), C.byref(h)))
         self.handle = h
+        self._owned = _Handle(h, lib.b2g_matrix_destroy, (mesh._owned,))
         self.mesh = mesh
 
     def set_coeffs(self, diag, upper):
@@ -404,12 +435,6 @@ class Matrix:
         _check(lib.b2g_matrix_gamg_solve(self.handle, _ptr(source), _ptr(psi), C.byref(controls), ms, C.byref(p),
                                          C.byref(lb.log)))
         return SolverPerformance(p.initialResidual, p.finalResidual, p.nIterations), lb.history()
-
-    def __del__(self):
-        h = getattr(self, "handle", None)
-        if h is not None and h.value and lib is not None:
-            lib.b2g_matrix_destroy(h)
-            self.handle = None
 
     def level(self, level: int):
         nc, nf = self.mesh.level_size(level)
@@ -703,7 +728,7 @@ class Server:
             pass
 
 
-class Batch:
+class Batch(_Owner):
     """The batched form (b2g_batch_*): many matrices, each on its own mesh, solved together with every
     level step one launch over all cases. The matrices are kept alive as long as the batch."""
 
@@ -713,6 +738,7 @@ class Batch:
         h = C.c_void_p()
         _check(lib.b2g_batch_create(arr, len(self.matrices), C.byref(h)))
         self.handle = h
+        self._owned = _Handle(h, lib.b2g_batch_destroy, [m._owned for m in self.matrices])
 
     def solve(self, sources, psis, controls: Controls):
         """Solves every case: sources[k], psis[k] (numpy arrays or CUDA tensors, all of one kind, natural
@@ -739,9 +765,3 @@ class Batch:
         v = C.c_longlong()
         _check(lib.b2g_batch_launches(self.handle, C.byref(v)))
         return v.value
-
-    def __del__(self):
-        h = getattr(self, "handle", None)
-        if h is not None and h.value and lib is not None:
-            lib.b2g_batch_destroy(h)
-            self.handle = None

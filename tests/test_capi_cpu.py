@@ -22,6 +22,45 @@ def test_library_exports_every_declared_symbol():
     assert sorted(n.EXPORTED) == declared
 
 
+@pytest.mark.parametrize("order", [(0, 1, 2), (2, 1, 0), (1, 0, 2), (1, 2, 0)])
+def test_handles_freed_in_one_cycle(monkeypatch, order):
+    # a mesh, its matrix and a batch of it that the garbage collector frees together, whatever order it
+    # finalises them in: the library sees the batch go before the matrix, and the matrix before the mesh
+    import ctypes as C
+    import gc
+    import types
+
+    import numpy as np
+
+    import brae_b200.native as n
+    gone = []
+    fake = types.SimpleNamespace()
+    for k, (kind, create) in enumerate((("mesh", "mesh_create"), ("matrix", "matrix_create"), ("batch", "batch_create"))):
+        def make(*args, value=k + 1):
+            out = args[-1]._obj
+            out.value = value
+            return 0
+        setattr(fake, "b2g_" + create, make)
+        setattr(fake, f"b2g_{kind}_destroy", lambda h, kind=kind: gone.append(kind))
+    monkeypatch.setattr(n, "lib", fake)
+    one = np.zeros(1, np.int32)
+    mesh = n.Mesh(one, one, np.zeros((1, 3)), np.zeros(1), 2)
+    mat = n.Matrix(mesh, np.zeros(2), np.zeros(1))
+    batch = n.Batch([mat])
+    ring = [mesh, mat, batch]
+    mesh.ring = ring
+    gc.collect()
+    gc.disable()
+    try:
+        for i in order:  # finalisers in this order, then what the collector finds of the cycle
+            ring[i].__del__()
+        del mesh, mat, batch, ring
+        gc.collect()
+    finally:
+        gc.enable()
+    assert gone == ["batch", "matrix", "mesh"]
+
+
 def test_controls_defaults():
     import brae_b200 as b
     c = b.controls_default()
