@@ -288,6 +288,9 @@ __global__ void __launch_bounds__(kUpThreads, 1) scaleProlongCluster(Rows<T> A, 
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int rank = static_cast<int>(cluster.block_rank()), C = static_cast<int>(cluster.num_blocks());
     const int nPart = (A.n + 255) / 256;
+    // CTA 0's shared memory may be written once CTA 0 is known to run: the arrival here, the wait for the
+    // others' before the first such store, behind the rows' loads
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
     T fc[kUpCells], ac[kUpCells];
 #pragma unroll
     for (int i = 0; i < kUpCells; ++i)
@@ -344,6 +347,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) scaleProlongCluster(Rows<T> A, 
             sh[2 * warp + 1] = den;
         }
         __syncthreads();
+        if (i == 0) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         if ((warp & 7) == 0)
         {
             T a = lane < 8 ? sh[2 * (warp + lane)] : T(0), b = lane < 8 ? sh[2 * (warp + lane) + 1] : T(0);

@@ -179,3 +179,8 @@ def test_solve_at_transfer_edges(b2g, oracle, nx, ny, nz):
     perf, _, _ = A.solve(dev(c.source), x, b2g.controls_default(tolerance=1e-8))
     assert perf.nIterations == want["perf"][2]
     assert np.abs(x.cpu().numpy() - want["psi"]).max() <= 1e-10 * np.abs(want["psi"]).max()
+    # the order of the sums is fixed: every further solve gives the same bits
+    for _ in range(4):
+        again = dev(np.zeros(c.n_cells))
+        A.solve(dev(c.source), again, b2g.controls_default(tolerance=1e-8))
+        assert torch.equal(again, x)
