@@ -3,6 +3,7 @@
 // refusals (readGamgControls, src/matrices/lduMatrix/solvers/GAMG/gamg_solver_cpp.cu:801-928, and
 // the PCG keys of src/applications/solvers/interFoam/inter_case_cpp.cu:1519-1572).
 #include "capi_internal.cuh"
+#include "flow.cuh"
 
 #include <cctype>
 #include <cstdio>
@@ -933,6 +934,60 @@ b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const do
             b2g::fail(B2G_ERR_ARGUMENT, "b2g_level_smooth_flow: the level does not fit that many CTAs");
         A.fromPos(level, static_cast<const double*>(A.ioBuf(0)), psi);
         B2G_CUDA(cudaStreamSynchronize(A.stream));
+    });
+}
+
+b2g_status b2g_flow_handovers(int nCells, int nFaces, const int32_t* lower, const int32_t* upper, const int32_t* colours,
+                              int nSweeps, int symmetric, int ranks, int weight, int valueBytes, long long counts[4])
+{
+    return guarded([&] {
+        need(nCells >= 1 && nFaces >= 0 && counts && (nFaces == 0 || (lower && upper)), "b2g_flow_handovers: bad addressing");
+        need(nSweeps >= 1 && ranks >= 1 && weight >= 1 && weight <= 64, "b2g_flow_handovers: bad shape");
+        need(valueBytes == 4 || valueBytes == 8, "b2g_flow_handovers: valueBytes must be 4 or 8");
+        b2g::FlowLevel H;
+        H.n = nCells;
+        H.nF = nFaces;
+        H.lower.assign(lower, lower + nFaces);
+        H.upper.assign(upper, upper + nFaces);
+        H.posCell.resize(nCells);
+        H.posRow.assign(static_cast<size_t>(nCells) + 1, 0);
+        for (int f = 0; f < nFaces; ++f)
+        {
+            need(lower[f] >= 0 && lower[f] < upper[f] && upper[f] < nCells && (f == 0 || lower[f] >= lower[f - 1]),
+                 "b2g_flow_handovers: faces must be upper-triangular, by owner");
+            ++H.posRow[lower[f] + 1];
+            ++H.posRow[upper[f] + 1];
+        }
+        for (int c = 0; c < nCells; ++c)
+        {
+            H.posCell[c] = c;
+            H.posRow[c + 1] += H.posRow[c];
+        }
+        H.cellPos = H.posCell;
+        // a row's lower neighbours, then its upper ones
+        H.entColPos.resize(2 * static_cast<size_t>(nFaces));
+        std::vector<int> at(H.posRow.begin(), H.posRow.end() - 1);
+        for (int f = 0; f < nFaces; ++f) H.entColPos[at[upper[f]]++] = lower[f];
+        for (int f = 0; f < nFaces; ++f) H.entColPos[at[lower[f]]++] = upper[f];
+        int visits = symmetric ? 2 * nSweeps : nSweeps, nSteps = 0;
+        std::vector<int> T;
+        if (colours)
+        {
+            const std::vector<int> colourOf(colours, colours + nCells);
+            T = b2g::colourSteps(H, colourOf, 1 + *std::max_element(colourOf.begin(), colourOf.end()), nSweeps,
+                                 symmetric != 0, ranks, weight, visits, nSteps);
+            need(!T.empty(), "b2g_flow_handovers: a cell has no colour");
+        }
+        else
+            T = b2g::flowSteps(H, nSweeps, symmetric != 0, ranks, weight, nSteps);
+        b2g::FlowProgram F;
+        if (!b2g::buildFlowProgram(H, T, visits, nSteps, ranks, static_cast<size_t>(valueBytes), F))
+            b2g::fail(B2G_ERR_ARGUMENT, "b2g_flow_handovers: no such schedule");
+        const b2g::FlowHandOvers o = b2g::flowHandOvers(H, F);
+        counts[0] = o.stored;
+        counts[1] = o.taken;
+        counts[2] = o.unread;
+        counts[3] = o.missing;
     });
 }
 

@@ -46,6 +46,15 @@ struct FlowProgram
 
 FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s);
 std::vector<int> flowSteps(const FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps);
+std::vector<int> colourSteps(const FlowLevel& H, const std::vector<int>& colourOf, int nColours, int nSweeps,
+                             bool symmetric, int R, int weight, int& visits, int& nSteps);
+// A program's hand-overs between ranks: values stored to a mailbox, values polled for; of the (cell, visit) pairs
+// stored those that no rank polls for, and of those polled for the ones that nothing stores.
+struct FlowHandOvers
+{
+    long long stored = 0, taken = 0, unread = 0, missing = 0;
+};
+FlowHandOvers flowHandOvers(const FlowLevel& H, const FlowProgram& F);
 // The program for R ranks of items (visit q, cell c) at steps T[q * n + c], values of vb bytes; false when
 // a rank's live values or chunks do not fit its shared memory, or a row is too long.
 bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb, FlowProgram& F);

@@ -21,7 +21,10 @@
 // there and put the value into the ghost's slot. One mailbox per cell is enough, and ghosts may be
 // written as soon as they arrive: version s+1 of a cell exists only after every reader of version s
 // has run -- its upper neighbours' sweep-s items and its lower neighbours' sweep-(s+1) items, all of
-// which (s+1, c) reads -- and a reader runs only after its own halo warp took version s.
+// which (s+1, c) reads -- and a reader runs only after its own halo warp took version s. That orders the
+// stores of versions that another rank reads, and only those are stored: a symmetric order has versions that
+// nobody elsewhere reads (the last colour's forward visit, say), whose store could land after the next
+// version's, from the other team, and hide it from its reader for good.
 // The same argument covers psi itself: the initial values are fetched from global psi just before
 // their first use and the last sweep writes there, and a cell's last write comes after every reader of
 // its initial value.

@@ -44,22 +44,37 @@ ItemRef itemRef(int p, int q, int w, bool out)
 }
 constexpr unsigned long long kItemLater = 1ull << 62;
 
+// The visit of cell cn whose value visit q of its neighbour c reads: its latest before that item (-1: the
+// initial value)
+int versionRead(const std::vector<int>& T, size_t n, int q, int c, int cn)
+{
+    const int step = T[q * n + c];
+    int ver = q;
+    while (ver >= 0 && T[ver * n + cn] >= step) --ver;
+    return ver;
+}
+
 void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int c0, int c1, size_t vb,
                RankScratch& X, RankProgram& P)
 {
     const size_t n = static_cast<size_t>(H.n);
     const int nOwn = c1 - c0;
     if (X.localOf.size() != n) X.localOf.assign(n, -1);
-    // cells another rank reads: those with a neighbour there
-    std::vector<char> exported(nOwn, 0);
+    // the visits of a cell whose value another rank reads, a bit each
+    std::vector<unsigned long long> exported(nOwn, 0);
     if (H.crosses)
         for (int c = c0; c < c1; ++c)
         {
             const int p = H.cellPos[c];
-            for (int e = H.posRow[p]; e < H.posRow[p + 1] && !exported[c - c0]; ++e)
+            for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e)
             {
                 const int cn = H.posCell[H.entColPos[e]];
-                exported[c - c0] = cn < c0 || cn >= c1;
+                if (cn >= c0 && cn < c1) continue;
+                for (int q = 0; q < S; ++q)
+                {
+                    const int ver = versionRead(T, n, q, cn, c);
+                    if (ver >= 0) exported[c - c0] |= 1ull << ver;
+                }
             }
         }
     // items by step; of a step of several chunks those that another rank reads first, so that their way there
@@ -75,7 +90,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
             for (int c = c0; c < c1; ++c)
             {
                 const int p = H.cellPos[c];
-                items[cur[T[q * n + c]]++] = itemRef(p, q, H.posRow[p + 1] - H.posRow[p], exported[c - c0] != 0);
+                items[cur[T[q * n + c]]++] = itemRef(p, q, H.posRow[p + 1] - H.posRow[p], exported[c - c0] >> q & 1u);
             }
     }
     struct Span
@@ -206,7 +221,6 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         {
             const int p = items[a + i].p(), visitOf = items[a + i].q();
             const int c = H.posCell[p];
-            const int step = T[visitOf * n + c];
             const int st = k::flowStride(m, i / 32);
             const int at0 = first[i / 32], l = i % 32, vg = vb == 8 ? 2 : 4;
             for (int e = H.posRow[p], q = 0; e < H.posRow[p + 1]; ++e, ++q)
@@ -214,9 +228,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
                 const int pn = H.entColPos[e];
                 const int cn = H.posCell[pn];
                 const int v = localId(cn);
-                // the neighbour's latest visit before this item (-1: its initial value)
-                int ver = visitOf;
-                while (ver >= 0 && T[ver * n + cn] >= step) --ver;
+                const int ver = versionRead(T, n, visitOf, c, cn);
                 if (v < nOwn)
                 {
                     if (!slot[v])
@@ -405,6 +417,64 @@ std::vector<int> flowSteps(const FlowLevel& H, int nSweeps, bool symmetric, int 
     return T;
 }
 
+// The multicolour smoother's sweeps as steps on R ranks. The colours are an order of visits like the exact
+// sweeps' cell order, so an item runs one step after the last visit it reads, `weight` steps after one of another
+// rank: only the cells near a rank's border wait for a hand-over, the others run ahead into the next colours.
+// Every row still reads its neighbours of earlier colours at this visit and the others at the one before, as the
+// colour-by-colour sweep does. Symmetric sweeps visit the colours forward then back, each cell twice a sweep.
+// Empty when a cell has no colour.
+std::vector<int> colourSteps(const FlowLevel& H, const std::vector<int>& colourOf, int nColours, int nSweeps,
+                             bool symmetric, int R, int weight, int& visits, int& nSteps)
+{
+    const int n = H.n;
+    std::vector<int> byColour(n), start(static_cast<size_t>(nColours) + 1, 0);
+    for (int c = 0; c < n; ++c)
+    {
+        if (colourOf[c] < 0 || colourOf[c] >= nColours) return {};
+        ++start[colourOf[c] + 1];
+    }
+    for (int k = 0; k < nColours; ++k) start[k + 1] += start[k];
+    {
+        std::vector<int> at(start.begin(), start.end() - 1);
+        for (int c = 0; c < n; ++c) byColour[at[colourOf[c]]++] = c;
+    }
+    visits = symmetric ? 2 * nSweeps : nSweeps;
+    std::vector<int> rank(R > 1 ? n : 0);
+    for (size_t c = 0; c < rank.size(); ++c) rank[c] = flowRank(static_cast<int>(c), n, R);
+    std::vector<int> T(static_cast<size_t>(visits) * n);
+    for (int v = 0; v < visits; ++v)
+    {
+        int* cur = T.data() + static_cast<size_t>(v) * n;
+        const int* prev = v > 0 ? cur - n : nullptr;
+        const bool back = symmetric && (v & 1);
+        for (int i = 0; i < nColours; ++i)
+        {
+            const int k = back ? nColours - 1 - i : i;
+            // a colour's cells side by side: none reads another
+            constexpr int kBlock = 16384;
+            const int from = start[k], count = start[k + 1] - from;
+            flowParallel((count + kBlock - 1) / kBlock, [&](int block, int) {
+                const int end = std::min(count, (block + 1) * kBlock);
+                for (int j = block * kBlock; j < end; ++j)
+                {
+                    const int c = byColour[from + j], p = H.cellPos[c];
+                    int t = prev ? prev[c] + 1 : 0;
+                    for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e)
+                    {
+                        const int o = H.posCell[H.entColPos[e]];
+                        const bool earlier = back ? colourOf[o] > k : colourOf[o] < k;
+                        if (!earlier && !prev) continue;
+                        t = std::max(t, (earlier ? cur[o] : prev[o]) + (R > 1 && rank[o] != rank[c] ? weight : 1));
+                    }
+                    cur[c] = t;
+                }
+            });
+        }
+    }
+    nSteps = T.empty() ? 0 : *std::max_element(T.begin(), T.end()) + 1;
+    return T;
+}
+
 bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb, FlowProgram& F)
 {
     if (H.n == 0 || R < 1 || R > H.n || S < 1 || S > k::kFlowMaxVisits) return false;
@@ -450,6 +520,39 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
         valAt += P.src.size();
     }
     return true;
+}
+
+// Every hand-over of a program, replayed in step order.
+FlowHandOvers flowHandOvers(const FlowLevel& H, const FlowProgram& F)
+{
+    FlowHandOvers out;
+    std::vector<unsigned long long> stored(H.n, 0), taken(H.n, 0);
+    for (const RankProgram& P : F.prog)
+        for (const k::FlowRec& r : P.rec)
+        {
+            const unsigned char* M = P.meta.data() + 16 * static_cast<size_t>(r.meta16);
+            unsigned w[2];
+            for (int i = 0; i < r.m; ++i)
+            {
+                std::memcpy(w, M + 8 * (static_cast<size_t>(r.items8) + i), 8);
+                if (!(w[1] & 0x40000000u)) continue;
+                ++out.stored;
+                stored[w[0]] |= 1ull << (w[1] >> 16 & 0x3f);
+            }
+            for (unsigned i = 0; i < static_cast<unsigned>(r.counts) >> 16; ++i)
+            {
+                std::memcpy(w, M + 8 * (static_cast<size_t>(r.halo8) + i), 8);
+                ++out.taken;
+                taken[w[0]] |= 1ull << (w[1] >> 16);
+            }
+        }
+    for (int p = 0; p < H.n; ++p)
+        for (int q = 0; q < 64; ++q)
+        {
+            if (stored[p] & ~taken[p] & 1ull << q) ++out.unread;
+            if (taken[p] & ~stored[p] & 1ull << q) ++out.missing;
+        }
+    return out;
 }
 
 }  // namespace b2g

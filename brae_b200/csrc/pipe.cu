@@ -168,67 +168,6 @@ std::unique_ptr<PipeSchedule> assemble(const LevelHost& H, const std::vector<int
     return P;
 }
 
-// The multicolour smoother's sweeps as steps on R ranks. The colours are an order of visits like the exact
-// sweeps' cell order, so an item runs one step after the last visit it reads, `weight` steps after one of another
-// rank: only the cells near a rank's border wait for a hand-over, the others run ahead into the next colours.
-// Every row still reads its neighbours of earlier colours at this visit and the others at the one before, as the
-// colour-by-colour sweep does. Symmetric sweeps visit the colours forward then back, each cell twice a sweep.
-// Empty when a cell has no colour.
-std::vector<int> colourSteps(const FlowLevel& H, const Colouring& C, const std::vector<int>& rowPos, int nSweeps,
-                             bool symmetric, int R, int weight, int& visits, int& nSteps)
-{
-    const int n = H.n;
-    std::vector<int> colourOf(n, -1), byColour, start(1, 0);
-    byColour.reserve(n);
-    for (int k = 0; k < C.nColours; ++k)
-    {
-        for (int r = C.colourStart[k]; r < C.colourStart[k + 1]; ++r)
-            if (rowPos[r] >= 0)
-            {
-                byColour.push_back(H.posCell[rowPos[r]]);
-                colourOf[byColour.back()] = k;
-            }
-        start.push_back(static_cast<int>(byColour.size()));
-    }
-    for (int c = 0; c < n; ++c)
-        if (colourOf[c] < 0) return {};
-    visits = symmetric ? 2 * nSweeps : nSweeps;
-    std::vector<int> rank(R > 1 ? n : 0);
-    for (size_t c = 0; c < rank.size(); ++c) rank[c] = flowRank(static_cast<int>(c), n, R);
-    std::vector<int> T(static_cast<size_t>(visits) * n);
-    for (int v = 0; v < visits; ++v)
-    {
-        int* cur = T.data() + static_cast<size_t>(v) * n;
-        const int* prev = v > 0 ? cur - n : nullptr;
-        const bool back = symmetric && (v & 1);
-        for (int i = 0; i < C.nColours; ++i)
-        {
-            const int k = back ? C.nColours - 1 - i : i;
-            // a colour's cells side by side: none reads another
-            constexpr int kBlock = 16384;
-            const int from = start[k], count = start[k + 1] - from;
-            flowParallel((count + kBlock - 1) / kBlock, [&](int block, int) {
-                const int end = std::min(count, (block + 1) * kBlock);
-                for (int j = block * kBlock; j < end; ++j)
-                {
-                    const int c = byColour[from + j], p = H.cellPos[c];
-                    int t = prev ? prev[c] + 1 : 0;
-                    for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e)
-                    {
-                        const int o = H.posCell[H.entColPos[e]];
-                        const bool earlier = back ? colourOf[o] > k : colourOf[o] < k;
-                        if (!earlier && !prev) continue;
-                        t = std::max(t, (earlier ? cur[o] : prev[o]) + (R > 1 && rank[o] != rank[c] ? weight : 1));
-                    }
-                    cur[c] = t;
-                }
-            });
-        }
-    }
-    nSteps = T.empty() ? 0 : *std::max_element(T.begin(), T.end()) + 1;
-    return T;
-}
-
 template <class T>
 void allowPipeSmem()
 {
@@ -667,7 +606,11 @@ void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
     const int one = std::min(DeviceInfo::get().numSMs, (L.nCells + per - 1) / per);
     const FlowShape f = one <= 2 ? FlowShape{1, 1} : FlowShape{one, 4};
     int visits = 0, nSteps = 0;
-    const std::vector<int> T = colourSteps(H, C, rowPos, nSweeps, symmetric, f.ranks, f.weight, visits, nSteps);
+    std::vector<int> colourOf(H.n, -1);
+    for (int k = 0; k < C.nColours; ++k)
+        for (int r = C.colourStart[k]; r < C.colourStart[k + 1]; ++r)
+            if (rowPos[r] >= 0) colourOf[H.posCell[rowPos[r]]] = k;
+    const std::vector<int> T = colourSteps(H, colourOf, C.nColours, nSweeps, symmetric, f.ranks, f.weight, visits, nSteps);
     std::unique_ptr<FlowSchedule> F;
     if (!T.empty()) F = buildFlow(H, T, visits, nSteps, f.ranks, sizeof(float), stream);
     if (F)

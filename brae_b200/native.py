@@ -78,6 +78,7 @@ def _load():
         "b2g_level_grid_stall": (ip, [vp, ip, vp, vp, ip, ip, C.c_longlong]),
         "b2g_level_smooth_pipelined": (ip, [vp, ip, vp, vp, ip, ip]),
         "b2g_level_smooth_flow": (ip, [vp, ip, vp, vp, ip, ip, ip, ip, C.c_longlong, C.POINTER(C.c_float)]),
+        "b2g_flow_handovers": (ip, [ip, ip, vp, vp, vp, ip, ip, ip, ip, ip, C.POINTER(C.c_longlong)]),
         "b2g_level_pipe_shape": (ip, [vp, ip, ip, ip, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_float),
                                       C.POINTER(C.c_float), C.POINTER(C.c_float), C.POINTER(C.c_float),
                                       C.POINTER(C.c_float), C.POINTER(C.c_int)]),
@@ -159,7 +160,7 @@ EXPORTED = [
     "b2g_batch_launches", "b2g_batch_destroy", "b2g_mesh_set_pair", "b2g_mesh_level_pair",
     "b2g_gamg_solve_coupled", "b2g_matrix_create_coupled", "b2g_matrix_level_pair_coeffs", "b2g_matrix_gamg_solve",
     "b2g_matrix_set_coeffs", "b2g_matrix_level_timings", "b2g_level_smooth_stall", "b2g_set_sweep_pipeline",
-    "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
+    "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_flow_handovers", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
 ]
 
 
@@ -551,6 +552,17 @@ class Matrix(_Owner):
 def set_part_cells(cells: int) -> None:
     """The multi-part sweep's part rule for meshes created from now on (b2g_set_part_cells)."""
     _check(lib.b2g_set_part_cells(int(cells)))
+
+
+def flow_handovers(lower, upper, n_cells, n_sweeps, ranks, weight=4, symmetric=False, colours=None,
+                   value_bytes=8) -> dict:
+    """The hand-overs of the data-flow launch of these sweeps (b2g_flow_handovers; needs no device)."""
+    lower, upper = _as_host(lower, np.int32), _as_host(upper, np.int32)
+    colours = None if colours is None else _as_host(colours, np.int32)
+    n = (C.c_longlong * 4)()
+    _check(lib.b2g_flow_handovers(int(n_cells), int(lower.shape[0]), _ptr(lower), _ptr(upper), _ptr(colours),
+                                  int(n_sweeps), int(symmetric), int(ranks), int(weight), int(value_bytes), n))
+    return {"stored": n[0], "taken": n[1], "unread": n[2], "missing": n[3]}
 
 
 def set_profiling(on: bool) -> None:

@@ -410,6 +410,14 @@ B2G_API b2g_status b2g_level_smooth_pipelined(b2g_matrix* m, int level, double* 
  * (psi then holds 5 * nSweeps sweeps). B2G_ERR_ARGUMENT when the level has no such schedule. For tests and tuning. */
 B2G_API b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const double* source, int nSweeps,
                                          int symmetric, int ranks, int weight, long long stallLimit, float* ms);
+/* The hand-overs between CTAs of the data-flow launch that nSweeps sweeps of this addressing take on `ranks` CTAs
+ * (host arrays; no device needed): the exact Gauss-Seidel order, or with `colours` (a colour per cell from 0; no
+ * two cells of a colour share a face) the multicolour one. counts: values stored for another CTA, values another
+ * CTA polls for, stored values that none polls for, and polled-for values that none stores; the last two are 0 in
+ * a sound schedule. B2G_ERR_ARGUMENT when the addressing has no such schedule. Diagnostic. */
+B2G_API b2g_status b2g_flow_handovers(int nCells, int nFaces, const int32_t* lower, const int32_t* upper,
+                                      const int32_t* colours, int nSweeps, int symmetric, int ranks, int weight,
+                                      int valueBytes, long long counts[4]);
 /* psi = A^-1 source on the coarsest level by its dense Cholesky factor (device pointers, natural
  * cell order): the direct coarsest solve the FP32-preconditioned forms take (coarsestDirect).
  * B2G_ERR_ARGUMENT when the level has more than 96 cells or is not positive definite. The factor of
