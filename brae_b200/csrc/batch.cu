@@ -1294,6 +1294,7 @@ void Batch::preparePipe(int lv, int nSweeps)
             psi = reinterpret_cast<T*>(lv == 0 ? A.w32.p : A.v32.corr[lv - 1].p);
         }
         table.push_back(A.flowArgs<T>(lv, *S, psi, b));
+        ownWaits(table.back());
         B2G_CUDA(cudaStreamSynchronize(A.stream));  // its values were filled there
         caseOf.push_back(c);
         small[c] = 1;
@@ -1325,8 +1326,9 @@ void Batch::preparePipe(int lv, int nSweeps)
             P.flow[i].remote = i == 0;
             if (!v.empty()) P.flow[i].blocks.upload(v.data(), v.size(), stream);
         }
-        P.table.upload(reinterpret_cast<const unsigned char*>(table.data()), sizeof(k::FlowArgs<T>) * table.size(),
-                       stream);
+        const auto* bytes = reinterpret_cast<const unsigned char*>(table.data());
+        P.hostTable.assign(bytes, bytes + sizeof(k::FlowArgs<T>) * table.size());
+        P.table.upload(P.hostTable.data(), P.hostTable.size(), stream);
         P.caseOf.upload(caseOf.data(), caseOf.size(), stream);
         B2G_CUDA(cudaStreamSynchronize(stream));  // the host lists go out of scope
     }
@@ -1352,11 +1354,41 @@ void Batch::preparePipe(int lv, int nSweeps)
         return ms / 2.f;
     };
     P.msPipe = timeIt(true);
+    const bool gaveUp = takeError();  // (the timed sweeps are scratch: the sweep-by-sweep launches do)
     P.msSweeps = timeIt(false);
-    P.use = P.msPipe < P.msSweeps;
+    P.use = !gaveUp && P.msPipe < P.msSweeps;
     launches = l0;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+}
+
+// Whether a bounded wait has given up since the last call (the word is cleared).
+bool Batch::takeError()
+{
+    int e = 0;
+    B2G_CUDA(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    B2G_CUDA(cudaStreamSynchronize(stream));
+    if (e) err.zero(stream);
+    return e != 0;
+}
+
+void Batch::stall(long long limit)
+{
+    flowSpinLimit = limit > 0 ? limit : k::kSpinLimit;
+    flowPublish = limit > 0 ? 0 : 1;
+    auto patch = [&](BatchLevel::Pipe& P, auto T0) {
+        auto* a = reinterpret_cast<k::FlowArgs<decltype(T0)>*>(P.hostTable.data());
+        for (int i = 0; i < P.nSmall; ++i) ownWaits(a[i]);
+        if (P.nSmall)
+            B2G_CUDA(cudaMemcpyAsync(P.table.p, P.hostTable.data(), P.hostTable.size(), cudaMemcpyHostToDevice, stream));
+    };
+    for (BatchLevel& B : lev)
+        for (auto& kv : B.pipe)
+        {
+            if (kv.first % 16 == static_cast<int>(sizeof(double))) patch(kv.second, double());
+            else patch(kv.second, float());
+        }
+    B2G_CUDA(cudaStreamSynchronize(stream));
 }
 
 // Every batched pipelined sweep the controls' V-cycle makes, before the iterations run.
@@ -1717,15 +1749,9 @@ void Batch::solve(const b2g_controls& c, const double* const* source, double* co
         B2G_CUDA(cudaMemcpyAsync(psi[k], cases[k]->fc.p, sizeof(double) * cases[k]->n(0), out, stream));
     std::vector<BatchPerf> hp(K);
     B2G_CUDA(cudaMemcpyAsync(hp.data(), perf.p, sizeof(BatchPerf) * K, cudaMemcpyDeviceToHost, stream));
-    int e = 0;
-    B2G_CUDA(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    B2G_CUDA(cudaStreamSynchronize(stream));
-    if (e)
-    {
-        err.zero(stream);
+    if (takeError())
         fail(B2G_ERR_DEVICE_TIMEOUT,
              "b2g: a bounded device-side wait in the Gauss-Seidel sweep gave up; the result is invalid.");
-    }
     for (int k = 0; k < K; ++k)
     {
         perfs[k].initialResidual = hp[k].initialResidual;
@@ -1826,6 +1852,15 @@ B2G_API b2g_status b2g_batch_launches(const b2g_batch* b, long long* launches)
     return guarded([&] {
         need(b && launches, "b2g_batch_launches: null argument");
         *launches = b->batch->launches;
+    });
+}
+
+B2G_API b2g_status b2g_batch_stall(b2g_batch* b, long long spinLimit)
+{
+    return guarded([&] {
+        need(b != nullptr, "b2g_batch_stall: null batch");
+        need(spinLimit >= 0 && spinLimit <= b2g::k::kSpinLimit, "b2g_batch_stall: spinLimit out of range");
+        b->batch->stall(spinLimit);
     });
 }
 

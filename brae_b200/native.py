@@ -124,6 +124,7 @@ def _load():
         "b2g_batch_create": (ip, [C.POINTER(vp), ip, C.POINTER(vp)]),
         "b2g_batch_solve": (ip, [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(Controls), ip, C.POINTER(_Perf)]),
         "b2g_batch_launches": (ip, [vp, C.POINTER(C.c_longlong)]),
+        "b2g_batch_stall": (ip, [vp, C.c_longlong]),
         "b2g_batch_destroy": (ip, [vp]),
         "b2g_server_create": (ip, [C.c_ulonglong, ip, C.POINTER(vp)]),
         "b2g_server_destroy": (ip, [vp]),
@@ -157,7 +158,7 @@ EXPORTED = [
     "b2g_matrix_pcg_solve", "b2g_matrix_timings", "b2g_level_smooth_trace", "b2g_level_pcg_dic_static",
     "b2g_level_schedule", "b2g_level_colouring", "b2g_fold_boundary", "b2g_level_sweep_shape", "b2g_level_mc_pipe", "b2g_server_create", "b2g_server_destroy", "b2g_server_add_case",
     "b2g_server_submit", "b2g_server_wait", "b2g_server_case_bytes", "b2g_batch_create", "b2g_batch_solve",
-    "b2g_batch_launches", "b2g_batch_destroy", "b2g_mesh_set_pair", "b2g_mesh_level_pair",
+    "b2g_batch_launches", "b2g_batch_stall", "b2g_batch_destroy", "b2g_mesh_set_pair", "b2g_mesh_level_pair",
     "b2g_gamg_solve_coupled", "b2g_matrix_create_coupled", "b2g_matrix_level_pair_coeffs", "b2g_matrix_gamg_solve",
     "b2g_matrix_set_coeffs", "b2g_matrix_level_timings", "b2g_level_smooth_stall", "b2g_set_sweep_pipeline",
     "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_flow_handovers", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
@@ -772,6 +773,10 @@ class Batch(_Owner):
         perfs = (_Perf * K)()
         _check(lib.b2g_batch_solve(self.handle, src_p, psi_p, C.byref(controls), ms, perfs))
         return [SolverPerformance(p.initialResidual, p.finalResidual, p.nIterations) for p in perfs]
+
+    def stall(self, spin_limit: int) -> None:
+        """A test of the batched launches' bounded waits (b2g_batch_stall); 0 puts them back."""
+        _check(lib.b2g_batch_stall(self.handle, int(spin_limit)))
 
     def launches(self) -> int:
         v = C.c_longlong()

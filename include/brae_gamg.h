@@ -490,6 +490,12 @@ B2G_API b2g_status b2g_batch_solve(b2g_batch* batch, const double* const* source
                                    const b2g_controls* controls, int memspace, b2g_perf* perfs);
 /* Kernel launches of the last b2g_batch_solve (a graph replay counts its launches). */
 B2G_API b2g_status b2g_batch_launches(const b2g_batch* batch, long long* launches);
+/* Diagnostic, for testing that the batched smoothing launches' waits end and are reported: with spinLimit > 0
+ * (up to 2^24) no CTA of the batch's data-flow launches, as its solves so far have prepared them, hands its
+ * values over, and every wait gives up after that many polls; a solve whose cases' levels span several CTAs then
+ * returns B2G_ERR_DEVICE_TIMEOUT with psi invalid and the context still usable. 0 puts the waits back. No
+ * counterpart in the reference. */
+B2G_API b2g_status b2g_batch_stall(b2g_batch* batch, long long spinLimit);
 B2G_API b2g_status b2g_batch_destroy(b2g_batch* batch);
 
 /* ---- the serving form: many independent cases, solves queued as they arrive ------------------ */

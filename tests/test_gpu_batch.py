@@ -198,3 +198,29 @@ def test_batch_part_rule(b2g, oracle):
         assert tuple(perf) == want["perf"] and np.array_equal(psi, want["psi"])
     with pytest.raises(b2g.GamgError):
         b2g.set_part_cells(0)
+
+
+# a batch whose larger cases' levels span several CTAs of the data-flow launch
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond"])
+def test_batched_wait_gives_up(b2g, precision):
+    # no CTA hands its values over: the solve must report it (its waits' error word is the batch's own), leave the
+    # matrices' own calls alone, and the next solve of the same batch is the first one's, bit for bit
+    built, meshes, mats = _build(b2g, BOXES)
+    batch = b2g.Batch(mats)
+    ctl = b2g.controls_default(tolerance=1e-8, relTol=0.0, precision=precision)
+    srcs = [c.source for c in built]
+    first = [np.zeros(c.n_cells) for c in built]
+    perfs = batch.solve(srcs, first, ctl)
+    batch.stall(1 << 12)
+    short = b2g.controls_default(tolerance=1e-8, relTol=0.0, precision=precision, maxIter=2)
+    with pytest.raises(b2g.GamgError) as e:
+        batch.solve(srcs, [np.zeros(c.n_cells) for c in built], short)
+    assert e.value.status == "DEVICE_TIMEOUT"
+    x = np.zeros(built[4].n_cells)
+    p, _, _ = mats[4].solve(srcs[4], x, ctl)
+    assert p.finalResidual <= 1e-8
+    batch.stall(0)
+    again = [np.zeros(c.n_cells) for c in built]
+    assert batch.solve(srcs, again, ctl) == perfs
+    for a, b in zip(first, again):
+        assert np.array_equal(a, b)
