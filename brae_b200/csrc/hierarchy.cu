@@ -159,15 +159,17 @@ __global__ void kSeedFrontier(int n, const int* __restrict__ ctr, int* __restric
 // (25-40 us a round; a 260 k-cell box takes some 4,000 rounds over its levels). Every wait is bounded.
 struct FrontierLoop
 {
+    // blocks that have reached a barrier, over all rounds: 64 bits, since blocks times rounds passes 2^32 on a
+    // line of 29 M cells (a round per cell), and a wrapped count would let blocks through early
+    unsigned long long arrived;
     int size[3];       // the frontier's size by round modulo 3: this round's, the next one's, the one after
-    unsigned arrived;  // blocks that have reached a barrier, over all rounds
     int resolved;      // cells taken off the frontier, and the rounds it took
     int rounds;
     int err;           // a barrier gave up
 };
 
 // all blocks of the launch (all resident); false when the wait gave up
-__device__ bool frontierBarrier(FrontierLoop* F, unsigned& target)
+__device__ bool frontierBarrier(FrontierLoop* F, unsigned long long& target)
 {
     __shared__ int ok;
     target += gridDim.x;
@@ -176,7 +178,7 @@ __device__ bool frontierBarrier(FrontierLoop* F, unsigned& target)
     {
         ok = 1;
         __threadfence();
-        atomicAdd(&F->arrived, 1u);
+        atomicAdd(&F->arrived, 1ull);
         long long it = 0;
         while (ldAcquire(&F->arrived) < target)
             if (++it > k::kSpinLimit || ((it & 4095) == 0 && *reinterpret_cast<volatile int*>(&F->err)))
@@ -196,7 +198,7 @@ __device__ bool frontierBarrier(FrontierLoop* F, unsigned& target)
 template <bool kWarp, class Visit>
 __device__ void frontierRounds(int* fa, int* fb, FrontierLoop* F, Visit&& visit)
 {
-    unsigned target = 0;
+    unsigned long long target = 0;
     int resolved = 0, round = 0;
     constexpr int kPer = kWarp ? 32 : 1;
     const int t0 = (blockIdx.x * blockDim.x + threadIdx.x) / kPer, stride = gridDim.x * blockDim.x / kPer;
