@@ -210,25 +210,10 @@ void Matrix::flowLaunch(int level, const FlowSchedule& F, T* psiL, const T* src,
     ++launches;
 }
 
-// The mean milliseconds of a few calls, after one that fills the values.
 template <class T>
 float Matrix::flowTime(int level, const FlowSchedule& F, T* psiL, const T* src, bool fma)
 {
-    constexpr int kCalls = 3;
-    flowLaunch<T>(level, F, psiL, src, fma);
-    cudaEvent_t e0, e1;
-    B2G_CUDA(cudaEventCreate(&e0));
-    B2G_CUDA(cudaEventCreate(&e1));
-    B2G_CUDA(cudaEventRecord(e0, stream));
-    for (int i = 0; i < kCalls; ++i) flowLaunch<T>(level, F, psiL, src, fma);
-    B2G_CUDA(cudaEventRecord(e1, stream));
-    B2G_CUDA(cudaEventSynchronize(e1));
-    float ms = 0.f;
-    B2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    checkDeviceError();
-    return ms / kCalls;
+    return callTime([&] { flowLaunch<T>(level, F, psiL, src, fma); });
 }
 
 // nSweeps sweeps of `level` as one data-flow launch on `ranks` CTAs, whatever the tuned choice (for
@@ -255,9 +240,13 @@ bool Matrix::flowForced(int level, T* psiL, const T* src, int nSweeps, bool symm
     return true;
 }
 
-// The symmetric sweeps' launch of `level` (null: the level has no such schedule). Not timed against the sweeps' own launches, two and two
-// vector moves a sweep: on a 61 x 47 x 53 box those took 0.17 (33 cells) to 1.5 ms (19 k cells) a call of
-// four sweeps. Outside any capture.
+// The symmetric sweeps' launch of `level`, kept where it beats the sweeps' own launches (null else, or when the
+// level has no such schedule). Those are two walks a sweep and two vector moves; the two walks are timed, both
+// by the forward layout (the reversed one has the same depth), so that a level that takes the data flow never
+// needs the reversed one. On half the CTAs of a forward call, where they hold the level: the walks of a
+// symmetric call follow one another, so a step has a share of the items. Measured per call, half against as many
+// (FP64, boxes of 151 k and 1 M cells, their levels): 0.37 and 0.50 ms on 152 k cells, 0.34 and 0.40 on 76 k, 0.84
+// and 0.96 on 512 k, 0.67 and 0.72 on 64 k; 0.16 and 0.12 on 10 k. Outside any capture.
 template <class T>
 void Matrix::ensureSymFlow(int level, int nSweeps)
 {
@@ -271,26 +260,23 @@ void Matrix::ensureSymFlow(int level, int nSweeps)
     b.alloc(nAlloc(level), stream);
     x.zero(stream);
     b.zero(stream);
-    FlowLevel H = flowDownload(L, stream);
-    float best = 0.f;
     const long long l0 = launches;
-    // (the walks of a symmetric call follow one another, so a step has a share of the items it has in a forward
-    // call of as many sweeps: half the CTAs)
-    for (const FlowShape& f : {FlowShape{std::max(1, flowShapes(L.nCells).front().ranks / 2), 4}})
+    const float msSweeps = callTime([&] {
+        for (int w = 0; w < 2 * nSweeps; ++w) gsLaunch<T>(L, data<T>().coef[level], x.p, b.p, nullptr, false);
+    });
+    FlowLevel H = flowDownload(L, stream);
+    const int forward = flowShapes(L.nCells).front().ranks;
+    for (int ranks : {std::max(1, forward / 2), forward})
     {
         int nSteps = 0;
-        const std::vector<int> steps = flowSteps(H, nSweeps, true, f.ranks, f.weight, nSteps);
-        std::unique_ptr<FlowSchedule> F = buildFlow(H, steps, 2 * nSweeps, nSteps, f.ranks, sizeof(T), stream);
+        const std::vector<int> steps = flowSteps(H, nSweeps, true, ranks, 4, nSteps);
+        std::unique_ptr<FlowSchedule> F = buildFlow(H, steps, 2 * nSweeps, nSteps, ranks, sizeof(T), stream);
         if (!F) continue;
-        const float ms = flowTime<T>(level, *F, x.p, b.p);
-        if (!kept || ms < best)
-        {
-            best = ms;
-            if (kept) data<T>().flows.erase(kept->id);
+        if (flowTime<T>(level, *F, x.p, b.p) < msSweeps)
             kept = std::move(F);
-        }
         else
             data<T>().flows.erase(F->id);
+        break;
     }
     launches = l0;
     B2G_CUDA(cudaStreamSynchronize(stream));

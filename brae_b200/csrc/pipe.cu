@@ -20,6 +20,12 @@
 namespace b2g {
 namespace {
 
+// The share of the sweep-by-sweep time up to which a data-flow launch is taken without trying the other forms.
+// Measured per call (FP64 and FP32, all levels of boxes of 24 k to 2.4 M cells, in grid order and numbered by
+// colour): at up to 0.6 of it the best other form took 1.3 to 4 times the data flow's time; the levels above
+// it are the shallow ones (finest level numbered by colour, 13 steps: sweeps 29 us, grid form 17, data flow 38 on
+// 24 k cells; 79, 44 and 56 on 262 k), where the others win.
+constexpr float kFlowClear = 0.6f;
 constexpr int kMcFlowCells = 600000;  // the largest level whose colours are tried as a data flow
 constexpr size_t kPipeSmemCap = 220 * 1024;  // dynamic shared memory of one rank: its psi slots and step table
 
@@ -404,9 +410,10 @@ void Matrix::itemsLaunch(int level, const GsSchedule& G, T* psiL, const T* src)
 }
 
 // The pipelined smoothing call of `level` for nSweeps sweeps, tried once per (level, sweep count,
-// value type) on this matrix's values: every shared-memory shape whose slots fit (one CTA; clusters
-// of 2, 4, 8, 16 CTAs that can be resident) and, on a multi-part level, the item schedule, against
-// the sweep-by-sweep launches; the fastest is kept. Every shape computes every row from the same
+// value type) on this matrix's values: the data-flow launch on a few CTA counts against the sweep-by-sweep
+// launches and, unless it is far faster than those (kFlowClear), every shared-memory shape whose slots
+// fit (one CTA; clusters of 2, 4, 8, 16 CTAs that can be resident) and, on a multi-part level, the grid form
+// and the item schedule; the fastest tried is kept. Every shape computes every row from the same
 // operands in the same order, so the choice changes the time only. Outside any capture (it
 // synchronises); the work vectors it sweeps are scratch.
 template <class T>
@@ -456,9 +463,10 @@ void Matrix::ensurePipe(int level, int nSweeps)
             const long long id = F->id;
             const float ms = timeIt([&] { flowLaunch<T>(level, *F, x.p, b.p); });
             checkDeviceError();
-            if (C.mode != 3 || ms < C.msFlow)
+            if (C.msFlow == 0.f || ms < C.msFlow) C.msFlow = ms;
+            if (ms < best)
             {
-                C.msFlow = ms;
+                best = ms;
                 if (C.flow) data<T>().flows.erase(C.flow->id);
                 C.flow = std::move(F);
                 C.mode = 3;
@@ -467,7 +475,12 @@ void Matrix::ensurePipe(int level, int nSweeps)
                 data<T>().flows.erase(id);
         }
     }
-    if (C.mode != 3 && L.nCells <= k::kPipeMaxRanks * static_cast<int>(kPipeSmemCap / sizeof(T)))
+    const bool others = C.mode != 3 || best > kFlowClear * C.msSweeps;
+    auto dropFlow = [&] {
+        if (C.flow) data<T>().flows.erase(C.flow->id);
+        C.flow.reset();
+    };
+    if (others && L.nCells <= k::kPipeMaxRanks * static_cast<int>(kPipeSmemCap / sizeof(T)))
     {
         const LevelHost H = download(L, stream);
         int nSteps = 0;
@@ -483,11 +496,12 @@ void Matrix::ensurePipe(int level, int nSweeps)
             {
                 best = ms;
                 C.sched = std::move(P);
+                dropFlow();
                 C.mode = 1;
             }
         }
     }
-    if (C.mode != 3 && L.gs.nParts > 1)
+    if (others && L.gs.nParts > 1)
     {
         // the grid form: one CTA per SM, or per two
         const LevelHost H = download(L, stream);
@@ -516,6 +530,7 @@ void Matrix::ensurePipe(int level, int nSweeps)
             {
                 best = ms;
                 C.sched = std::move(P);
+                dropFlow();
                 C.mode = 1;
             }
         }
@@ -544,6 +559,7 @@ void Matrix::ensurePipe(int level, int nSweeps)
                 best = ms;
                 C.items = std::move(G);
                 C.sched.reset();
+                dropFlow();
                 C.mode = 2;
             }
             else

@@ -206,6 +206,26 @@ struct Matrix
     template <class T> k::FlowArgs<T> flowArgs(int level, const FlowSchedule& F, T* psi, const T* source);
     template <class T> void flowLaunch(int level, const FlowSchedule& F, T* psi, const T* source, bool fma = false);
     template <class T> bool flowForced(int level, T* psi, const T* source, int nSweeps, bool symmetric, int ranks, int weight, float* ms);
+    // the mean milliseconds of a few calls, after one that fills what is filled on first use
+    template <class Call>
+    float callTime(Call&& call)
+    {
+        constexpr int kCalls = 3;
+        call();
+        cudaEvent_t e0, e1;
+        B2G_CUDA(cudaEventCreate(&e0));
+        B2G_CUDA(cudaEventCreate(&e1));
+        B2G_CUDA(cudaEventRecord(e0, stream));
+        for (int i = 0; i < kCalls; ++i) call();
+        B2G_CUDA(cudaEventRecord(e1, stream));
+        B2G_CUDA(cudaEventSynchronize(e1));
+        float ms = 0.f;
+        B2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        checkDeviceError();
+        return ms / kCalls;
+    }
     template <class T> float flowTime(int level, const FlowSchedule& F, T* psi, const T* source, bool fma = false);
     template <class T> void ensureSymFlow(int level, int nSweeps);
     template <class T> bool symFlowSweeps(int level, T* psi, const T* source, int nSweeps);

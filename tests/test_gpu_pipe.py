@@ -185,3 +185,49 @@ def test_grid_form_wait_gives_up(b2g, oracle):
     x = dev(x0)
     A.smooth_pipelined(1, x, dev(b), 2, sms)
     assert np.array_equal(x.cpu().numpy(), oracle.smooth(lo, up, d, u, x0, b, 2))
+
+
+def _by_colour(c, nx, ny):
+    """The box's cells numbered red first, then black: every level-0 walk is two steps deep."""
+    idx = np.arange(c.n_cells)
+    red = (idx % nx + idx // nx % ny + idx // (nx * ny)) % 2
+    order = np.lexsort((idx, red))
+    new = np.empty(c.n_cells, np.int64)
+    new[order] = idx
+    lo, up = np.minimum(new[c.lower], new[c.upper]), np.maximum(new[c.lower], new[c.upper])
+    f = np.lexsort((up, lo))
+    return lo[f].astype(np.int32), up[f].astype(np.int32), c.Sf[f], c.magSf[f], c.diag[order], c.coef[f], c.source[order]
+
+
+@pytest.mark.parametrize("smoother", ["GaussSeidel", "symGaussSeidel"])
+@pytest.mark.parametrize("precision,value_bytes", [("fp64", 8), ("fp32_precond", 4)])
+def test_tuner_keeps_nothing_slower_than_the_sweeps(b2g, oracle, smoother, precision, value_bytes):
+    # a level whose sweeps are two steps deep, where a launch a sweep is bound by bandwidth and the data flow has
+    # nothing to overlap, and the deep levels below it: whatever the tuner keeps, it measured no slower than the
+    # sweep-by-sweep launches, and the field is the one those give
+    nx, ny, nz = 46, 23, 23
+    c = cases.box_case(nx, ny, nz, (2.0, 1.0, 1.0), 20.0)
+    lo, up, Sf, magSf, diag, coef, source = _by_colour(c, nx, ny)
+    mesh = b2g.Mesh(lo, up, Sf, magSf, c.n_cells, 10, True)
+    ctl = b2g.controls_default(tolerance=1e-8, relTol=0.0, precision=precision, smoother=smoother)
+    out = {}
+    try:
+        for on in (True, False):
+            b2g.set_sweep_pipeline(on)
+            psi = np.zeros(c.n_cells)
+            perf = b2g.pcg_gamg_solve(mesh, diag, coef, source, psi, ctl)[0]
+            out[on] = (psi, tuple(perf))
+    finally:
+        b2g.set_sweep_pipeline(True)
+    assert out[True][1] == out[False][1]
+    assert np.array_equal(out[True][0], out[False][0])
+    if smoother != "GaussSeidel":
+        return
+    tuned = 0
+    for lv in range(mesh.n_levels):
+        s = mesh.pipe_shape(lv, 2 if lv == 0 else min(2 + lv - 1, 4), value_bytes)
+        assert s["ms_sweep_by_sweep"] > 0.0, lv
+        if s["ranks"]:
+            assert s["ms_pipelined"] <= s["ms_sweep_by_sweep"], (lv, s)
+            tuned += 1
+    assert tuned > 3
