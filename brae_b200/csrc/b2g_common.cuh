@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <new>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -107,6 +108,26 @@ struct DBuf
     T* get() const { return p; }
     size_t bytes() const { return n * sizeof(T); }
 };
+
+// Runs body; false when it failed: out of memory, a launch refused, a bounded wait that gave up. For attempts at a
+// faster form of work that has another.
+template <class Body>
+bool attempt(Body&& body)
+{
+    try
+    {
+        body();
+        return true;
+    }
+    catch (const Error&)
+    {
+        cudaGetLastError();
+    }
+    catch (const std::bad_alloc&)
+    {
+    }
+    return false;
+}
 
 inline int ceilDiv(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 

@@ -1293,6 +1293,7 @@ void Batch::preparePipe(int lv, int nSweeps)
             b = reinterpret_cast<const T*>(lv == 0 ? A.r32.p : A.v32.src[lv - 1].p);
             psi = reinterpret_cast<T*>(lv == 0 ? A.w32.p : A.v32.corr[lv - 1].p);
         }
+        if (!A.flowReady<T>(lv, *S)) continue;
         table.push_back(A.flowArgs<T>(lv, *S, psi, b));
         ownWaits(table.back());
         B2G_CUDA(cudaStreamSynchronize(A.stream));  // its values were filled there
@@ -1353,8 +1354,8 @@ void Batch::preparePipe(int lv, int nSweeps)
         B2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         return ms / 2.f;
     };
-    P.msPipe = timeIt(true);
-    const bool gaveUp = takeError();  // (the timed sweeps are scratch: the sweep-by-sweep launches do)
+    // (the timed sweeps are scratch: the sweep-by-sweep launches do)
+    const bool gaveUp = !attempt([&] { P.msPipe = timeIt(true); }) || takeError();
     P.msSweeps = timeIt(false);
     P.use = !gaveUp && P.msPipe < P.msSweeps;
     launches = l0;

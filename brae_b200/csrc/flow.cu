@@ -158,6 +158,22 @@ const T* Matrix::flowValuesOf(int level, const FlowSchedule& F)
     return B.val.p;
 }
 
+// Whether this matrix has the schedule's values, filled here outside a capture; false when there is no memory
+// for them, and the level then runs its other form (tried again with the next solve).
+template <class T>
+bool Matrix::flowReady(int level, const FlowSchedule& F)
+{
+    auto& flows = data<T>().flows;
+    const auto it = flows.find(F.id);
+    if (it != flows.end() && it->second.gen == coefGen) return true;
+    if (capturing && it != flows.end() && it->second.refused == coefGen) return false;
+    if (attempt([&] { flowValuesOf<T>(level, F); })) return true;
+    if (capturing) fail(B2G_ERR_STATE, "b2g: a smoothing schedule's values were not filled before the capture");
+    flows.erase(F.id);
+    flows[F.id].refused = coefGen;
+    return false;
+}
+
 template <class T>
 k::FlowArgs<T> Matrix::flowArgs(int level, const FlowSchedule& F, T* psiL, const T* src)
 {
@@ -256,8 +272,11 @@ void Matrix::ensureSymFlow(int level, int nSweeps)
     std::unique_ptr<FlowSchedule>& kept = L.flowSym[key];
     if (nSweeps < 1 || L.nCells == 0) return;
     DBuf<T> x, b;
-    x.alloc(nAlloc(level), stream);
-    b.alloc(nAlloc(level), stream);
+    if (!attempt([&] {
+            x.alloc(nAlloc(level), stream);
+            b.alloc(nAlloc(level), stream);
+        }))
+        return;
     x.zero(stream);
     b.zero(stream);
     const long long l0 = launches;
@@ -268,11 +287,16 @@ void Matrix::ensureSymFlow(int level, int nSweeps)
     const int forward = flowShapes(L.nCells).front().ranks;
     for (int ranks : {std::max(1, forward / 2), forward})
     {
-        int nSteps = 0;
-        const std::vector<int> steps = flowSteps(H, nSweeps, true, ranks, 4, nSteps);
-        std::unique_ptr<FlowSchedule> F = buildFlow(H, steps, 2 * nSweeps, nSteps, ranks, sizeof(T), stream);
+        std::unique_ptr<FlowSchedule> F;
+        float ms = 0.f;
+        const bool ran = attempt([&] {
+            int nSteps = 0;
+            const std::vector<int> steps = flowSteps(H, nSweeps, true, ranks, 4, nSteps);
+            F = buildFlow(H, steps, 2 * nSweeps, nSteps, ranks, sizeof(T), stream);
+            if (F) ms = flowTime<T>(level, *F, x.p, b.p);
+        });
         if (!F) continue;
-        if (flowTime<T>(level, *F, x.p, b.p) < msSweeps)
+        if (ran && ms < msSweeps)
             kept = std::move(F);
         else
             data<T>().flows.erase(F->id);
@@ -296,7 +320,7 @@ bool Matrix::symFlowSweeps(int level, T* psiL, const T* src, int nSweeps)
         ensureSymFlow<T>(level, nSweeps);
         it = L.flowSym.find(key);
     }
-    if (!it->second) return false;
+    if (!it->second || !flowReady<T>(level, *it->second)) return false;
     flowLaunch<T>(level, *it->second, psiL, src);
     return true;
 }
@@ -307,7 +331,7 @@ void Matrix::refreshSymFlows()
 {
     for (int lv = 0; lv <= nLevels(); ++lv)
         for (auto& kv : mesh->lev[lv].flowSym)
-            if (kv.second && kv.first % 16 == static_cast<int>(sizeof(T))) flowValuesOf<T>(lv, *kv.second);
+            if (kv.second && kv.first % 16 == static_cast<int>(sizeof(T))) flowReady<T>(lv, *kv.second);
 }
 
 void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStream_t s)
@@ -329,18 +353,21 @@ void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStrea
         jobs[i].level->flowBatch[keyOf(jobs[i])];  // (a level listed twice is built once)
         work.emplace_back();
         work.back().job = i;
-        work.back().H = flowDownload(*jobs[i].level, s);
+        // (no memory for it, here and below: the level has no schedule)
+        if (!attempt([&] { work.back().H = flowDownload(*jobs[i].level, s); })) work.pop_back();
     }
     flowParallel(static_cast<int>(work.size()), [&](int i, int) {
         Work& w = work[i];
         const int R = jobs[w.job].ranks;
-        const std::vector<int> steps = flowSteps(w.H, nSweeps, false, R, 4, w.nSteps);
-        w.ok = buildFlowProgram(w.H, steps, nSweeps, w.nSteps, R, vb, w.G);
+        attempt([&] {
+            const std::vector<int> steps = flowSteps(w.H, nSweeps, false, R, 4, w.nSteps);
+            w.ok = buildFlowProgram(w.H, steps, nSweeps, w.nSteps, R, vb, w.G);
+        });
     });
     for (Work& w : work)
     {
         const FlowJob& j = jobs[w.job];
-        if (w.ok) j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, nSweeps, w.nSteps, j.ranks, s);
+        if (w.ok) attempt([&] { j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, nSweeps, w.nSteps, j.ranks, s); });
     }
     for (FlowJob& j : jobs) j.flow = j.level->flowBatch[keyOf(j)].get();
 }
@@ -381,6 +408,8 @@ template float Matrix::flowTime<double>(int, const FlowSchedule&, double*, const
 template float Matrix::flowTime<float>(int, const FlowSchedule&, float*, const float*, bool);
 template void Matrix::flowLaunch<double>(int, const FlowSchedule&, double*, const double*, bool);
 template void Matrix::flowLaunch<float>(int, const FlowSchedule&, float*, const float*, bool);
+template bool Matrix::flowReady<double>(int, const FlowSchedule&);
+template bool Matrix::flowReady<float>(int, const FlowSchedule&);
 template const double* Matrix::flowValuesOf<double>(int, const FlowSchedule&);
 template const float* Matrix::flowValuesOf<float>(int, const FlowSchedule&);
 

@@ -426,8 +426,11 @@ void Matrix::ensurePipe(int level, int nSweeps)
     if (nSweeps < 2 || L.nCells == 0) return;
     allowPipeSmem<T>();
     DBuf<T> x, b;
-    x.alloc(nAlloc(level), stream);
-    b.alloc(nAlloc(level), stream);
+    if (!attempt([&] {
+            x.alloc(nAlloc(level), stream);
+            b.alloc(nAlloc(level), stream);
+        }))
+        return;
     x.zero(stream);
     b.zero(stream);
     cudaEvent_t e0, e1;
@@ -456,15 +459,19 @@ void Matrix::ensurePipe(int level, int nSweeps)
         FlowLevel H = flowDownload(L, stream);
         for (const FlowShape& f : flowShapes(L.nCells))
         {
-            int nSteps = 0;
-            const std::vector<int> steps = flowSteps(H, nSweeps, false, f.ranks, f.weight, nSteps);
-            std::unique_ptr<FlowSchedule> F = buildFlow(H, steps, nSweeps, nSteps, f.ranks, sizeof(T), stream);
+            std::unique_ptr<FlowSchedule> F;
+            float ms = 0.f;
+            const bool ran = attempt([&] {
+                int nSteps = 0;
+                const std::vector<int> steps = flowSteps(H, nSweeps, false, f.ranks, f.weight, nSteps);
+                F = buildFlow(H, steps, nSweeps, nSteps, f.ranks, sizeof(T), stream);
+                if (F) ms = timeIt([&] { flowLaunch<T>(level, *F, x.p, b.p); });
+                checkDeviceError();
+            });
             if (!F) continue;
             const long long id = F->id;
-            const float ms = timeIt([&] { flowLaunch<T>(level, *F, x.p, b.p); });
-            checkDeviceError();
-            if (C.msFlow == 0.f || ms < C.msFlow) C.msFlow = ms;
-            if (ms < best)
+            if (ran && (C.msFlow == 0.f || ms < C.msFlow)) C.msFlow = ms;
+            if (ran && ms < best)
             {
                 best = ms;
                 if (C.flow) data<T>().flows.erase(C.flow->id);
@@ -487,10 +494,14 @@ void Matrix::ensurePipe(int level, int nSweeps)
         const std::vector<int> Tsteps = combinedSteps(H, nSweeps, nSteps);
         for (int R : {1, 2, 4, 8, 16})
         {
-            std::unique_ptr<PipeSchedule> P = assemble(H, Tsteps, nSweeps, nSteps, R, sizeof(T), stream);
-            if (!P) continue;
-            if (R > 1 && !pipeClusterFits<T>(R, pipeSmemBytes(*P, sizeof(T)), stream)) continue;
-            const float ms = timeIt([&] { pipeLaunch<T>(level, *P, x.p, b.p); });
+            std::unique_ptr<PipeSchedule> P;
+            float ms = 0.f;
+            const bool ran = attempt([&] {
+                P = assemble(H, Tsteps, nSweeps, nSteps, R, sizeof(T), stream);
+                if (P && R > 1 && !pipeClusterFits<T>(R, pipeSmemBytes(*P, sizeof(T)), stream)) P.reset();
+                if (P) ms = timeIt([&] { pipeLaunch<T>(level, *P, x.p, b.p); });
+            });
+            if (!P || !ran) continue;
             if (C.msPipe == 0.f || ms < C.msPipe) C.msPipe = ms;
             if (ms < best)
             {
@@ -511,20 +522,16 @@ void Matrix::ensurePipe(int level, int nSweeps)
         for (int R : {sms, sms / 2})
         {
             if (R < 2 || R > L.nCells) continue;
-            std::unique_ptr<PipeSchedule> P = assemble(H, Tsteps, nSweeps, nSteps, R, sizeof(T), stream, true);
-            if (!P || !pipeGridFits<T>(R, pipeSmemBytes(*P, sizeof(T)))) continue;
+            std::unique_ptr<PipeSchedule> P;
             float ms = 0.f;
-            try
-            {
+            const bool ran = attempt([&] {
+                P = assemble(H, Tsteps, nSweeps, nSteps, R, sizeof(T), stream, true);
+                if (P && !pipeGridFits<T>(R, pipeSmemBytes(*P, sizeof(T)))) P.reset();
+                if (!P) return;
                 ms = timeIt([&] { pipeLaunch<T>(level, *P, x.p, b.p); });
                 checkDeviceError();
-            }
-            catch (const Error&)
-            {
-                // a cooperative launch of that many CTAs refused here
-                cudaGetLastError();
-                continue;
-            }
+            });
+            if (!P || !ran) continue;
             if (C.msGrid == 0.f || ms < C.msGrid) C.msGrid = ms;
             if (ms < best)
             {
@@ -534,22 +541,17 @@ void Matrix::ensurePipe(int level, int nSweeps)
                 C.mode = 1;
             }
         }
-        std::unique_ptr<GsSchedule> G = buildGsItems(L, nSweeps, stream);
+        std::unique_ptr<GsSchedule> G;
         float ms = 0.f;
-        if (G)
-        {
-            try
-            {
+        if (!attempt([&] {
+                G = buildGsItems(L, nSweeps, stream);
+                if (!G) return;
                 ms = timeIt([&] { itemsLaunch<T>(level, *G, x.p, b.p); });
                 checkDeviceError();
-            }
-            catch (const Error&)
-            {
-                // a cooperative launch of that many parts refused here: no item schedule for the level
-                cudaGetLastError();
-                G.reset();
-                data<T>().items.erase(std::make_pair(level, nSweeps));
-            }
+            }))
+        {
+            G.reset();
+            data<T>().items.erase(std::make_pair(level, nSweeps));
         }
         if (G)
         {
@@ -593,7 +595,7 @@ void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
     auto known = C.pipe.find(key);
     if (known != C.pipe.end())
     {
-        if (known->second.use) flowValuesOf<float>(level, *known->second.flow);
+        if (known->second.use) flowReady<float>(level, *known->second.flow);
         return;
     }
     Colouring::Pipe& M = C.pipe[key];
@@ -626,13 +628,15 @@ void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
     for (int k = 0; k < C.nColours; ++k)
         for (int r = C.colourStart[k]; r < C.colourStart[k + 1]; ++r)
             if (rowPos[r] >= 0) colourOf[H.posCell[rowPos[r]]] = k;
-    const std::vector<int> T = colourSteps(H, colourOf, C.nColours, nSweeps, symmetric, f.ranks, f.weight, visits, nSteps);
     std::unique_ptr<FlowSchedule> F;
-    if (!T.empty()) F = buildFlow(H, T, visits, nSteps, f.ranks, sizeof(float), stream);
+    const bool ran = attempt([&] {
+        const std::vector<int> T = colourSteps(H, colourOf, C.nColours, nSweeps, symmetric, f.ranks, f.weight, visits, nSteps);
+        if (!T.empty()) F = buildFlow(H, T, visits, nSteps, f.ranks, sizeof(float), stream);
+        if (F) M.msPipe = flowTime<float>(level, *F, x, b, true);
+    });
     if (F)
     {
-        M.msPipe = flowTime<float>(level, *F, x, b, true);
-        M.use = M.msPipe < M.msColours;
+        M.use = ran && M.msPipe < M.msColours;
         if (M.use)
             M.flow = std::move(F);
         else
@@ -653,7 +657,7 @@ void Matrix::refreshItems()
         {
             if (kv.first % 16 != static_cast<int>(sizeof(T))) continue;
             if (kv.second.mode == 2) itemBuffers<T>(lv, *kv.second.items);
-            if (kv.second.mode == 3) flowValuesOf<T>(lv, *kv.second.flow);
+            if (kv.second.mode == 3) flowReady<T>(lv, *kv.second.flow);
         }
 }
 
@@ -682,7 +686,7 @@ bool Matrix::pipeSweeps(int level, T* psiL, const T* src, int nSweeps)
         itemsLaunch<T>(level, *C.items, psiL, src);
         return true;
     }
-    if (C.mode == 3)
+    if (C.mode == 3 && flowReady<T>(level, *C.flow))
     {
         flowLaunch<T>(level, *C.flow, psiL, src);
         return true;

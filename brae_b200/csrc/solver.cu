@@ -1116,7 +1116,11 @@ void Matrix::prepareSmoother(const b2g_controls& c)
     auto symLaunches = [&](int level, size_t valueBytes) {
         bool all = g_pipeline && !mesh->lev[level].flowSym.empty();
         for (const auto& kv : mesh->lev[level].flowSym)
-            if (kv.first % 16 == static_cast<int>(valueBytes) && !kv.second) all = false;
+        {
+            if (kv.first % 16 != static_cast<int>(valueBytes)) continue;
+            if (!kv.second) all = false;
+            else if (!(valueBytes == 8 ? flowReady<double>(level, *kv.second) : flowReady<float>(level, *kv.second))) all = false;
+        }
         return all;
     };
     for (int i = 0; i < nLevels(); ++i)
@@ -1261,7 +1265,7 @@ void Matrix::mcSmooth(int level, float* psiL, const float* src, int nSweeps, boo
     const Colouring& C = mesh->lev[level].mc;
     // the call as one pipelined launch over the colours, where that measured faster (ensureMcPipe)
     const auto it = C.pipe.find(nSweeps * 2 + (symmetric ? 1 : 0));
-    if (g_pipeline && it != C.pipe.end() && it->second.use)
+    if (g_pipeline && it != C.pipe.end() && it->second.use && flowReady<float>(level, *it->second.flow))
     {
         flowLaunch<float>(level, *it->second.flow, psiL, src, true);
         return;

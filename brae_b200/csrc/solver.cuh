@@ -75,6 +75,7 @@ struct VCycleData
         DBuf<unsigned char> mail;   // {value, tag} by position, and the launch counter with the ranks that
         DBuf<unsigned> ctl;         // have finished (more than one rank)
         long long gen = -1;
+        long long refused = -1;     // the generation whose values found no memory (flowReady)
     };
     std::map<long long, FlowBuffers> flows;
     // FP32 form only: dense Cholesky of the coarsest level
@@ -203,6 +204,7 @@ struct Matrix
     template <class T> void refreshItems();
     // the data-flow launch of a smoothing call (flow.cu)
     template <class T> const T* flowValuesOf(int level, const FlowSchedule& F);
+    template <class T> bool flowReady(int level, const FlowSchedule& F);
     template <class T> k::FlowArgs<T> flowArgs(int level, const FlowSchedule& F, T* psi, const T* source);
     template <class T> void flowLaunch(int level, const FlowSchedule& F, T* psi, const T* source, bool fma = false);
     template <class T> bool flowForced(int level, T* psi, const T* source, int nSweeps, bool symmetric, int ranks, int weight, float* ms);

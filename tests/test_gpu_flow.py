@@ -184,3 +184,57 @@ def test_solve_at_transfer_edges(b2g, oracle, nx, ny, nz):
         again = dev(np.zeros(c.n_cells))
         A.solve(dev(c.source), again, b2g.controls_default(tolerance=1e-8))
         assert torch.equal(again, x)
+
+
+_FULL_DEVICE = """
+import sys
+sys.path.insert(0, {repo!r})
+import numpy as np
+import torch
+import brae_b200.native as b
+from brae_b200 import cases
+
+c = cases.box_case(180, 110, 100, (2.0, 1.0, 1.0), 5.0)
+mesh = b.Mesh(c.lower, c.upper, c.Sf, c.magSf, c.n_cells, 10, True)
+A = b.Matrix(mesh, c.diag, c.coef)
+batch_mesh = b.Mesh(c.lower, c.upper, c.Sf, c.magSf, c.n_cells, 10, True)
+batch = b.Batch([b.Matrix(batch_mesh, c.diag, c.coef)])
+forms = [(p, s) for p in ("fp64", "fp32_precond", "fp32_precond_multicolour") for s in ("GaussSeidel", "symGaussSeidel")]
+
+
+def solve_all():
+    out = {{}}
+    for p, s in forms:
+        ctl = b.controls_default(tolerance=1e-12, relTol=0.0, precision=p, smoother=s, maxIter=2)
+        psi = np.zeros(c.n_cells)
+        A.solve(c.source, psi, ctl)
+        out[p, s] = psi
+        if s == "GaussSeidel":
+            psi = np.zeros(c.n_cells)
+            batch.solve([c.source], [psi], ctl)
+            out[p, "batch"] = psi
+    return out
+
+
+# everything but the smoothing calls' schedules is there once these have run
+b.set_sweep_pipeline(False)
+want = solve_all()
+torch.cuda.synchronize()
+free, _ = torch.cuda.mem_get_info()
+hold = torch.empty(free - (160 << 20), dtype=torch.uint8, device="cuda")
+b.set_sweep_pipeline(True)
+got = solve_all()
+assert all(np.array_equal(want[k], got[k]) for k in want), [k for k in want if not np.array_equal(want[k], got[k])]
+print("SAME", mesh.pipe_shape(0, 2, 8)["ranks"])
+"""
+
+
+def test_no_memory_takes_the_other_forms():
+    # a device that has no room for the finest levels' schedules (2 M cells: 0.7 GB and more each): every form
+    # solves as it does without them, bit for bit. In a process of its own, whose memory pool holds nothing else.
+    import os
+    import subprocess
+    import sys
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _FULL_DEVICE.format(repo=repo)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "SAME" in r.stdout, (r.stdout[-500:], r.stderr[-1500:])
