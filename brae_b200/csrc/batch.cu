@@ -1295,7 +1295,7 @@ void Batch::preparePipe(int lv, int nSweeps)
         }
         if (!A.flowReady<T>(lv, *S)) continue;
         table.push_back(A.flowArgs<T>(lv, *S, psi, b));
-        ownWaits(table.back());
+        ownWaits(table.back(), *S);
         B2G_CUDA(cudaStreamSynchronize(A.stream));  // its values were filled there
         caseOf.push_back(c);
         small[c] = 1;
@@ -1373,13 +1373,21 @@ bool Batch::takeError()
     return e != 0;
 }
 
+template <class T>
+void Batch::ownWaits(k::FlowArgs<T>& a, const FlowSchedule& F) const
+{
+    a.err = err.p;
+    a.spinLimit = flowSpinLimit(spinLimit, F);
+    a.publish = flowPublish;
+}
+
 void Batch::stall(long long limit)
 {
-    flowSpinLimit = limit > 0 ? limit : k::kSpinLimit;
+    spinLimit = limit > 0 ? limit : k::kSpinLimit;
     flowPublish = limit > 0 ? 0 : 1;
     auto patch = [&](BatchLevel::Pipe& P, auto T0) {
         auto* a = reinterpret_cast<k::FlowArgs<decltype(T0)>*>(P.hostTable.data());
-        for (int i = 0; i < P.nSmall; ++i) ownWaits(a[i]);
+        for (int i = 0; i < P.nSmall; ++i) ownWaits(a[i], *P.flows[i].second);
         if (P.nSmall)
             B2G_CUDA(cudaMemcpyAsync(P.table.p, P.hostTable.data(), P.hostTable.size(), cudaMemcpyHostToDevice, stream));
     };

@@ -149,19 +149,15 @@ struct Batch
     template <class T> void preparePipe(int lv, int nSweeps);
     void preparePipes(const b2g_controls& c);
     bool pipeOn = false;                    // the current solve takes the batched pipelined sweeps
-    // The waits of the data-flow launches report to the batch's own error word, which solve reads.
-    long long flowSpinLimit = k::kSpinLimit;
+    // The waits of the data-flow launches are the batch's own (ownWaits): they report to its error word, which
+    // solve reads.
+    long long spinLimit = k::kSpinLimit;
     int flowPublish = 1;
     // A test of those waits: with limit > 0 no CTA of the tables in place hands its values over and every wait
     // gives up after that many polls; 0 puts them back.
     void stall(long long limit);
     bool takeError();
-    template <class T> void ownWaits(k::FlowArgs<T>& a) const
-    {
-        a.err = err.p;
-        a.spinLimit = flowSpinLimit;
-        a.publish = flowPublish;
-    }
+    template <class T> void ownWaits(k::FlowArgs<T>& a, const FlowSchedule& F) const;
     DBuf<int> active;                       // [K]
     DBuf<int> nActive;                      // [1]
     DBuf<int> err;

@@ -189,7 +189,7 @@ k::FlowArgs<T> Matrix::flowArgs(int level, const FlowSchedule& F, T* psiL, const
     a.ctl = B.ctl.p;
     a.ranks = F.ranks;
     a.slots = F.slots;
-    a.spinLimit = spinLimit;
+    a.spinLimit = flowSpinLimit(spinLimit, F);
     a.err = err.p;
     a.publish = publish;
     return a;

@@ -85,6 +85,15 @@ struct FlowShape
     int ranks, weight;
 };
 std::vector<FlowShape> flowShapes(int n);
+// The polls after which a wait of a launch gives up. The last rank may wait until the front has passed all
+// others, nearly all of the launch's steps: at 0.45-0.8 us a step that is longer than kSpinLimit polls of shared
+// memory (1.5 s, measured) from about 2 M steps on, a line of as many cells, say. kPollsPerStep polls take some
+// 90 us. A limit set for a test is taken as it is.
+constexpr long long kPollsPerStep = 1024;
+inline long long flowSpinLimit(long long limit, const FlowSchedule& F)
+{
+    return limit == k::kSpinLimit ? limit + kPollsPerStep * F.nSteps : limit;
+}
 // whether a launch of that many ranks can be resident (one CTA per SM)
 bool flowFits(int ranks);
 

@@ -238,3 +238,17 @@ def test_no_memory_takes_the_other_forms():
     repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _FULL_DEVICE.format(repo=repo)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "SAME" in r.stdout, (r.stdout[-500:], r.stderr[-1500:])
+
+
+def test_long_chain_of_steps(b2g):
+    # a line of cells is one chain of steps: the last CTA waits for nearly all of them without taking that for a
+    # stall; the result is the sweep-by-sweep one
+    n = 200_000
+    c = cases.box_case(n, 1, 1)
+    mesh, A = _build(b2g, c)
+    rng = np.random.default_rng(8)
+    x0, b = dev(rng.uniform(-1.0, 1.0, n)), dev(rng.uniform(-1.0, 1.0, n))
+    x, want = x0.clone(), x0.clone()
+    A.smooth_flow(0, x, b, 1, torch.cuda.get_device_properties(0).multi_processor_count, 4)
+    A.smooth(0, want, b, 1)  # one sweep: no data flow
+    assert torch.equal(x, want)
