@@ -449,9 +449,11 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
             {
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + ((j - 1) & 1)), "n"(64 * kTeamWarps) : "memory");
                 // (never after a stop: the chunks that a stopped warp skipped may still be read by the other
-                // roles, see LIMITS. The last warp publishes, since it has no row in a chunk of fewer slices)
+                // roles, see LIMITS. A release, which carries the reads that the barrier has gathered to the
+                // producer's acquire: measured within 0.3 % of a plain store on solves of 24 k to 1 M cells. By the
+                // last warp, which has no row and no mailbox stores under way in a chunk of fewer slices)
                 if (wi == kTeamWarps - 1 && lane == 0 && *reinterpret_cast<volatile unsigned*>(&S.stop) == 0)
-                    *reinterpret_cast<volatile unsigned*>(&S.consumed) = static_cast<unsigned>(j);
+                    stReleaseCta(&S.consumed, static_cast<unsigned>(j));
             }
             if (kRemote && ok && !haloOk)
                 ok = flowWait(S, a.err, a.spinLimit, [&] { return hasHalo(j); });
