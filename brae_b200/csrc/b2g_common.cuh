@@ -19,7 +19,8 @@ namespace b2g {
 struct Error : std::runtime_error
 {
     b2g_status code;
-    Error(b2g_status c, const std::string& m) : std::runtime_error(m), code(c) {}
+    bool deviceMemory = false;  // the device had no room (not an admission cap, nor host memory)
+    Error(b2g_status c, const std::string& m, bool dm = false) : std::runtime_error(m), code(c), deviceMemory(dm) {}
 };
 
 [[noreturn]] inline void fail(b2g_status c, const std::string& m) { throw Error(c, m); }
@@ -28,9 +29,11 @@ inline void cudaCheck(cudaError_t e, const char* what, const char* file, int lin
 {
     if (e != cudaSuccess)
     {
-        const b2g_status st = (e == cudaErrorMemoryAllocation) ? B2G_ERR_NO_MEMORY : B2G_ERR_CUDA;
-        fail(st, std::string("b2g: CUDA error in ") + what + " (" + file + ":" + std::to_string(line) +
-                     "): " + cudaGetErrorString(e));
+        const bool memory = e == cudaErrorMemoryAllocation;
+        throw Error(memory ? B2G_ERR_NO_MEMORY : B2G_ERR_CUDA,
+                    std::string("b2g: CUDA error in ") + what + " (" + file + ":" + std::to_string(line) + "): " +
+                        cudaGetErrorString(e),
+                    memory);
     }
 }
 #define B2G_CUDA(x) ::b2g::cudaCheck((x), #x, __FILE__, __LINE__)

@@ -751,6 +751,11 @@ Batch::Batch(std::vector<Matrix*> cs, cudaStream_t s) : stream(s), cases(std::mo
 {
     const int K = static_cast<int>(cases.size());
     if (K < 1) fail(B2G_ERR_ARGUMENT, "b2g batch: no cases");
+    {
+        std::set<Mesh*> once;
+        for (Matrix* A : cases) once.insert(A->mesh);
+        meshes.assign(once.begin(), once.end());
+    }
     int dev = 0;
     B2G_CUDA(cudaGetDevice(&dev));
     {
@@ -1299,7 +1304,7 @@ void Batch::preparePipe(int lv, int nSweeps)
         B2G_CUDA(cudaStreamSynchronize(A.stream));  // its values were filled there
         caseOf.push_back(c);
         small[c] = 1;
-        P.flows.push_back({c, S});
+        P.flows.push_back({c, S, S->held});
     }
     std::vector<int4> big;
     for (const int4& q : B.hostParts)
@@ -1381,8 +1386,24 @@ void Batch::ownWaits(k::FlowArgs<T>& a, const FlowSchedule& F) const
     a.publish = flowPublish;
 }
 
+std::vector<std::shared_lock<std::shared_mutex>> Batch::useMeshes()
+{
+    std::vector<std::shared_lock<std::shared_mutex>> use;
+    long long epochs = 0;
+    for (Mesh* M : meshes)
+    {
+        use.emplace_back(M->use);
+        epochs += M->flowEpoch;
+    }
+    if (epochs != flowEpochs)
+        for (BatchLevel& B : lev) B.pipe.clear();
+    flowEpochs = epochs;
+    return use;
+}
+
 void Batch::stall(long long limit)
 {
+    const auto use = useMeshes();
     spinLimit = limit > 0 ? limit : k::kSpinLimit;
     flowPublish = limit > 0 ? 0 : 1;
     auto patch = [&](BatchLevel::Pipe& P, auto T0) {
@@ -1646,6 +1667,7 @@ void Batch::solve(const b2g_controls& c, const double* const* source, double* co
     if (memspace != B2G_MEM_HOST && memspace != B2G_MEM_DEVICE) fail(B2G_ERR_ARGUMENT, "b2g batch: bad memspace");
     if (c.precision < B2G_PRECISION_FP64 || c.precision > B2G_PRECISION_FP32_PRECOND_MULTICOLOUR)
         fail(B2G_ERR_ARGUMENT, "b2g batch: unknown precision form");
+    const auto use = useMeshes();
     multicolour = c.precision == B2G_PRECISION_FP32_PRECOND_MULTICOLOUR;
     if (multicolour) prepareMulticolour();
     denseNow = false;

@@ -115,7 +115,13 @@ struct BatchLevel
         DBuf<unsigned char> table;   // k::FlowArgs<T>[nSmall]
         std::vector<unsigned char> hostTable;  // and on the host
         FlowBlocks flow[2];          // the launches: with more than one rank, and one CTA each
-        std::vector<std::pair<int, const FlowSchedule*>> flows;  // {case, its schedule}
+        struct Held
+        {
+            int first;                    // the case
+            const FlowSchedule* second;   // its schedule, which stays while held is copied
+            std::shared_ptr<char> held;
+        };
+        std::vector<Held> flows;
         DBuf<int> caseOf;            // [nSmall]
         DBuf<int4> partsBig;         // the parts of the cases that do not fit
         int nPartsBig = 0;
@@ -148,6 +154,11 @@ struct Batch
     unsigned long long layoutFingerprint() const;
     template <class T> void preparePipe(int lv, int nSweeps);
     void preparePipes(const b2g_controls& c);
+    // The cases' meshes, each once; a solve holds their schedules (Mesh::use), and forgets what it has tabulated of
+    // them when some were dropped meanwhile.
+    std::vector<Mesh*> meshes;
+    long long flowEpochs = -1;
+    std::vector<std::shared_lock<std::shared_mutex>> useMeshes();
     bool pipeOn = false;                    // the current solve takes the batched pipelined sweeps
     // The waits of the data-flow launches are the batch's own (ownWaits): they report to its error word, which
     // solve reads.

@@ -471,6 +471,7 @@ void solveOn(b2g::Matrix& A, const double* source, double* psi, const b2g_contro
                                    "pair (b2g_gamg_solve_coupled)");
     if (A.coupled && c->precision != B2G_PRECISION_FP64)
         b2g::fail(B2G_ERR_REFUSED, "b2g: a matrix with a coupled pair is solved in the FP64 form only");
+    const std::shared_lock<std::shared_mutex> use(A.mesh->use);
     const int n0 = A.n(0);
     // the solve runs in the finest level's position order: host fields are staged in fc/fr (free
     // outside a solve) and permuted on the device; device fields are permuted in place of a copy
@@ -781,6 +782,7 @@ b2g_status b2g_level_smooth(b2g_matrix* m, int level, int smoother, double* psi,
         need(m && psi && source, "b2g_level_smooth: null argument");
         need(level >= 0 && level <= m->mat->nLevels(), "b2g_level_smooth: level out of range");
         b2g::Matrix& A = *m->mat;
+        const std::shared_lock<std::shared_mutex> use(A.mesh->use);
         A.toPos(level, static_cast<const double*>(psi), A.ioBuf(0));
         A.toPos(level, source, A.ioBuf(1));
         A.smooth<double>(level, smoother, A.ioBuf(0), A.ioBuf(1), nSweeps);
@@ -914,6 +916,7 @@ b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const do
         need(stallLimit >= 0 && stallLimit <= b2g::k::kSpinLimit, "b2g_level_smooth_flow: stallLimit out of range");
         b2g::Matrix& A = *m->mat;
         need(!A.coupled, "b2g_level_smooth_flow: not for a coupled matrix");
+        const std::shared_lock<std::shared_mutex> use(A.mesh->use);
         A.toPos(level, static_cast<const double*>(psi), A.ioBuf(0));
         A.toPos(level, source, A.ioBuf(1));
         struct Waits
@@ -1020,6 +1023,7 @@ b2g_status b2g_level_pipe_shape(const b2g_mesh* mesh, int level, int nSweeps, in
         need(mesh != nullptr, "b2g_level_pipe_shape: null mesh");
         need(level >= 0 && level <= mesh->m.nLevels(), "b2g_level_pipe_shape: level out of range");
         need(valueBytes == 4 || valueBytes == 8, "b2g_level_pipe_shape: valueBytes is 4 or 8");
+        const std::shared_lock<std::shared_mutex> use(mesh->m.use);
         const auto& pipe = mesh->m.lev[level].pipe;
         const auto it = pipe.find(nSweeps * 16 + valueBytes);
         const bool have = it != pipe.end();
@@ -1087,6 +1091,7 @@ b2g_status b2g_level_mc_pipe(const b2g_mesh* mesh, int level, int nSweeps, int s
     return guarded([&] {
         need(mesh != nullptr, "b2g_level_mc_pipe: null mesh");
         need(level >= 0 && level <= mesh->m.nLevels(), "b2g_level_mc_pipe: no such level");
+        const std::shared_lock<std::shared_mutex> use(mesh->m.use);
         const b2g::Colouring& C = mesh->m.lev[level].mc;
         const auto it = C.pipe.find(nSweeps * 2 + (symmetric ? 1 : 0));
         const bool have = it != C.pipe.end();
@@ -1232,6 +1237,7 @@ b2g_status b2g_precondition(b2g_matrix* m, const b2g_controls* controls, double*
         need(m && controls && w && r, "b2g_precondition: null argument");
         b2g::Matrix& A = *m->mat;
         need(A.nLevels() > 0, "b2g_precondition: the mesh has no coarse levels");
+        const std::shared_lock<std::shared_mutex> use(A.mesh->use);
         A.resetLog(log ? std::max(log->coarsestCapacity, 0) : 0);
         A.serial = controls->reduction == B2G_REDUCTION_SERIAL;
         A.toPos(0, r, A.ioBuf(1));

@@ -27,29 +27,35 @@ namespace capi {
 
 extern thread_local std::string lastError;
 
-// Runs f, turning the library's exceptions into status codes and the thread's last-error string.
+// Runs f, turning the library's exceptions into status codes and the thread's last-error string. When the device
+// has no room, the smoothing schedules of idle meshes go (they only make a call faster) and f runs once more: an
+// entry writes its caller's data last, so it can.
 template <class F>
 b2g_status guarded(F&& f)
 {
-    try
+    for (bool again = true;; again = false)
     {
-        f();
-        return B2G_OK;
-    }
-    catch (const b2g::Error& e)
-    {
-        lastError = e.what();
-        return e.code;
-    }
-    catch (const std::bad_alloc&)
-    {
-        lastError = "b2g: host allocation failed";
-        return B2G_ERR_NO_MEMORY;
-    }
-    catch (const std::exception& e)
-    {
-        lastError = e.what();
-        return B2G_ERR_STATE;
+        try
+        {
+            f();
+            return B2G_OK;
+        }
+        catch (const b2g::Error& e)
+        {
+            if (e.deviceMemory && again && b2g::dropIdleFlows()) continue;
+            lastError = e.what();
+            return e.code;
+        }
+        catch (const std::bad_alloc&)
+        {
+            lastError = "b2g: host allocation failed";
+            return B2G_ERR_NO_MEMORY;
+        }
+        catch (const std::exception& e)
+        {
+            lastError = e.what();
+            return B2G_ERR_STATE;
+        }
     }
 }
 

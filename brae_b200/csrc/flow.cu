@@ -6,6 +6,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <mutex>
+#include <set>
 #include <vector>
 
 namespace b2g {
@@ -34,7 +36,171 @@ void allowFlowSmem()
     done.fetch_or(bit);
 }
 
+// every live mesh, and through it every live matrix
+std::mutex& g_meshesMu = *new std::mutex;  // (never destroyed: a mesh may go at the process's end)
+std::set<Mesh*>& g_meshes = *new std::set<Mesh*>;
+
+// What a mesh's schedules took is freed in each buffer's stream; the streams, to be waited for.
+struct Dropped
+{
+    size_t bytes = 0;
+    std::set<cudaStream_t> streams;
+    template <class B>
+    void take(B& b)
+    {
+        if (!b.p) return;
+        bytes += b.bytes();
+        streams.insert(b.s);
+        b.release();
+    }
+    void take(FlowSchedule& F)
+    {
+        take(F.chunkStart);
+        take(F.rec);
+        take(F.meta);
+        take(F.src);
+    }
+};
+
+// (g_meshesMu and M.use held)
+void dropLocked(Mesh& M, Dropped& D)
+{
+    const size_t had = D.bytes;
+    for (LevelAddr& L : M.lev)
+    {
+        for (auto it = L.pipe.begin(); it != L.pipe.end();)
+        {
+            if (it->second.flow) D.take(*it->second.flow);
+            // (chosen anew without it)
+            it = it->second.mode == 3 ? L.pipe.erase(it) : std::next(it);
+        }
+        for (auto& kv : L.flowBatch)
+            if (kv.second) D.take(*kv.second);
+        L.flowBatch.clear();
+        for (auto& kv : L.flowSym)
+            if (kv.second)
+            {
+                D.take(*kv.second);
+                kv.second.reset();
+            }
+        for (auto& kv : L.mc.pipe)
+            if (kv.second.flow)
+            {
+                D.take(*kv.second.flow);
+                kv.second.flow.reset();
+                kv.second.use = false;
+            }
+    }
+    for (Matrix* A : M.matrices)
+    {
+        auto drop = [&](auto& flows) {
+            for (auto& kv : flows)
+            {
+                D.take(kv.second.val);
+                D.take(kv.second.mail);
+                D.take(kv.second.ctl);
+            }
+            flows.clear();
+        };
+        drop(A->v64.flows);
+        drop(A->v32.flows);
+    }
+    if (D.bytes == had) return;
+    M.flowOff = true;
+    ++M.flowEpoch;
+}
+
+void giveBack(const Dropped& D)
+{
+    for (cudaStream_t s : D.streams) B2G_CUDA(cudaStreamSynchronize(s));
+    // (in one piece again for whatever is asked for next)
+    if (D.bytes) B2G_CUDA(cudaMemPoolTrimTo(libraryPool(), 0));
+}
+
 }  // namespace
+
+Mesh::Mesh()
+{
+    std::lock_guard<std::mutex> lk(g_meshesMu);
+    g_meshes.insert(this);
+}
+Mesh::~Mesh()
+{
+    std::lock_guard<std::mutex> lk(g_meshesMu);
+    g_meshes.erase(this);
+}
+void joinMesh(Matrix& A)
+{
+    std::lock_guard<std::mutex> lk(g_meshesMu);
+    A.mesh->matrices.insert(&A);
+}
+void leaveMesh(Matrix& A)
+{
+    std::lock_guard<std::mutex> lk(g_meshesMu);
+    // (a mesh destroyed before its matrix has left already)
+    if (g_meshes.count(A.mesh)) A.mesh->matrices.erase(&A);
+}
+
+bool dropIdleFlows()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    Dropped D;
+    return attempt([&] {
+               std::lock_guard<std::mutex> lk(g_meshesMu);
+               for (Mesh* M : g_meshes)
+               {
+                   if (M->device != dev || !M->use.try_lock()) continue;
+                   std::lock_guard<std::shared_mutex> own(M->use, std::adopt_lock);
+                   dropLocked(*M, D);
+               }
+               giveBack(D);
+           }) &&
+           D.bytes > 0;
+}
+
+size_t dropFlows(Mesh& M)
+{
+    std::lock_guard<std::mutex> lk(g_meshesMu);
+    if (!M.use.try_lock()) return 0;
+    std::lock_guard<std::shared_mutex> own(M.use, std::adopt_lock);
+    Dropped D;
+    dropLocked(M, D);
+    return D.bytes;
+}
+
+size_t flowBytes(const Mesh& M)
+{
+    std::lock_guard<std::mutex> lk(g_meshesMu);
+    size_t n = 0;
+    for (const LevelAddr& L : M.lev)
+    {
+        for (const auto& kv : L.pipe)
+            if (kv.second.flow) n += kv.second.flow->bytes();
+        for (const auto& kv : L.flowBatch)
+            if (kv.second) n += kv.second->bytes();
+        for (const auto& kv : L.flowSym)
+            if (kv.second) n += kv.second->bytes();
+        for (const auto& kv : L.mc.pipe)
+            if (kv.second.flow) n += kv.second.flow->bytes();
+    }
+    for (const Matrix* A : M.matrices)
+    {
+        for (const auto& kv : A->v64.flows) n += kv.second.val.bytes() + kv.second.mail.bytes();
+        for (const auto& kv : A->v32.flows) n += kv.second.val.bytes() + kv.second.mail.bytes();
+    }
+    return n;
+}
+
+bool flowRoom(size_t bytes)
+{
+    size_t freeB = 0, total = 0;
+    unsigned long long reserved = 0, used = 0;
+    B2G_CUDA(cudaMemGetInfo(&freeB, &total));
+    B2G_CUDA(cudaMemPoolGetAttribute(libraryPool(), cudaMemPoolAttrReservedMemCurrent, &reserved));
+    B2G_CUDA(cudaMemPoolGetAttribute(libraryPool(), cudaMemPoolAttrUsedMemCurrent, &used));
+    return freeB + (reserved - used) >= bytes + total / 8;
+}
 
 FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s)
 {
@@ -62,7 +228,8 @@ std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T,
                                         cudaStream_t s)
 {
     FlowProgram G;
-    if (!buildFlowProgram(H, T, S, nSteps, R, vb, G)) return nullptr;
+    if (!flowRoom(0) || !buildFlowProgram(H, T, S, nSteps, R, vb, G)) return nullptr;
+    if (!flowRoom(G.metaBytes + sizeof(k::FlowRec) * G.rec.size() + vb * G.nVal)) return nullptr;
     return uploadFlow(G, S, nSteps, R, s);
 }
 
@@ -167,7 +334,9 @@ bool Matrix::flowReady(int level, const FlowSchedule& F)
     const auto it = flows.find(F.id);
     if (it != flows.end() && it->second.gen == coefGen) return true;
     if (capturing && it != flows.end() && it->second.refused == coefGen) return false;
-    if (attempt([&] { flowValuesOf<T>(level, F); })) return true;
+    const bool have = it != flows.end() && it->second.val.p;  // (a refill, into the same buffer)
+    if ((capturing || have || flowRoom(sizeof(T) * static_cast<size_t>(F.nVal))) && attempt([&] { flowValuesOf<T>(level, F); }))
+        return true;
     if (capturing) fail(B2G_ERR_STATE, "b2g: a smoothing schedule's values were not filled before the capture");
     flows.erase(F.id);
     flows[F.id].refused = coefGen;
@@ -270,7 +439,7 @@ void Matrix::ensureSymFlow(int level, int nSweeps)
     const int key = nSweeps * 16 + static_cast<int>(sizeof(T));
     if (L.flowSym.count(key)) return;
     std::unique_ptr<FlowSchedule>& kept = L.flowSym[key];
-    if (nSweeps < 1 || L.nCells == 0) return;
+    if (nSweeps < 1 || L.nCells == 0 || mesh->flowOff) return;
     DBuf<T> x, b;
     if (!attempt([&] {
             x.alloc(nAlloc(level), stream);
@@ -350,7 +519,14 @@ void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStrea
     {
         auto known = jobs[i].level->flowBatch.find(keyOf(jobs[i]));
         if (known != jobs[i].level->flowBatch.end()) continue;
+        // the level's schedules of this call for other CTA counts that no batch holds any more make room
+        for (auto it = jobs[i].level->flowBatch.begin(); it != jobs[i].level->flowBatch.end();)
+        {
+            const bool old = it->first.first == keyOf(jobs[i]).first && it->second && it->second->held.use_count() == 1;
+            it = old ? jobs[i].level->flowBatch.erase(it) : std::next(it);
+        }
         jobs[i].level->flowBatch[keyOf(jobs[i])];  // (a level listed twice is built once)
+        if (!flowRoom(0)) continue;
         work.emplace_back();
         work.back().job = i;
         // (no memory for it, here and below: the level has no schedule)
@@ -367,7 +543,8 @@ void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStrea
     for (Work& w : work)
     {
         const FlowJob& j = jobs[w.job];
-        if (w.ok) attempt([&] { j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, nSweeps, w.nSteps, j.ranks, s); });
+        if (w.ok && flowRoom(w.G.metaBytes + sizeof(k::FlowRec) * w.G.rec.size() + vb * w.G.nVal))
+            attempt([&] { j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, nSweeps, w.nSteps, j.ranks, s); });
     }
     for (FlowJob& j : jobs) j.flow = j.level->flowBatch[keyOf(j)].get();
 }

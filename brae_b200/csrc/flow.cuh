@@ -94,6 +94,9 @@ inline long long flowSpinLimit(long long limit, const FlowSchedule& F)
 {
     return limit == k::kSpinLimit ? limit + kPollsPerStep * F.nSteps : limit;
 }
+// Whether the device has room for `bytes` more of schedules: an eighth of its memory stays free of them, for the
+// buffers that every form needs.
+bool flowRoom(size_t bytes);
 // whether a launch of that many ranks can be resident (one CTA per SM)
 bool flowFits(int ranks);
 

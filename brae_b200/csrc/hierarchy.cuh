@@ -8,8 +8,12 @@
 
 #include <map>
 #include <memory>
+#include <set>
+#include <shared_mutex>
 
 namespace b2g {
+
+struct Matrix;
 
 // The sweep order of one level and its Gauss-Seidel schedule (gs_kernels.cuh). Cells are split into
 // `nParts` contiguous index ranges; each part lists its cells by (depth, cell), depth being the cell's
@@ -100,6 +104,8 @@ struct PipeSchedule
 struct FlowSchedule
 {
     long long id = 0;             // names the schedule in the matrices' value buffers
+    std::shared_ptr<char> held = std::make_shared<char>();  // copies of it: batches whose launches read the schedule
+    size_t bytes() const { return chunkStart.bytes() + rec.bytes() + meta.bytes() + src.bytes(); }
     int sweeps = 0;
     int ranks = 0;
     int nSteps = 0;
@@ -266,7 +272,26 @@ struct Mesh
     float buildMs = 0.f;
     bool hasPair = false;        // b2g_mesh_set_pair was called (every level's PairLevel is built)
     int nLevels() const { return static_cast<int>(step.size()); }
+    // The smoothing schedules of the levels (FlowSchedule) and the matrices' values of them only make calls
+    // faster, so they are dropped when the device runs out of memory (flow.cu dropIdleFlows). A call that uses
+    // them holds `use` shared; who drops them holds it exclusively. What is captured or tabulated with their
+    // addresses is remade when flowEpoch has moved on.
+    mutable std::shared_mutex use;
+    std::set<Matrix*> matrices;  // the mesh's live matrices (under the registry's lock)
+    long long flowEpoch = 0;
+    bool flowOff = false;        // dropped once: the mesh keeps the other forms
+    Mesh();
+    ~Mesh();
 };
+
+// Drops the smoothing schedules of every mesh of the current device that no call is using, so that their memory
+// can be had; false when there were none.
+bool dropIdleFlows();
+// The same of one mesh, without waiting for its streams (the memory is reused in their order). The bytes it had;
+// 0 while a call is using it.
+size_t dropFlows(Mesh& M);
+// A mesh's schedules and its matrices' values of them, in bytes.
+size_t flowBytes(const Mesh& M);
 
 // Builds the derived layouts of `L` from its lower/upper (already on the device). Validates the
 // upper-triangular order (faces sorted by owner, owner < neighbour).

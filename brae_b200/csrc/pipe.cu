@@ -456,8 +456,9 @@ void Matrix::ensurePipe(int level, int nSweeps)
     float best = C.msSweeps;
     {
         // the data-flow launch on a few CTA counts
-        FlowLevel H = flowDownload(L, stream);
-        for (const FlowShape& f : flowShapes(L.nCells))
+        FlowLevel H;
+        if (!mesh->flowOff) H = flowDownload(L, stream);
+        for (const FlowShape& f : mesh->flowOff ? std::vector<FlowShape>{} : flowShapes(L.nCells))
         {
             std::unique_ptr<FlowSchedule> F;
             float ms = 0.f;
@@ -599,7 +600,7 @@ void Matrix::ensureMcPipe(int level, int nSweeps, bool symmetric)
         return;
     }
     Colouring::Pipe& M = C.pipe[key];
-    if (nSweeps < 1 || L.nCells == 0 || C.nColours == 0 || !C.tuned || L.nCells > kMcFlowCells) return;
+    if (nSweeps < 1 || L.nCells == 0 || C.nColours == 0 || !C.tuned || L.nCells > kMcFlowCells || mesh->flowOff) return;
     float* x = level == 0 ? w32.p : v32.corr[level - 1].p;
     float* b = level == 0 ? r32.p : v32.src[level - 1].p;
     // scratch vectors of the level (the times do not depend on the values)

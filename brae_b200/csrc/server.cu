@@ -49,7 +49,8 @@ struct b2g_server
     {
         std::unique_ptr<b2g_mesh> mesh;
         std::unique_ptr<b2g::Matrix> mat;
-        size_t bytes = 0;
+        size_t bytes = 0;      // admitted with
+        size_t flowBytes = 0;  // its smoothing schedules, as its last solve left them
         int nCells = 0;
         bool busy = false;
         bool alive = true;
@@ -201,6 +202,26 @@ void runGroup(std::vector<b2g_server::Request>& group, b2g::Batch& batch, const 
     }
 }
 
+// The cases' smoothing schedules, which their solves make, take what the admitted footprints leave under the cap:
+// beyond it those of idle cases go, least recently used first, and these cases solve without. (The server's lock held)
+void fitSchedules(b2g_server& S)
+{
+    for (;;)
+    {
+        size_t total = S.resident;
+        b2g_server::Case* victim = nullptr;
+        for (const auto& c : S.cases)
+        {
+            if (!c->alive) continue;
+            total += c->flowBytes;
+            if (!c->busy && c->flowBytes && (!victim || c->lastUse < victim->lastUse)) victim = c.get();
+        }
+        if (total <= S.capBytes || !victim) return;
+        b2g::dropFlows(victim->mesh->m);
+        victim->flowBytes = 0;
+    }
+}
+
 void workerLoop(b2g_server* S, int slot)
 {
     cudaSetDevice(S->device);
@@ -321,13 +342,18 @@ void workerLoop(b2g_server* S, int slot)
                 cache.push_back(std::move(cb));
             }
         }
+        std::vector<size_t> flows(group.size());
+        for (size_t i = 0; i < group.size(); ++i) flows[i] = b2g::flowBytes(S->cases[group[i].caseId]->mesh->m);
         {
             std::lock_guard<std::mutex> lk(S->mu);
             for (size_t i = 0; i < group.size(); ++i)
             {
+                b2g_server::Case& c = *S->cases[group[i].caseId];
                 S->results[group[i].ticket] = std::move(res[i]);
-                S->cases[group[i].caseId]->busy = false;
+                c.busy = false;
+                c.flowBytes = flows[i];
             }
+            fitSchedules(*S);
         }
         S->cvDone.notify_all();
         S->cvWork.notify_all();  // requests queued behind these cases may run now
@@ -367,6 +393,7 @@ void evictFor(b2g_server& S, size_t need)
         victim->alive = false;
         S.resident -= victim->bytes;
         victim->bytes = 0;
+        victim->flowBytes = 0;
     }
 }
 
@@ -464,6 +491,7 @@ B2G_API b2g_status b2g_server_add_case(b2g_server* S, int nCells, int nFaces, co
             b2g::fail(B2G_ERR_NO_MEMORY, "b2g_server_add_case: the case does not fit under the HBM cap beside "
                                          "the cases in use");
         S->resident += c->bytes;
+        fitSchedules(*S);
         c->lastUse = ++S->useClock;
         S->cases.push_back(std::move(c));
         *caseId = static_cast<int>(S->cases.size()) - 1;

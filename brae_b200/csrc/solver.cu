@@ -688,6 +688,7 @@ void Matrix::timingsEnd()
 
 Matrix::~Matrix()
 {
+    leaveMesh(*this);
     for (IterationGraph* g : {&pcgGraph, &gamgGraph}) releaseGraph(*g);
     for (const TimedRegion& r : evOpen) evFree.emplace_back(r.start, r.end);
     for (auto& e : evFree)
@@ -731,6 +732,7 @@ Matrix::Matrix(Mesh* m, cudaStream_t s) : mesh(m), stream(s)
     allowSweepSmem<double>(dev);
     allowSweepSmem<float>(dev);
     upCtas = std::min(upClusterCtas<double>(dev), upClusterCtas<float>(dev));
+    joinMesh(*this);
 }
 
 void Matrix::setFine(const double* diag, const double* upper, int memspace)
@@ -1905,7 +1907,8 @@ unsigned long long Matrix::layoutFingerprint() const
         mix(kv.second.mail.p);
     }
     for (const void* q : {(const void*)denseL.p}) mix(q);
-    return h;
+    h ^= static_cast<unsigned long long>(mesh->flowEpoch);  // (a schedule dropped and made anew may be elsewhere)
+    return h * 1099511628211ull;
 }
 
 template <class F>

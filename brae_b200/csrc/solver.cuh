@@ -122,6 +122,10 @@ k::Rows<T> rowsOf(const LevelAddr& L, const LevelCoef<T>& C)
     return r;
 }
 
+// The registry of live matrices by mesh (flow.cu), for dropFlows.
+void joinMesh(Matrix& A);
+void leaveMesh(Matrix& A);
+
 // Whether smoothing calls may take the pipelined multi-sweep launch (pipe.cu; b2g_set_sweep_pipeline).
 extern bool g_pipeline;
 

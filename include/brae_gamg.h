@@ -516,7 +516,9 @@ B2G_API b2g_status b2g_server_create(unsigned long long hbmCapBytes, int nSlots,
 B2G_API b2g_status b2g_server_destroy(b2g_server* server);
 /* Registers a case: builds its hierarchy and its matrix (FP64 and FP32 levels) and keeps both
  * resident, admitted by their HBM footprint: idle cases without queued requests are evicted, least
- * recently used first, until the case fits under the cap; else B2G_ERR_NO_MEMORY. Arguments as
+ * recently used first, until the case fits under the cap; else B2G_ERR_NO_MEMORY. The smoothing schedules that
+ * a case's solves make take what the footprints leave under the cap: beyond it those of idle cases are dropped,
+ * least recently used first, and these cases solve without them, to the same result. Arguments as
  * b2g_mesh_create and b2g_matrix_create (folded diagonal, upper == lower coefficients). */
 B2G_API b2g_status b2g_server_add_case(b2g_server* server, int nCells, int nFaces, const int32_t* lower,
                                        const int32_t* upper, const double* Sf, const double* magSf,

@@ -252,3 +252,71 @@ def test_long_chain_of_steps(b2g):
     A.smooth_flow(0, x, b, 1, torch.cuda.get_device_properties(0).multi_processor_count, 4)
     A.smooth(0, want, b, 1)  # one sweep: no data flow
     assert torch.equal(x, want)
+
+
+_SCHEDULES_GO = """
+import sys
+sys.path.insert(0, {repo!r})
+import numpy as np
+import torch
+import brae_b200.native as b
+from brae_b200 import cases
+
+c = cases.box_case(180, 110, 100, (2.0, 1.0, 1.0), 5.0)
+new_mesh = lambda: b.Mesh(c.lower, c.upper, c.Sf, c.magSf, c.n_cells, 10, True)
+ctl = b.controls_default(tolerance=1e-12, relTol=0.0, maxIter=2)
+
+
+def solve(A):
+    psi = np.zeros(c.n_cells)
+    A.solve(c.source, psi, ctl)
+    return psi
+
+
+mesh = new_mesh()
+A = b.Matrix(mesh, c.diag, c.coef)
+batch_mesh = new_mesh()
+batch = b.Batch([b.Matrix(batch_mesh, c.diag, c.coef)])
+
+
+def solve_batch():
+    psi = np.zeros(c.n_cells)
+    batch.solve([c.source], [psi], ctl)
+    return psi
+
+
+want, want_batch = solve(A), solve_batch()
+before = mesh.pipe_shape(0, 2, 8)
+assert before["ranks"] > 0 and not before["grid"], before
+# leave a few GB (and the room rule's eighth is gone): the next matrices, without pipelined launches, take it all
+free, _ = torch.cuda.mem_get_info()
+hold = torch.empty(free - (2 << 30), dtype=torch.uint8, device="cuda")
+more = new_mesh()
+b.set_sweep_pipeline(False)
+kept = []
+try:
+    for k in range(200):
+        kept.append(b.Matrix(more, c.diag, c.coef))
+        solve(kept[-1])
+except b.GamgError as e:
+    assert e.status == "NO_MEMORY", e
+else:
+    raise AssertionError("the device was never full")
+b.set_sweep_pipeline(True)
+after = mesh.pipe_shape(0, 2, 8)
+assert after["ms_sweep_by_sweep"] == 0.0, after   # the mesh's schedules went before the call failed
+assert np.array_equal(solve(A), want)
+assert np.array_equal(solve_batch(), want_batch)
+print("SAME", len(kept))
+"""
+
+
+def test_schedules_go_when_memory_is_short():
+    # matrices are made until none fits: the schedules of idle meshes are dropped before a call fails, and what
+    # had been captured or tabulated with them (a solve's graph, a batch's tables) is remade without, bit for bit
+    import os
+    import subprocess
+    import sys
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _SCHEDULES_GO.format(repo=repo)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "SAME" in r.stdout, (r.stdout[-500:], r.stderr[-1500:])

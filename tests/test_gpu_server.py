@@ -135,3 +135,31 @@ def test_wait_timeout_keeps_the_request(b2g):
             srv.wait(t)  # collected already
     finally:
         srv.close()
+
+
+def test_schedules_stay_under_the_cap(b2g):
+    # a cap with room for the cases but hardly for their smoothing schedules: those of idle cases go, and the
+    # cases solve to the same result as where there is room
+    built = [cases.box_case(nx=30 + 2 * s, ny=28, nz=26, lengths=(2.0, 1.0, 1.0), grading_y=20.0, seed=s) for s in range(3)]
+    ctl = b2g.controls_default(tolerance=1e-8, relTol=0.0)
+    want, need = [], 0
+    roomy = b2g.Server(64 << 30, slots=2)
+    try:
+        ids = [_add(roomy, c) for c in built]
+        need = sum(roomy.case_bytes(i) for i in ids)
+        want = [roomy.wait(roomy.submit(i, c.source, ctl))[:2] for i, c in zip(ids, built)]
+    finally:
+        roomy.close()
+    tight = b2g.Server(need + (1 << 20), slots=2)
+    try:
+        ids = [_add(tight, c) for c in built]
+        for _ in range(3):
+            for i, c, (psi, perf) in zip(ids, built, want):
+                got = tight.wait(tight.submit(i, c.source, ctl))
+                assert tuple(got[1]) == tuple(perf) and np.array_equal(got[0], psi)
+            together = [tight.submit(i, c.source, ctl) for i, c in zip(ids, built)]
+            for t, (psi, perf) in zip(together, want):
+                got = tight.wait(t)
+                assert tuple(got[1]) == tuple(perf) and np.array_equal(got[0], psi)
+    finally:
+        tight.close()
