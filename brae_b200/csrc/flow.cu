@@ -58,7 +58,6 @@ struct Dropped
         take(F.chunkStart);
         take(F.rec);
         take(F.meta);
-        take(F.src);
     }
 };
 
@@ -209,7 +208,6 @@ FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s)
     H.nF = L.nFaces;
     H.lower = L.lower.download(s);
     H.upper = L.upper.download(s);
-    H.depth = L.gs.depth.download(s);
     H.posCell = L.gs.posCell.download(s);
     H.posRow = L.gs.posRow.download(s);
     H.entColPos = L.gs.entColPos.download(s);
@@ -222,7 +220,7 @@ FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s)
     return H;
 }
 
-static std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int S, int nSteps, int R, cudaStream_t s);
+static std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int nSteps, int R, cudaStream_t s);
 
 std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb,
                                         cudaStream_t s)
@@ -230,30 +228,26 @@ std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T,
     FlowProgram G;
     if (!flowRoom(0) || !buildFlowProgram(H, T, S, nSteps, R, vb, G)) return nullptr;
     if (!flowRoom(G.metaBytes + sizeof(k::FlowRec) * G.rec.size() + vb * G.nVal)) return nullptr;
-    return uploadFlow(G, S, nSteps, R, s);
+    return uploadFlow(G, nSteps, R, s);
 }
 
-std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int S, int nSteps, int R, cudaStream_t s)
+std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int nSteps, int R, cudaStream_t s)
 {
     auto F = std::make_unique<FlowSchedule>();
     static std::atomic<long long> nextId{1};
     F->id = nextId++;
-    F->sweeps = S;
     F->ranks = R;
     F->nSteps = nSteps;
     F->slots = G.slots;
     F->nVal = static_cast<long long>(G.nVal);
+    F->nChunks = static_cast<int>(G.rec.size());
     F->meta.alloc(std::max<size_t>(G.metaBytes, 16), s);
-    F->src.alloc(std::max<size_t>(G.nVal, 1), s);
-    size_t metaAt = 0, valAt = 0;
+    size_t metaAt = 0;
     for (const RankProgram& P : G.prog)
     {
         if (!P.meta.empty())
             B2G_CUDA(cudaMemcpyAsync(F->meta.p + metaAt, P.meta.data(), P.meta.size(), cudaMemcpyHostToDevice, s));
-        if (!P.src.empty())
-            B2G_CUDA(cudaMemcpyAsync(F->src.p + valAt, P.src.data(), sizeof(int) * P.src.size(), cudaMemcpyHostToDevice, s));
         metaAt += P.meta.size();
-        valAt += P.src.size();
     }
     F->chunkStart.upload(G.chunkStart.data(), G.chunkStart.size(), s);
     F->rec.upload(reinterpret_cast<const int4*>(G.rec.data()), 3 * G.rec.size(), s);
@@ -308,9 +302,10 @@ const T* Matrix::flowValuesOf(int level, const FlowSchedule& F)
     {
         if (capturing) fail(B2G_ERR_STATE, "b2g: a smoothing schedule's values were not filled before the capture");
         B.val.ensure(static_cast<size_t>(std::max<long long>(F.nVal, 1)), stream);
-        if (F.nVal)
-            k::flowValues<T><<<std::min(ceilDiv(F.nVal, 256), 8192), 256, 0, stream>>>(
-                F.nVal, F.src.p, D.coef[level].rowVal.p, D.coef[level].gsDiag.p, B.val.p);
+        if (F.nChunks)
+            k::flowValues<T><<<std::min(F.nChunks, 8192), 32 * k::kFlowTeam, 0, stream>>>(
+                F.nChunks, F.rec.p, F.meta.p, mesh->lev[level].gs.posRow.p, D.coef[level].rowVal.p,
+                D.coef[level].gsDiag.p, B.val.p);
         B2G_LAUNCH_CHECK();
         if (F.ranks > 1 && !B.mail.p)
         {
@@ -544,7 +539,7 @@ void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStrea
     {
         const FlowJob& j = jobs[w.job];
         if (w.ok && flowRoom(w.G.metaBytes + sizeof(k::FlowRec) * w.G.rec.size() + vb * w.G.nVal))
-            attempt([&] { j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, nSweeps, w.nSteps, j.ranks, s); });
+            attempt([&] { j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, w.nSteps, j.ranks, s); });
     }
     for (FlowJob& j : jobs) j.flow = j.level->flowBatch[keyOf(j)].get();
 }

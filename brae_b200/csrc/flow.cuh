@@ -14,7 +14,7 @@ namespace b2g {
 struct FlowLevel
 {
     int n = 0, nF = 0;
-    std::vector<int> lower, upper, depth, posCell, posRow, entColPos, cellPos;
+    std::vector<int> lower, upper, posCell, posRow, entColPos, cellPos;
     bool crosses = false;  // more than one rank
 };
 
@@ -24,12 +24,12 @@ inline int flowRank(int c, int n, int R) { return static_cast<int>(static_cast<l
 
 constexpr size_t kFlowSmem = 220 * 1024;  // dynamic shared memory of a CTA: value slots and ring
 
-// One rank's program .
+// One rank's program.
 struct RankProgram
 {
     std::vector<k::FlowRec> rec;
     std::vector<unsigned char> meta;
-    std::vector<int> src;     // per value (flowValues)
+    size_t nVal = 0;          // its values (flowValues)
     int slots = 1;            // value slots used (slot 0 is the zero)
     bool ok = true;
 };

@@ -619,21 +619,37 @@ __global__ void __launch_bounds__(flowThreads(kRemote), 1) gsFlowBatch(const Flo
     flowBody<T, false, kRemote>(a, w.y);
 }
 
-// the values of a schedule's chunks, from the level's rows by position: src >= 0 a row entry, -1 zero,
-// else of the diagonal of position -(src + 2) / 2: itself (even) or its reciprocal (odd; flowRcp)
+// The values of a schedule's chunks, from the level's rows by position: a warp per slice, a lane per item. Where
+// each comes from is in the chunk's own meta blob (its items' positions), so no index a value is kept.
 template <class T>
-__global__ void flowValues(long long n, const int* __restrict__ src, const T* __restrict__ rowVal, const T* __restrict__ diag,
+__global__ void flowValues(int nChunks, const int4* __restrict__ rec, const unsigned char* __restrict__ meta,
+                           const int* __restrict__ posRow, const T* __restrict__ rowVal, const T* __restrict__ diag,
                            T* __restrict__ out)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    constexpr int kPer = 16 / sizeof(T);  // coefficients a lane reads with one load
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = blockDim.x >> 5;
+    for (int j = blockIdx.x; j < nChunks; j += gridDim.x)
     {
-        const int e = src[i];
-        if (e >= -1)
-            out[i] = e >= 0 ? rowVal[e] : T(0);
-        else
+        const int4 r0 = rec[3 * static_cast<size_t>(j)], r1 = rec[3 * static_cast<size_t>(j) + 1];
+        const unsigned char* M = meta + 16 * static_cast<size_t>(r0.x);
+        // (offsets within a chunk run on from its meta blob to its values)
+        T* V = out + kPer * static_cast<size_t>(r1.x);
+        for (int s = warp; s < r1.w; s += nWarps)
         {
-            const T d = diag[-(e + 2) >> 1];
-            out[i] = (-(e + 2) & 1) ? flowRcp(d) : d;
+            const FlowSlice h = reinterpret_cast<const FlowSlice*>(M)[s];
+            const bool has = lane < h.count;
+            const int p = has ? reinterpret_cast<const int2*>(M + 8 * static_cast<size_t>(h.items8))[lane].x : 0;
+            const T d = has ? diag[p] : T(0);
+            T* dv = V + (8 * static_cast<size_t>(h.diag8) - r0.y) / sizeof(T) + 2 * lane;
+            dv[0] = d;
+            dv[1] = has ? flowRcp(d) : T(0);
+            if (lane >= h.stride) continue;
+            const int e0 = has ? posRow[p] : 0, w = has ? posRow[p + 1] - e0 : 0;
+            T* ev = V + (8 * static_cast<size_t>(h.vals8) - r0.y) / sizeof(T) + kPer * lane;
+            for (int q = 0; q < h.width; q += kPer)
+#pragma unroll
+                for (int i = 0; i < kPer; ++i)
+                    ev[static_cast<size_t>(h.stride) * q + i] = q + i < w ? rowVal[e0 + q + i] : T(0);
         }
     }
 }

@@ -170,10 +170,9 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
     {
         unsigned a, b;
     };
-    // (about what the items take: records, sources and rows padded by a quarter)
+    // (about what the items take: records, and rows padded by a quarter)
     size_t rowEntries = 0;
     for (const ItemRef& it : items) rowEntries += static_cast<size_t>((it.w() + 3) & ~3);
-    P.src.reserve(2 * items.size() + rowEntries * 5 / 4 + 128 * static_cast<size_t>(nCh));
     P.meta.reserve(16 * items.size() + rowEntries * 5 / 2 + 1024 * static_cast<size_t>(nCh));
     std::vector<Pair> fetch, halo;
     std::vector<unsigned short> codes;
@@ -207,22 +206,13 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         fetch.clear();
         halo.clear();
         codes.assign(nEnt, 0);
-        const size_t srcAt = P.src.size();
-        P.src.resize(srcAt + 64 * static_cast<size_t>(nSl) + nEnt, -1);
-        int* diagSrc = P.src.data() + srcAt;
-        int* entSrc = diagSrc + 64 * nSl;
-        for (int i = 0; i < m; ++i)
-        {
-            diagSrc[2 * i] = -(2 * items[a + i].p() + 2);
-            diagSrc[2 * i + 1] = -(2 * items[a + i].p() + 3);
-        }
         // (a chunk's values are read before its items write: every read first, then the writes)
         for (int i = 0; i < m; ++i)
         {
             const int p = items[a + i].p(), visitOf = items[a + i].q();
             const int c = H.posCell[p];
             const int st = k::flowStride(m, i / 32);
-            const int at0 = first[i / 32], l = i % 32, vg = vb == 8 ? 2 : 4;
+            const int at0 = first[i / 32], l = i % 32;
             for (int e = H.posRow[p], q = 0; e < H.posRow[p + 1]; ++e, ++q)
             {
                 const int pn = H.entColPos[e];
@@ -247,7 +237,6 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
                     visit[v] = ver;
                 }
                 codes[at0 + 4 * (st * (q / 4) + l) + q % 4] = static_cast<unsigned short>(slot[v]);
-                entSrc[at0 + vg * (st * (q / vg) + l) + q % vg] = e;
             }
         }
         for (int i = 0; i < m; ++i) give(H.posCell[items[a + i].p()] - c0);
@@ -304,6 +293,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         r.counts = static_cast<int>(static_cast<unsigned>(fetch.size()) | static_cast<unsigned>(halo.size()) << 16);
         valAt += nVal;
     }
+    P.nVal = static_cast<size_t>(valAt);
     for (int g : ghostCell) X.localOf[g] = -1;
 }
 
@@ -492,7 +482,7 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
         if (!P.ok) return false;
         F.slots = std::max(F.slots, P.slots);
         F.metaBytes += P.meta.size();
-        F.nVal += P.src.size();
+        F.nVal += P.nVal;
     }
     // the ring holds three chunks at least: one computed, one loaded by the other team, one on its way
     const size_t ringAt = k::flowRingAt(F.slots, vb);
@@ -517,7 +507,7 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
         }
         F.chunkStart[r + 1] = static_cast<int>(F.rec.size());
         metaAt += P.meta.size();
-        valAt += P.src.size();
+        valAt += P.nVal;
     }
     return true;
 }

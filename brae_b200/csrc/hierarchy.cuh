@@ -99,22 +99,20 @@ struct PipeSchedule
 };
 
 // One smoothing call's sweeps of a level as a data flow between `ranks` CTAs (flow_kernels.cuh), for
-// values of one size: every rank's chunks with their place in the shared-memory ring, and where each
-// chunk's values come from. A matrix keeps the values themselves (VCycleData::flows).
+// values of one size: every rank's chunks with their place in the shared-memory ring. A matrix keeps the values themselves (VCycleData::flows).
 struct FlowSchedule
 {
     long long id = 0;             // names the schedule in the matrices' value buffers
     std::shared_ptr<char> held = std::make_shared<char>();  // copies of it: batches whose launches read the schedule
-    size_t bytes() const { return chunkStart.bytes() + rec.bytes() + meta.bytes() + src.bytes(); }
-    int sweeps = 0;
+    size_t bytes() const { return chunkStart.bytes() + rec.bytes() + meta.bytes(); }
     int ranks = 0;
     int nSteps = 0;
     int slots = 0;                // value slots of a CTA
-    long long nVal = 0;
+    int nChunks = 0;
+    long long nVal = 0;           // values (k::flowValues fills them)
     DBuf<int> chunkStart;         // [ranks + 1]
     DBuf<int4> rec;               // [chunks][3] k::FlowRec
     DBuf<unsigned char> meta;     // the chunks' meta blobs
-    DBuf<int> src;                // [nVal] row entry or diagonal of each value (k::flowValues)
 };
 
 // The dynamic shared memory of a pipelined launch in values of valueBytes (pipe.cu): the rank's
