@@ -11,6 +11,7 @@
 #include "capi_internal.cuh"
 
 #include <algorithm>
+#include <set>
 #include <cstddef>
 #include <cstring>
 #include <mutex>
@@ -21,7 +22,10 @@ namespace {
 
 constexpr int BT = 256;       // threads per tile block
 constexpr int kTile = 2048;   // cells per tile
-constexpr int kFlowBatchCells = 300000;   // the largest level whose batched sweeps are data-flow launches
+// The most cells of all the cases' levels together for data-flow launches. Measured (40 mixed cases, FP32, ms a
+// smoothing call, data flow against the sweep-by-sweep launch): 0.53 M cells 0.64 and 2.16, 1.07 M 0.84 and 2.00, 2.14 M
+// 1.02 and 2.07, 4.28 M 1.52 and 1.71, 8.56 M 2.42 and 1.53. Many cases fill the SMs by themselves.
+constexpr long long kFlowBatchCells = 3000000;
 constexpr int kFlowBatchShare = 1600;     // its cells per CTA, while the CTAs fit the SMs
 constexpr int kWarpsPerBlock = BT / 32;
 
@@ -1221,11 +1225,47 @@ void Batch::smooth(int lv, int nSweeps)
     }
 }
 
-// The batched sweeps of level lv for nSweeps sweeps in T as data-flow launches (flow_kernels.cuh): each case's
+// The batched sweeps of level lv for nSweeps sweeps as data-flow launches (flow_kernels.cuh): each case's
 // level on a share of the SMs by its size, a power of two of CTAs (so a mesh keeps few schedules). All in one
 // cooperative launch while the CTAs fit the SMs; the cases with one CTA, which wait for nobody, in a launch of
-// their own when not. Levels above kFlowBatchCells keep the sweep-by-sweep launch: they would hold the GPU's
-// SMs anyway, and their schedules would weigh on every resident case's memory. Outside any capture.
+// their own when not. None when the cases' levels together have more than kFlowBatchCells cells. The level's
+// jobs, case by case.
+void Batch::flowJobs(int lv, int nSweeps, size_t vb, std::vector<FlowJob>& jobs, std::vector<int>& jobCase) const
+{
+    const int K = static_cast<int>(cases.size());
+    std::vector<int> ranks(K, 0);
+    const int sms = DeviceInfo::get().numSMs;
+    long long cells = 0;
+    for (int c = 0; c < K; ++c)
+        if (nLevelsOf[c] >= lv + 1) cells += cases[c]->mesh->lev[lv].nCells;
+    if (cells > kFlowBatchCells) return;
+    // a CTA per kFlowBatchShare cells, fewer for all when that is more than the SMs
+    double share = kFlowBatchShare;
+    for (bool fits = false; !fits; share *= 1.1)
+    {
+        int remote = 0, single = 0;
+        for (int c = 0; c < K; ++c)
+        {
+            if (nLevelsOf[c] < lv + 1) continue;
+            const int n = cases[c]->mesh->lev[lv].nCells;
+            if (n == 0) continue;
+            int r = 1;
+            while (2 * r * share <= n && 2 * r <= sms) r *= 2;
+            ranks[c] = r;
+            if (r > 1) remote += r;
+            else ++single;
+        }
+        fits = remote == 0 || remote + std::min(single, sms / 2) <= sms;
+    }
+    for (int c = 0; c < K; ++c)
+    {
+        if (ranks[c] == 0 || cases[c]->mesh->flowOff) continue;
+        jobs.push_back({&cases[c]->mesh->lev[lv], nSweeps, ranks[c], vb, nullptr});
+        jobCase.push_back(c);
+    }
+}
+
+// Their tables and the choice, by measurement, between them and the sweep-by-sweep launches. Outside any capture.
 template <class T>
 void Batch::preparePipe(int lv, int nSweeps)
 {
@@ -1249,37 +1289,16 @@ void Batch::preparePipe(int lv, int nSweeps)
     std::vector<k::FlowArgs<T>> table;
     std::vector<int> caseOf;
     std::vector<char> small(K, 0);
-    std::vector<int> ranks(K, 0);
     const int sms = DeviceInfo::get().numSMs;
-    {
-        // a CTA per kFlowBatchShare cells, fewer for all when that is more than the SMs
-        double share = kFlowBatchShare;
-        for (bool fits = false; !fits; share *= 1.1)
-        {
-            int remote = 0, single = 0;
-            for (int c = 0; c < K; ++c)
-            {
-                if (nLevelsOf[c] < lv + 1) continue;
-                const int n = cases[c]->mesh->lev[lv].nCells;
-                if (n == 0 || n > kFlowBatchCells) continue;
-                int r = 1;
-                while (2 * r * share <= n && 2 * r <= sms) r *= 2;
-                ranks[c] = r;
-                if (r > 1) remote += r;
-                else ++single;
-            }
-            fits = remote == 0 || remote + std::min(single, sms / 2) <= sms;
-        }
-    }
     std::vector<FlowJob> jobs;
     std::vector<int> jobCase;
-    for (int c = 0; c < K; ++c)
-    {
-        if (ranks[c] == 0) continue;
-        jobs.push_back({&cases[c]->mesh->lev[lv], ranks[c], nullptr});
-        jobCase.push_back(c);
-    }
-    flowsForBatch(jobs, nSweeps, sizeof(T), stream);
+    flowJobs(lv, nSweeps, sizeof(T), jobs, jobCase);
+    flowsForBatch(jobs, stream);  // (made by preparePipes, for all levels at once)
+    std::set<cudaStream_t> filled;
+    size_t need = 0;
+    for (const FlowJob& j : jobs)
+        if (j.flow) need += sizeof(T) * static_cast<size_t>(j.flow->nVal);
+    const bool room = flowRoom(need);
     for (size_t i = 0; i < jobs.size(); ++i)
     {
         const int c = jobCase[i];
@@ -1298,14 +1317,15 @@ void Batch::preparePipe(int lv, int nSweeps)
             b = reinterpret_cast<const T*>(lv == 0 ? A.r32.p : A.v32.src[lv - 1].p);
             psi = reinterpret_cast<T*>(lv == 0 ? A.w32.p : A.v32.corr[lv - 1].p);
         }
-        if (!A.flowReady<T>(lv, *S)) continue;
+        if (!A.flowReady<T>(lv, *S, room)) continue;
         table.push_back(A.flowArgs<T>(lv, *S, psi, b));
         ownWaits(table.back(), *S);
-        B2G_CUDA(cudaStreamSynchronize(A.stream));  // its values were filled there
+        filled.insert(A.stream);  // its values were filled there
         caseOf.push_back(c);
         small[c] = 1;
         P.flows.push_back({c, S, S->held});
     }
+    for (cudaStream_t s : filled) B2G_CUDA(cudaStreamSynchronize(s));
     std::vector<int4> big;
     for (const int4& q : B.hostParts)
         if (!small[q.z]) big.push_back(q);
@@ -1363,6 +1383,18 @@ void Batch::preparePipe(int lv, int nSweeps)
     const bool gaveUp = !attempt([&] { P.msPipe = timeIt(true); }) || takeError();
     P.msSweeps = timeIt(false);
     P.use = !gaveUp && P.msPipe < P.msSweeps;
+    if (!P.use)
+    {
+        // not kept: their memory goes, schedules and values
+        for (const BatchLevel::Pipe::Held& f : P.flows)
+        {
+            cases[f.first]->data<T>().flows.erase(f.second->id);
+            for (auto& kv : cases[f.first]->mesh->lev[lv].flowBatch)
+                if (kv.second.get() == f.second) kv.second.reset();
+        }
+        P.flows.clear();
+        P.nSmall = 0;
+    }
     launches = l0;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1427,10 +1459,9 @@ void Batch::preparePipes(const b2g_controls& c)
     pipeOn = g_pipeline && !multicolour && c.smoother == B2G_SMOOTHER_GAUSS_SEIDEL;
     if (!pipeOn) return;
     const bool fp64 = c.precision == B2G_PRECISION_FP64;
+    std::vector<std::pair<int, int>> wanted;  // {level, sweeps}
     auto want = [&](int lv, int s) {
-        if (s <= 0 || lv >= static_cast<int>(lev.size())) return;
-        if (fp64) preparePipe<double>(lv, s);
-        else preparePipe<float>(lv, s);
+        if (s > 0 && lv < static_cast<int>(lev.size())) wanted.push_back({lv, s});
     };
     want(0, c.nFinestSweeps);
     for (int lv = 1; lv < static_cast<int>(lev.size()); ++lv)
@@ -1438,6 +1469,23 @@ void Batch::preparePipes(const b2g_controls& c)
         const int li = lv - 1;
         want(lv, std::min(c.nPostSweeps + c.postSweepsLevelMultiplier * li, c.maxPostSweeps));
         if (c.nPreSweeps) want(lv, std::min(c.nPreSweeps + c.preSweepsLevelMultiplier * li, c.maxPreSweeps));
+    }
+    // every schedule that is missing, all levels together; then the levels' tables
+    const size_t vb = fp64 ? sizeof(double) : sizeof(float);
+    std::vector<FlowJob> jobs;
+    std::vector<int> jobCase;
+    for (const auto& w : wanted)
+        if (lev[w.first].nParts && !lev[w.first].pipe.count(w.second * 16 + static_cast<int>(vb)))
+            flowJobs(w.first, w.second, vb, jobs, jobCase);
+    if (!jobs.empty())
+    {
+        for (Matrix* A : cases) A->forgetFlows();
+        flowsForBatch(jobs, stream);
+    }
+    for (const auto& w : wanted)
+    {
+        if (fp64) preparePipe<double>(w.first, w.second);
+        else preparePipe<float>(w.first, w.second);
     }
 }
 

@@ -152,6 +152,7 @@ struct Batch
     bool denseAny = false;                  // some case has its dense factor
     void prepareDense();
     unsigned long long layoutFingerprint() const;
+    void flowJobs(int lv, int nSweeps, size_t vb, std::vector<struct FlowJob>& jobs, std::vector<int>& jobCase) const;
     template <class T> void preparePipe(int lv, int nSweeps);
     void preparePipes(const b2g_controls& c);
     // The cases' meshes, each once; a solve holds their schedules (Mesh::use), and forgets what it has tabulated of

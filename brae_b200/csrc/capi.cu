@@ -949,9 +949,6 @@ b2g_status b2g_flow_handovers(int nCells, int nFaces, const int32_t* lower, cons
         need(valueBytes == 4 || valueBytes == 8, "b2g_flow_handovers: valueBytes must be 4 or 8");
         b2g::FlowLevel H;
         H.n = nCells;
-        H.nF = nFaces;
-        H.lower.assign(lower, lower + nFaces);
-        H.upper.assign(upper, upper + nFaces);
         H.posCell.resize(nCells);
         H.posRow.assign(static_cast<size_t>(nCells) + 1, 0);
         for (int f = 0; f < nFaces; ++f)
@@ -968,10 +965,10 @@ b2g_status b2g_flow_handovers(int nCells, int nFaces, const int32_t* lower, cons
         }
         H.cellPos = H.posCell;
         // a row's lower neighbours, then its upper ones
-        H.entColPos.resize(2 * static_cast<size_t>(nFaces));
+        H.col.resize(2 * static_cast<size_t>(nFaces));
         std::vector<int> at(H.posRow.begin(), H.posRow.end() - 1);
-        for (int f = 0; f < nFaces; ++f) H.entColPos[at[upper[f]]++] = lower[f];
-        for (int f = 0; f < nFaces; ++f) H.entColPos[at[lower[f]]++] = upper[f];
+        for (int f = 0; f < nFaces; ++f) H.col[at[upper[f]]++] = lower[f];
+        for (int f = 0; f < nFaces; ++f) H.col[at[lower[f]]++] = upper[f];
         int visits = symmetric ? 2 * nSweeps : nSweeps, nSteps = 0;
         std::vector<int> T;
         if (colours)

@@ -8,6 +8,8 @@
 #include <atomic>
 #include <mutex>
 #include <set>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 namespace b2g {
@@ -55,9 +57,7 @@ struct Dropped
     }
     void take(FlowSchedule& F)
     {
-        take(F.chunkStart);
-        take(F.rec);
-        take(F.meta);
+        take(F.blob);
     }
 };
 
@@ -205,18 +205,15 @@ FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s)
 {
     FlowLevel H;
     H.n = L.nCells;
-    H.nF = L.nFaces;
-    H.lower = L.lower.download(s);
-    H.upper = L.upper.download(s);
-    H.posCell = L.gs.posCell.download(s);
-    H.posRow = L.gs.posRow.download(s);
-    H.entColPos = L.gs.entColPos.download(s);
-    H.lower.resize(H.nF);
-    H.upper.resize(H.nF);
-    H.posCell.resize(H.n);
-    H.posRow.resize(static_cast<size_t>(H.n) + 1);
-    H.cellPos.resize(H.n);
-    for (int p = 0; p < H.n; ++p) H.cellPos[H.posCell[p]] = p;
+    auto get = [&](const DBuf<int>& from, std::vector<int>& to, size_t n) {
+        to.resize(n);
+        if (n) B2G_CUDA(cudaMemcpyAsync(to.data(), from.p, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+    };
+    get(L.gs.posCell, H.posCell, H.n);
+    get(L.gs.posRow, H.posRow, static_cast<size_t>(H.n) + 1);
+    get(L.gs.entColPos, H.col, 2 * static_cast<size_t>(L.nFaces));
+    B2G_CUDA(cudaStreamSynchronize(s));
+    H.prepare();
     return H;
 }
 
@@ -227,8 +224,10 @@ std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T,
 {
     FlowProgram G;
     if (!flowRoom(0) || !buildFlowProgram(H, T, S, nSteps, R, vb, G)) return nullptr;
-    if (!flowRoom(G.metaBytes + sizeof(k::FlowRec) * G.rec.size() + vb * G.nVal)) return nullptr;
-    return uploadFlow(G, nSteps, R, s);
+    if (!flowRoom(G.deviceBytes(vb))) return nullptr;
+    std::unique_ptr<FlowSchedule> F = uploadFlow(G, nSteps, R, s);
+    B2G_CUDA(cudaStreamSynchronize(s));  // the host arrays go out of scope
+    return F;
 }
 
 std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int nSteps, int R, cudaStream_t s)
@@ -240,18 +239,20 @@ std::unique_ptr<FlowSchedule> uploadFlow(const FlowProgram& G, int nSteps, int R
     F->nSteps = nSteps;
     F->slots = G.slots;
     F->nVal = static_cast<long long>(G.nVal);
-    F->nChunks = static_cast<int>(G.rec.size());
-    F->meta.alloc(std::max<size_t>(G.metaBytes, 16), s);
-    size_t metaAt = 0;
+    F->nChunks = G.nChunks;
+    F->recAt = G.recAt;
+    F->metaAt = G.metaAt;
+    F->blob.alloc(G.blobBytes, s);
+    auto put = [&](size_t at, const std::vector<unsigned char>& v) {
+        if (!v.empty()) B2G_CUDA(cudaMemcpyAsync(F->blob.p + at, v.data(), v.size(), cudaMemcpyHostToDevice, s));
+    };
+    put(0, G.head);
+    size_t at = G.metaAt;
     for (const RankProgram& P : G.prog)
     {
-        if (!P.meta.empty())
-            B2G_CUDA(cudaMemcpyAsync(F->meta.p + metaAt, P.meta.data(), P.meta.size(), cudaMemcpyHostToDevice, s));
-        metaAt += P.meta.size();
+        put(at, P.meta);
+        at += P.meta.size();
     }
-    F->chunkStart.upload(G.chunkStart.data(), G.chunkStart.size(), s);
-    F->rec.upload(reinterpret_cast<const int4*>(G.rec.data()), 3 * G.rec.size(), s);
-    B2G_CUDA(cudaStreamSynchronize(s));  // the host arrays go out of scope
     return F;
 }
 
@@ -304,33 +305,43 @@ const T* Matrix::flowValuesOf(int level, const FlowSchedule& F)
         B.val.ensure(static_cast<size_t>(std::max<long long>(F.nVal, 1)), stream);
         if (F.nChunks)
             k::flowValues<T><<<std::min(F.nChunks, 8192), 32 * k::kFlowTeam, 0, stream>>>(
-                F.nChunks, F.rec.p, F.meta.p, mesh->lev[level].gs.posRow.p, D.coef[level].rowVal.p,
+                F.nChunks, F.rec(), F.meta(), mesh->lev[level].gs.posRow.p, D.coef[level].rowVal.p,
                 D.coef[level].gsDiag.p, B.val.p);
         B2G_LAUNCH_CHECK();
         if (F.ranks > 1 && !B.mail.p)
         {
             B.mail.alloc(2 * sizeof(T) * static_cast<size_t>(mesh->lev[level].nCells), stream);
             B.mail.zero(stream);
-            const unsigned first[2] = {1, 0};
-            B.ctl.upload(first, 2, stream);
-            B2G_CUDA(cudaStreamSynchronize(stream));  // first is on this frame
+            B.ctl.alloc(2, stream);
+            B.ctl.zero(stream);
         }
+        B.of = F.held;
         B.gen = coefGen;
     }
     return B.val.p;
 }
 
+void Matrix::forgetFlows()
+{
+    auto sweep = [](auto& flows) {
+        for (auto it = flows.begin(); it != flows.end();)
+            it = it->second.gen >= 0 && it->second.of.expired() ? flows.erase(it) : std::next(it);
+    };
+    sweep(v64.flows);
+    sweep(v32.flows);
+}
+
 // Whether this matrix has the schedule's values, filled here outside a capture; false when there is no memory
 // for them, and the level then runs its other form (tried again with the next solve).
 template <class T>
-bool Matrix::flowReady(int level, const FlowSchedule& F)
+bool Matrix::flowReady(int level, const FlowSchedule& F, bool room)
 {
     auto& flows = data<T>().flows;
     const auto it = flows.find(F.id);
     if (it != flows.end() && it->second.gen == coefGen) return true;
     if (capturing && it != flows.end() && it->second.refused == coefGen) return false;
     const bool have = it != flows.end() && it->second.val.p;  // (a refill, into the same buffer)
-    if ((capturing || have || flowRoom(sizeof(T) * static_cast<size_t>(F.nVal))) && attempt([&] { flowValuesOf<T>(level, F); }))
+    if ((capturing || have || room || flowRoom(sizeof(T) * static_cast<size_t>(F.nVal))) && attempt([&] { flowValuesOf<T>(level, F); }))
         return true;
     if (capturing) fail(B2G_ERR_STATE, "b2g: a smoothing schedule's values were not filled before the capture");
     flows.erase(F.id);
@@ -342,9 +353,9 @@ template <class T>
 k::FlowArgs<T> Matrix::flowArgs(int level, const FlowSchedule& F, T* psiL, const T* src)
 {
     k::FlowArgs<T> a;
-    a.chunkStart = F.chunkStart.p;
-    a.rec = F.rec.p;
-    a.meta = F.meta.p;
+    a.chunkStart = F.chunkStart();
+    a.rec = F.rec();
+    a.meta = F.meta();
     a.val = flowValuesOf<T>(level, F);
     a.b = src;
     a.psi = psiL;
@@ -498,49 +509,129 @@ void Matrix::refreshSymFlows()
             if (kv.second && kv.first % 16 == static_cast<int>(sizeof(T))) flowReady<T>(lv, *kv.second);
 }
 
-void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStream_t s)
+// The missing schedules go through three stages, a group of levels at a time: their addressing comes to the host, the
+// programs are built on its cores, the result goes to the device. While one group is built, the one before goes up
+// and the next one comes down.
+void flowsForBatch(std::vector<FlowJob>& jobs, cudaStream_t s)
 {
-    auto keyOf = [&](const FlowJob& j) { return std::pair<int, int>{nSweeps * 16 + static_cast<int>(vb), j.ranks}; };
-    struct Work
-    {
-        size_t job;
-        FlowLevel H;
-        FlowProgram G;
-        int nSteps = 0;
-        bool ok = false;
-    };
-    std::vector<Work> work;
+    constexpr long long kGroupItems = 4 << 20;  // items (cells times sweeps) of a group: some 0.4 GB of host memory
+    auto keyOf = [](const FlowJob& j) { return std::pair<int, int>{j.nSweeps * 16 + static_cast<int>(j.vb), j.ranks}; };
+    std::vector<size_t> missing;
     for (size_t i = 0; i < jobs.size(); ++i)
     {
-        auto known = jobs[i].level->flowBatch.find(keyOf(jobs[i]));
-        if (known != jobs[i].level->flowBatch.end()) continue;
+        auto& have = jobs[i].level->flowBatch;
+        if (have.count(keyOf(jobs[i]))) continue;
         // the level's schedules of this call for other CTA counts that no batch holds any more make room
-        for (auto it = jobs[i].level->flowBatch.begin(); it != jobs[i].level->flowBatch.end();)
+        for (auto it = have.begin(); it != have.end();)
         {
             const bool old = it->first.first == keyOf(jobs[i]).first && it->second && it->second->held.use_count() == 1;
-            it = old ? jobs[i].level->flowBatch.erase(it) : std::next(it);
+            it = old ? have.erase(it) : std::next(it);
         }
-        jobs[i].level->flowBatch[keyOf(jobs[i])];  // (a level listed twice is built once)
-        if (!flowRoom(0)) continue;
-        work.emplace_back();
-        work.back().job = i;
-        // (no memory for it, here and below: the level has no schedule)
-        if (!attempt([&] { work.back().H = flowDownload(*jobs[i].level, s); })) work.pop_back();
+        have[keyOf(jobs[i])];  // (a level listed twice is built once)
+        missing.push_back(i);
     }
-    flowParallel(static_cast<int>(work.size()), [&](int i, int) {
-        Work& w = work[i];
-        const int R = jobs[w.job].ranks;
-        attempt([&] {
-            const std::vector<int> steps = flowSteps(w.H, nSweeps, false, R, 4, w.nSteps);
-            w.ok = buildFlowProgram(w.H, steps, nSweeps, w.nSteps, R, vb, w.G);
-        });
-    });
-    for (Work& w : work)
+    struct Group
     {
-        const FlowJob& j = jobs[w.job];
-        if (w.ok && flowRoom(w.G.metaBytes + sizeof(k::FlowRec) * w.G.rec.size() + vb * w.G.nVal))
-            attempt([&] { j.level->flowBatch[keyOf(j)] = uploadFlow(w.G, w.nSteps, j.ranks, s); });
+        std::vector<size_t> job;
+        std::vector<FlowBuild> build;
+    };
+    size_t at = 0;
+    // (no memory for a level, here and below: it has no schedule)
+    auto fetch = [&] {
+        // the levels' arrays side by side on the device, then one copy: some hundred small ones cost more than it
+        Group g;
+        DBuf<int> side;
+        std::vector<int> host;
+        size_t ints = 0;
+        for (long long items = 0; at < missing.size() && items < kGroupItems; ++at)
+        {
+            const FlowJob& j = jobs[missing[at]];
+            items += static_cast<long long>(j.level->nCells) * j.nSweeps;
+            ints += 2 * static_cast<size_t>(j.level->nCells) + 1 + 2 * static_cast<size_t>(j.level->nFaces);
+            FlowBuild b;
+            b.S = j.nSweeps;
+            b.R = j.ranks;
+            b.vb = j.vb;
+            b.H.n = j.level->nCells;
+            g.job.push_back(missing[at]);
+            g.build.push_back(std::move(b));
+        }
+        auto each = [&](auto&& array) {
+            size_t from = 0;
+            for (size_t i = 0; i < g.job.size(); ++i)
+            {
+                const LevelAddr& L = *jobs[g.job[i]].level;
+                FlowLevel& H = g.build[i].H;
+                array(L.gs.posCell, H.posCell, from, static_cast<size_t>(L.nCells));
+                array(L.gs.posRow, H.posRow, from, static_cast<size_t>(L.nCells) + 1);
+                array(L.gs.entColPos, H.col, from, 2 * static_cast<size_t>(L.nFaces));
+            }
+        };
+        if (!g.job.empty() && (!flowRoom(sizeof(int) * ints) || !attempt([&] {
+                side.alloc(ints, s);
+                host.resize(ints);
+                each([&](const DBuf<int>& from, std::vector<int>&, size_t& to, size_t n) {
+                    if (n) B2G_CUDA(cudaMemcpyAsync(side.p + to, from.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
+                    to += n;
+                });
+                B2G_CUDA(cudaMemcpyAsync(host.data(), side.p, sizeof(int) * ints, cudaMemcpyDeviceToHost, s));
+                B2G_CUDA(cudaStreamSynchronize(s));
+                each([&](const DBuf<int>&, std::vector<int>& to, size_t& from, size_t n) {
+                    to.assign(host.begin() + from, host.begin() + from + n);
+                    from += n;
+                });
+            })))
+        {
+            g.job.clear();
+            g.build.clear();
+        }
+        return g;
+    };
+    auto upload = [&](const Group& g) {
+        size_t need = 0;
+        for (const FlowBuild& b : g.build)
+            if (b.ok) need += b.G.deviceBytes(b.vb);
+        const bool room = flowRoom(need);
+        for (size_t i = 0; i < g.job.size(); ++i)
+        {
+            const FlowJob& j = jobs[g.job[i]];
+            const FlowBuild& b = g.build[i];
+            if (b.ok && (room || flowRoom(b.G.deviceBytes(b.vb))))
+                attempt([&] { j.level->flowBatch[keyOf(j)] = uploadFlow(b.G, b.nSteps, b.R, s); });
+        }
+    };
+    Group built, next = fetch();
+    while (!next.job.empty() || at < missing.size())
+    {
+        Group now = std::move(next);
+        auto build = [&] {
+            if (!attempt([&] { buildFlowPrograms(now.build); }))
+                for (FlowBuild& b : now.build) b.ok = false;
+        };
+        {
+            struct Joined
+            {
+                std::thread t;
+                ~Joined()
+                {
+                    if (t.joinable()) t.join();
+                }
+            } worker;
+            try
+            {
+                worker.t = std::thread(build);
+            }
+            catch (const std::system_error&)
+            {
+                build();  // no more threads to be had
+            }
+            upload(built);
+            next = fetch();
+        }
+        built = std::move(now);
     }
+    upload(built);
+    B2G_CUDA(cudaStreamSynchronize(s));
     for (FlowJob& j : jobs) j.flow = j.level->flowBatch[keyOf(j)].get();
 }
 
@@ -580,8 +671,8 @@ template float Matrix::flowTime<double>(int, const FlowSchedule&, double*, const
 template float Matrix::flowTime<float>(int, const FlowSchedule&, float*, const float*, bool);
 template void Matrix::flowLaunch<double>(int, const FlowSchedule&, double*, const double*, bool);
 template void Matrix::flowLaunch<float>(int, const FlowSchedule&, float*, const float*, bool);
-template bool Matrix::flowReady<double>(int, const FlowSchedule&);
-template bool Matrix::flowReady<float>(int, const FlowSchedule&);
+template bool Matrix::flowReady<double>(int, const FlowSchedule&, bool);
+template bool Matrix::flowReady<float>(int, const FlowSchedule&, bool);
 template const double* Matrix::flowValuesOf<double>(int, const FlowSchedule&);
 template const float* Matrix::flowValuesOf<float>(int, const FlowSchedule&);
 

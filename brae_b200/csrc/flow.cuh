@@ -10,12 +10,24 @@
 
 namespace b2g {
 
-// The level's addressing on the host, as the schedule builder reads it.
+// The level's addressing on the host, as the schedule builder reads it, and the order of visits.
 struct FlowLevel
 {
-    int n = 0, nF = 0;
-    std::vector<int> lower, upper, posCell, posRow, entColPos, cellPos;
-    bool crosses = false;  // more than one rank
+    int n = 0;
+    std::vector<int> posCell, cellPos;  // cell of a position, position of a cell
+    std::vector<int> posRow, col;       // rows by position: their neighbours' cells (positions until prepare)
+    void prepare();                     // cellPos, and col's positions into cells
+    // The order of a visit: by colour where there are colours, else by cell; odd visits of a symmetric call run
+    // it backwards. A row reads the neighbours before its cell in the order at the same visit, the others at the
+    // visit before (-1: their initial value).
+    bool symmetric = false;
+    std::vector<int> colour;
+    int versionRead(int q, int c, int cn) const
+    {
+        const int d = colour.empty() ? cn - c : colour[cn] - colour[c];
+        return (symmetric && (q & 1) ? d > 0 : d < 0) ? q : q - 1;
+    }
+    bool crosses = false;               // more than one rank
 };
 
 // rank r's cells are [flowBegin(r), flowBegin(r + 1))
@@ -38,16 +50,21 @@ struct RankProgram
 struct FlowProgram
 {
     std::vector<RankProgram> prog;
-    std::vector<int> chunkStart;   // [ranks + 1]
-    std::vector<k::FlowRec> rec;
     int slots = 1;
-    size_t metaBytes = 0, nVal = 0;
+    size_t nVal = 0;
+    int nChunks = 0;
+    // FlowSchedule::blob up to the ranks' meta blobs, which follow one another at metaAt
+    std::vector<unsigned char> head;
+    size_t blobBytes = 0, recAt = 0, metaAt = 0;
+    // its device memory, the values of one matrix included
+    size_t deviceBytes(size_t vb) const { return blobBytes + vb * nVal; }
 };
 
 FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s);
-std::vector<int> flowSteps(const FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps);
-std::vector<int> colourSteps(const FlowLevel& H, const std::vector<int>& colourOf, int nColours, int nSweeps,
-                             bool symmetric, int R, int weight, int& visits, int& nSteps);
+// (both set the level's order)
+std::vector<int> flowSteps(FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps);
+std::vector<int> colourSteps(FlowLevel& H, const std::vector<int>& colourOf, int nColours, int nSweeps, bool symmetric,
+                             int R, int weight, int& visits, int& nSteps);
 // A program's hand-overs between ranks: values stored to a mailbox, values polled for; of the (cell, visit) pairs
 // stored those that no rank polls for, and of those polled for the ones that nothing stores.
 struct FlowHandOvers
@@ -61,15 +78,29 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
 // The same on the device, or null.
 std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb,
                                         cudaStream_t s);
-// The batched form's launches of nSweeps sweeps: per job its level on `ranks` CTAs, built once and kept on the
-// level, the missing ones side by side on the host's cores; job.flow is null when the level has none.
+// Programs of many levels (forward sweeps) side by side on the host's cores; ok is false where the level has
+// none. The levels' addressing is freed on the way.
+struct FlowBuild
+{
+    FlowLevel H;
+    int S = 0, R = 0, weight = 4;
+    size_t vb = 0;
+    std::vector<int> T;
+    int nSteps = 0;
+    FlowProgram G;
+    bool ok = false;
+};
+void buildFlowPrograms(std::vector<FlowBuild>& all);
+// The batched form's launches: per job its level's sweeps on `ranks` CTAs, built once and kept on the level; flow
+// is null when the level has none.
 struct FlowJob
 {
     LevelAddr* level;
-    int ranks;
+    int nSweeps, ranks;
+    size_t vb;
     const FlowSchedule* flow;
 };
-void flowsForBatch(std::vector<FlowJob>& jobs, int nSweeps, size_t vb, cudaStream_t s);
+void flowsForBatch(std::vector<FlowJob>& jobs, cudaStream_t s);
 // The batched launch (flow.cu): table = k::FlowArgs<T>[entries] on the device, blocks[i] = {entry, rank},
 // caseOf[entry] its case. `remote`: some entry has more than one rank (a cooperative launch).
 template <class T>

@@ -78,8 +78,8 @@ struct FlowRec
     int items8, fetch8, halo8, counts;          // its items, fetches and halo entries; nFetch | nHalo << 16
 };
 
-// The meta blob: [slices: nSl x 16 bytes (FlowSlice)][items: 32 nSl x {position, slot word}][fetches: nF x
-// {position, slot}][halo: nH x {position, slot | visit << 16}][codes], each 16-byte aligned; the value blob
+// The meta blob: [slices: nSl x 16 bytes (FlowSlice)][items: 32 nSl x {position, slot word}][codes][fetches: nF x
+// {position, slot}][halo: nH x {position, slot | visit << 16}], each 16-byte aligned; the value blob
 // follows it in the ring: [{diagonal, its reciprocal}: 32 nSl][coefficients]; then the source: 32 nSl. A slot
 // word is slot | visit << 16 | export << 30 | last << 31. Entries are sliced ELL in groups a lane reads with one load: four
 // codes (group g of lane l at stride * g + l, the stride being the slice's items rounded up to 8), two FP64 or
@@ -106,7 +106,7 @@ struct FlowArgs
     const T* __restrict__ b;                    // by position
     T* psi;                                     // by position
     void* mail;                                 // {value, tag} by position
-    unsigned* ctl;                              // [0] the launch's epoch, [1] ranks that have finished
+    unsigned* ctl;                              // [0] the launches so far, [1] ranks that have finished
                                                 // (null: one rank)
     int ranks;
     int slots;                                  // value slots (the ring follows them)
@@ -401,7 +401,7 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
     const unsigned ringA = xA + static_cast<unsigned>(flowRingAt(a.slots, sizeof(T)));
     const int c0 = a.chunkStart[rank];
     const int nCh = a.chunkStart[rank + 1] - c0;
-    const unsigned epoch = kRemote && a.ctl ? *reinterpret_cast<volatile unsigned*>(a.ctl) : 0u;
+    const unsigned epoch = kRemote && a.ctl ? *reinterpret_cast<volatile unsigned*>(a.ctl) + 1u : 0u;
     const unsigned tag0 = (epoch << 6) + 1u;
     const unsigned tagOut = a.publish ? tag0 : 0u;  // epochs start at 1: no tag is met when not publishing
     if (t == 0)
@@ -589,7 +589,7 @@ __device__ __forceinline__ void flowBody(const FlowArgs<T>& a, const int rank)
         if (t == 0 && atomicAdd(a.ctl + 1, 1u) == static_cast<unsigned>(a.ranks - 1))
         {
             a.ctl[1] = 0;
-            a.ctl[0] = epoch + 1;
+            a.ctl[0] = epoch;
         }
     }
 }

@@ -26,32 +26,44 @@ struct RankScratch
     std::vector<int> localOf;  // cell -> ghost index of the rank at work, -1
 };
 
-// An item as a sort key: [first: its step's other chunks go before it][65535 - row width][position][visit][out:
-// another rank reads it]
+// An item: [row width][position][visit][out: another rank reads it]
 struct ItemRef
 {
     unsigned long long key;
     int p() const { return static_cast<int>(key >> 7 & 0x7fffffffu); }
     int q() const { return static_cast<int>(key >> 1 & 0x3fu); }
-    int w() const { return 65535 - static_cast<int>(key >> 38 & 0xffffu); }
+    int w() const { return static_cast<int>(key >> 38); }
     bool out() const { return key & 1u; }
 };
 static_assert(k::kFlowMaxVisits < 64, "a visit has 6 bits of the key");
 ItemRef itemRef(int p, int q, int w, bool out)
 {
-    return {static_cast<unsigned long long>(65535 - std::min(w, 65535)) << 38 | static_cast<unsigned long long>(p) << 7 |
+    return {static_cast<unsigned long long>(w) << 38 | static_cast<unsigned long long>(p) << 7 |
             static_cast<unsigned long long>(q) << 1 | (out ? 1u : 0u)};
 }
-constexpr unsigned long long kItemLater = 1ull << 62;
 
-// The visit of cell cn whose value visit q of its neighbour c reads: its latest before that item (-1: the
-// initial value)
-int versionRead(const std::vector<int>& T, size_t n, int q, int c, int cn)
+// A step's items, those that another rank reads first (`apart`), then the longest rows, a counting sort; equal ones
+// stay as they are: by visit, then by cell.
+void sortStep(ItemRef* items, int m, bool apart, std::vector<ItemRef>& sorted)
 {
-    const int step = T[q * n + c];
-    int ver = q;
-    while (ver >= 0 && T[ver * n + cn] >= step) --ver;
-    return ver;
+    constexpr int kW = 256;  // (longer rows have no schedule: their order does not matter)
+    int lo = kW, hi = 0;
+    auto bucket = [&](const ItemRef& x) { return (apart && !x.out() ? kW : 0) + kW - 1 - std::min(x.w(), kW - 1); };
+    if (m < 2) return;
+    int count[2 * kW + 1];
+    std::memset(count, 0, sizeof(count));
+    for (int i = 0; i < m; ++i)
+    {
+        const int b = bucket(items[i]);
+        ++count[b + 1];
+        lo = std::min(lo, b);
+        hi = std::max(hi, b);
+    }
+    if (lo == hi) return;
+    for (int b = lo; b <= hi; ++b) count[b + 1] += count[b];
+    sorted.resize(m);
+    for (int i = 0; i < m; ++i) sorted[count[bucket(items[i])]++] = items[i];
+    std::memcpy(items, sorted.data(), sizeof(ItemRef) * static_cast<size_t>(m));
 }
 
 void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int c0, int c1, size_t vb,
@@ -59,7 +71,7 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
 {
     const size_t n = static_cast<size_t>(H.n);
     const int nOwn = c1 - c0;
-    if (X.localOf.size() != n) X.localOf.assign(n, -1);
+    if (X.localOf.size() < n) X.localOf.resize(n, -1);  // (every entry is -1 again when a rank is done)
     // the visits of a cell whose value another rank reads, a bit each
     std::vector<unsigned long long> exported(nOwn, 0);
     if (H.crosses)
@@ -68,11 +80,11 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
             const int p = H.cellPos[c];
             for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e)
             {
-                const int cn = H.posCell[H.entColPos[e]];
+                const int cn = H.col[e];
                 if (cn >= c0 && cn < c1) continue;
                 for (int q = 0; q < S; ++q)
                 {
-                    const int ver = versionRead(T, n, q, cn, c);
+                    const int ver = H.versionRead(q, cn, c);
                     if (ver >= 0) exported[c - c0] |= 1ull << ver;
                 }
             }
@@ -85,11 +97,20 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
     for (int i = 0; i < nSteps; ++i) start[i + 1] += start[i];
     std::vector<ItemRef> items(static_cast<size_t>(S) * nOwn);
     {
+        // a step's items of a visit by cell, in a colour's step by position: the order that coalesces better (a call
+        // of two sweeps on 2 M cells 0.77 ms by position, 0.72 by cell; a multicolour solve of 4 M cells 39.8 ms by
+        // position, 40.6 by cell)
+        std::vector<int> own;
+        if (!H.colour.empty())
+        {
+            for (int c = c0; c < c1; ++c) own.push_back(H.cellPos[c]);
+            std::sort(own.begin(), own.end());
+        }
         std::vector<int> cur(start.begin(), start.end() - 1);
         for (int q = 0; q < S; ++q)
-            for (int c = c0; c < c1; ++c)
+            for (int i = 0; i < nOwn; ++i)
             {
-                const int p = H.cellPos[c];
+                const int p = own.empty() ? H.cellPos[c0 + i] : own[i], c = H.posCell[p];
                 items[cur[T[q * n + c]]++] = itemRef(p, q, H.posRow[p + 1] - H.posRow[p], exported[c - c0] >> q & 1u);
             }
     }
@@ -98,15 +119,12 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         int a, b;
     };
     std::vector<Span> chunks;
+    std::vector<ItemRef> sorted;
     for (int st = 0; st < nSteps; ++st)
     {
         const int a = start[st], b = start[st + 1];
         if (a == b) continue;
-        const bool several = b - a > kFlowChunkItems;
-        if (several)
-            for (int i = a; i < b; ++i)
-                if (!items[i].out()) items[i].key |= kItemLater;
-        std::sort(items.begin() + a, items.begin() + b, [](const ItemRef& x, const ItemRef& y) { return x.key < y.key; });
+        sortStep(items.data() + a, b - a, b - a > kFlowChunkItems, sorted);
         // cut where the chunk is full: whole slices, its blobs and source within its share of the ring
         int from = a;
         size_t bytes = 64;
@@ -132,7 +150,8 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         chunks.push_back({from, b});
     }
     const int nCh = static_cast<int>(chunks.size());
-    // first pass: each local value's last use. Own cells are 0..nOwn-1, ghosts follow as they are met.
+    // first pass: each local value's last use, which is a last visit of its cell or of a neighbour (visits of a cell
+    // come in order). Own cells are 0..nOwn-1, ghosts follow as they are met.
     std::vector<int> last(nOwn, -1), ghostCell;
     auto localId = [&](int cell) {
         if (cell >= c0 && cell < c1) return cell - c0;
@@ -149,9 +168,10 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
     for (int j = 0; j < nCh; ++j)
         for (int i = chunks[j].a; i < chunks[j].b; ++i)
         {
+            if (items[i].q() != S - 1) continue;
             const int p = items[i].p();
             last[H.posCell[p] - c0] = j;
-            for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e) last[localId(H.posCell[H.entColPos[e]])] = j;
+            for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e) last[localId(H.col[e])] = j;
         }
     // second pass: slots (a value's from its first use to kFlowDepth chunks after its last), the
     // fetches of initial values, the ghosts' arrivals, the chunks' blobs
@@ -175,7 +195,6 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
     for (const ItemRef& it : items) rowEntries += static_cast<size_t>((it.w() + 3) & ~3);
     P.meta.reserve(16 * items.size() + rowEntries * 5 / 2 + 1024 * static_cast<size_t>(nCh));
     std::vector<Pair> fetch, halo;
-    std::vector<unsigned short> codes;
     int width[kFlowChunkItems / 32 + 1], first[kFlowChunkItems / 32 + 1];
     long long valAt = 0;
     for (int j = 0; j < nCh; ++j)
@@ -205,44 +224,47 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         }
         fetch.clear();
         halo.clear();
-        codes.assign(nEnt, 0);
+        const size_t itemsAt = 16 * static_cast<size_t>(nSl), codesAt = itemsAt + 256 * static_cast<size_t>(nSl);
+        const size_t fetchAt = codesAt + (2 * static_cast<size_t>(nEnt) + 15) / 16 * 16;
+        const size_t at = P.meta.size();
+        P.meta.resize(at + fetchAt, 0);
+        unsigned short* codes = reinterpret_cast<unsigned short*>(P.meta.data() + at + codesAt);
         // (a chunk's values are read before its items write: every read first, then the writes)
         for (int i = 0; i < m; ++i)
         {
             const int p = items[a + i].p(), visitOf = items[a + i].q();
             const int c = H.posCell[p];
-            const int st = k::flowStride(m, i / 32);
-            const int at0 = first[i / 32], l = i % 32;
-            for (int e = H.posRow[p], q = 0; e < H.posRow[p + 1]; ++e, ++q)
+            // (code q of lane l at 4 * (stride * (q / 4) + l) + q % 4)
+            const int jump = 4 * (k::flowStride(m, i / 32) - 1);
+            unsigned short* to = codes + first[i / 32] + 4 * (i % 32);
+            for (int e = H.posRow[p], q = 0; e < H.posRow[p + 1]; ++e, ++q, ++to)
             {
-                const int pn = H.entColPos[e];
-                const int cn = H.posCell[pn];
+                const int cn = H.col[e];
                 const int v = localId(cn);
-                const int ver = versionRead(T, n, visitOf, c, cn);
+                if (q && q % 4 == 0) to += jump;
                 if (v < nOwn)
                 {
                     if (!slot[v])
                     {
                         give(v);
-                        fetch.push_back({static_cast<unsigned>(pn), static_cast<unsigned>(slot[v])});
+                        fetch.push_back({static_cast<unsigned>(H.cellPos[cn]), static_cast<unsigned>(slot[v])});
                     }
                 }
-                else if (ver > visit[v])
+                else if (const int ver = H.versionRead(visitOf, c, cn); ver > visit[v])
                 {
                     give(v);
                     if (ver < 0)
-                        fetch.push_back({static_cast<unsigned>(pn), static_cast<unsigned>(slot[v])});
+                        fetch.push_back({static_cast<unsigned>(H.cellPos[cn]), static_cast<unsigned>(slot[v])});
                     else
-                        halo.push_back({static_cast<unsigned>(pn), static_cast<unsigned>(slot[v]) | static_cast<unsigned>(ver) << 16});
+                        halo.push_back({static_cast<unsigned>(H.cellPos[cn]), static_cast<unsigned>(slot[v]) | static_cast<unsigned>(ver) << 16});
                     visit[v] = ver;
                 }
-                codes[at0 + 4 * (st * (q / 4) + l) + q % 4] = static_cast<unsigned short>(slot[v]);
+                *to = static_cast<unsigned short>(slot[v]);
             }
         }
         for (int i = 0; i < m; ++i) give(H.posCell[items[a + i].p()] - c0);
-        const size_t itemsAt = 16 * static_cast<size_t>(nSl), fetchAt = itemsAt + 256 * static_cast<size_t>(nSl);
-        const size_t haloAt = fetchAt + (fetch.size() + 1) / 2 * 16, codesAt = haloAt + (halo.size() + 1) / 2 * 16;
-        const size_t metaBytes = codesAt + (2 * static_cast<size_t>(nEnt) + 15) / 16 * 16;
+        const size_t haloAt = fetchAt + (fetch.size() + 1) / 2 * 16;
+        const size_t metaBytes = haloAt + (halo.size() + 1) / 2 * 16;
         const size_t valsAt = metaBytes + 64 * static_cast<size_t>(nSl) * vb, srcBytesAt = valsAt + nEnt * vb;
         // (offsets within a chunk count 8 bytes in 16 bits)
         if (P.slots > k::kFlowMaxSlots || vb * P.slots > kFlowSmem || srcBytesAt + 32 * static_cast<size_t>(nSl) * vb > 8 * 65535u ||
@@ -251,7 +273,6 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
             P.ok = false;
             break;
         }
-        const size_t at = P.meta.size();
         P.meta.resize(at + metaBytes, 0);
         unsigned char* M = P.meta.data() + at;
         for (int s = 0; s < nSl; ++s)
@@ -278,7 +299,6 @@ void buildRank(const FlowLevel& H, const std::vector<int>& T, int S, int nSteps,
         }
         if (!fetch.empty()) std::memcpy(M + fetchAt, fetch.data(), 8 * fetch.size());
         if (!halo.empty()) std::memcpy(M + haloAt, halo.data(), 8 * halo.size());
-        if (nEnt) std::memcpy(M + codesAt, codes.data(), 2 * static_cast<size_t>(nEnt));
         k::FlowRec& r = P.rec[j];
         r.meta16 = static_cast<int>(at / 16);
         r.metaBytes = static_cast<int>(metaBytes);
@@ -327,6 +347,17 @@ bool placeInRing(std::vector<k::FlowRec>& rec, size_t ring, size_t vb)
 
 }  // namespace
 
+void FlowLevel::prepare()
+{
+    cellPos.resize(n);
+    for (int p = 0; p < n; ++p) cellPos[posCell[p]] = p;
+    constexpr int kBlock = 1 << 16;
+    const int m = static_cast<int>(col.size());
+    flowParallel((m + kBlock - 1) / kBlock, [&](int b, int) {
+        for (int e = b * kBlock; e < std::min(m, (b + 1) * kBlock); ++e) col[e] = posCell[col[e]];
+    });
+}
+
 void flowParallel(int n, const std::function<void(int, int)>& body)
 {
     // a loop within a loop runs on its own thread: the outer one has the cores
@@ -372,38 +403,39 @@ void flowParallel(int n, const std::function<void(int, int)>& body)
 // order, with the forward values, and the walk subtracts its own faces' terms ascending: the row's terms in
 // the row's order again. So a backward visit q is the same row reading its lower neighbours at visit q - 1
 // and its upper ones at visit q.
-std::vector<int> flowSteps(const FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps)
+std::vector<int> flowSteps(FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps)
 {
     const int S = symmetric ? 2 * nSweeps : nSweeps;
     const size_t n = static_cast<size_t>(H.n);
+    H.symmetric = symmetric;
+    H.colour.clear();
     std::vector<int> T(static_cast<size_t>(S) * n, 0);
-    std::vector<unsigned char> cross(R > 1 ? H.nF : 0);
-    if (R > 1)
-        for (int f = 0; f < H.nF; ++f) cross[f] = flowRank(H.lower[f], H.n, R) != flowRank(H.upper[f], H.n, R);
-    const int extra = weight - 1;
-    auto at = [&](int f) { return 1 + (R > 1 && cross[f] ? extra : 0); };
+    nSteps = 0;
     for (int s = 0; s < S; ++s)
     {
         int* cur = T.data() + s * n;
         const int* prev = s > 0 ? T.data() + (s - 1) * n : nullptr;
         const bool back = symmetric && (s & 1);
-        // the cell itself and the neighbours the walk has not reached: their previous visit
-        if (prev)
+        // cells in the walk's order: each neighbour the walk has passed is final at this visit
+        for (int i = 0; i < R; ++i)
         {
-            for (size_t c = 0; c < n; ++c) cur[c] = prev[c] + 1;
-            for (int f = 0; f < H.nF; ++f)
+            const int r = back ? R - 1 - i : i;
+            const int c0 = flowBegin(r, H.n, R), c1 = flowBegin(r + 1, H.n, R);
+            for (int x = c0; x < c1; ++x)
             {
-                const int c = back ? H.upper[f] : H.lower[f], o = back ? H.lower[f] : H.upper[f];
-                cur[c] = std::max(cur[c], prev[o] + at(f));
+                const int c = back ? c1 - 1 - (x - c0) : x, p = H.cellPos[c];
+                int t = prev ? prev[c] + 1 : 0;
+                for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e)
+                {
+                    const int o = H.col[e], w = o < c0 || o >= c1 ? weight : 1;
+                    if ((o < c) != back) t = std::max(t, cur[o] + w);
+                    else if (prev) t = std::max(t, prev[o] + w);
+                }
+                cur[c] = t;
+                nSteps = std::max(nSteps, t + 1);
             }
         }
-        // those it has: this visit (faces are sorted by owner, so in this order each is final when read)
-        if (!back)
-            for (int f = 0; f < H.nF; ++f) cur[H.upper[f]] = std::max(cur[H.upper[f]], cur[H.lower[f]] + at(f));
-        else
-            for (int f = H.nF - 1; f >= 0; --f) cur[H.lower[f]] = std::max(cur[H.lower[f]], cur[H.upper[f]] + at(f));
     }
-    nSteps = T.empty() ? 0 : *std::max_element(T.begin(), T.end()) + 1;
     return T;
 }
 
@@ -413,10 +445,12 @@ std::vector<int> flowSteps(const FlowLevel& H, int nSweeps, bool symmetric, int 
 // Every row still reads its neighbours of earlier colours at this visit and the others at the one before, as the
 // colour-by-colour sweep does. Symmetric sweeps visit the colours forward then back, each cell twice a sweep.
 // Empty when a cell has no colour.
-std::vector<int> colourSteps(const FlowLevel& H, const std::vector<int>& colourOf, int nColours, int nSweeps,
-                             bool symmetric, int R, int weight, int& visits, int& nSteps)
+std::vector<int> colourSteps(FlowLevel& H, const std::vector<int>& colourOf, int nColours, int nSweeps, bool symmetric,
+                             int R, int weight, int& visits, int& nSteps)
 {
     const int n = H.n;
+    H.symmetric = symmetric;
+    H.colour = colourOf;
     std::vector<int> byColour(n), start(static_cast<size_t>(nColours) + 1, 0);
     for (int c = 0; c < n; ++c)
     {
@@ -451,7 +485,7 @@ std::vector<int> colourSteps(const FlowLevel& H, const std::vector<int>& colourO
                     int t = prev ? prev[c] + 1 : 0;
                     for (int e = H.posRow[p]; e < H.posRow[p + 1]; ++e)
                     {
-                        const int o = H.posCell[H.entColPos[e]];
+                        const int o = H.col[e];
                         const bool earlier = back ? colourOf[o] > k : colourOf[o] < k;
                         if (!earlier && !prev) continue;
                         t = std::max(t, (earlier ? cur[o] : prev[o]) + (R > 1 && rank[o] != rank[c] ? weight : 1));
@@ -465,24 +499,30 @@ std::vector<int> colourSteps(const FlowLevel& H, const std::vector<int>& colourO
     return T;
 }
 
-bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb, FlowProgram& F)
+namespace {
+
+bool startFlowProgram(FlowLevel& H, int S, int R, FlowProgram& F)
 {
     if (H.n == 0 || R < 1 || R > H.n || S < 1 || S > k::kFlowMaxVisits) return false;
     H.crosses = R > 1;
     F.prog.clear();
     F.prog.resize(R);
-    std::vector<RankScratch> scratch(kFlowThreads);
-    flowParallel(R, [&](int r, int w) {
-        buildRank(H, T, S, nSteps, flowBegin(r, H.n, R), flowBegin(r + 1, H.n, R), vb, scratch[w], F.prog[r]);
-    });
+    return true;
+}
+
+// The ranks' programs as one: their common slots, their places in the ring, the blob.
+bool finishFlowProgram(int R, size_t vb, FlowProgram& F)
+{
     F.slots = 1;
-    F.metaBytes = F.nVal = 0;
+    size_t metaBytes = 0, chunks = 0;
+    F.nVal = 0;
     for (const RankProgram& P : F.prog)
     {
         if (!P.ok) return false;
         F.slots = std::max(F.slots, P.slots);
-        F.metaBytes += P.meta.size();
+        metaBytes += P.meta.size();
         F.nVal += P.nVal;
+        chunks += P.rec.size();
     }
     // the ring holds three chunks at least: one computed, one loaded by the other team, one on its way
     const size_t ringAt = k::flowRingAt(F.slots, vb);
@@ -491,25 +531,84 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
         for (const k::FlowRec& r : P.rec)
             chunk = std::max(chunk, static_cast<size_t>(r.metaBytes) + r.valBytes + 32 * static_cast<size_t>(r.nSlices) * vb);
     if (ringAt + 3 * chunk > kFlowSmem) return false;
-    if (F.metaBytes / 16 > 0x7fffffffull || F.nVal * vb / 16 > 0x7fffffffull) return false;
-    F.chunkStart.assign(static_cast<size_t>(R) + 1, 0);
-    F.rec.clear();
-    size_t metaAt = 0, valAt = 0;
+    if (metaBytes / 16 > 0x7fffffffull || F.nVal * vb / 16 > 0x7fffffffull || chunks > 0x7fffffffull) return false;
+    for (RankProgram& P : F.prog)
+        if (!placeInRing(P.rec, kFlowSmem - ringAt, vb)) return false;
+    F.nChunks = static_cast<int>(chunks);
+    F.recAt = (sizeof(int) * (static_cast<size_t>(R) + 1) + 15) / 16 * 16;
+    F.metaAt = F.recAt + sizeof(k::FlowRec) * chunks;
+    F.blobBytes = F.metaAt + metaBytes;
+    F.head.assign(F.metaAt, 0);
+    size_t chunkAt = 0, metaAt = 0, valAt = 0;
     for (int r = 0; r < R; ++r)
     {
-        RankProgram& P = F.prog[r];
-        if (!placeInRing(P.rec, kFlowSmem - ringAt, vb)) return false;
+        const RankProgram& P = F.prog[r];
+        k::FlowRec* to = reinterpret_cast<k::FlowRec*>(F.head.data() + F.recAt) + chunkAt;
         for (k::FlowRec x : P.rec)
         {
             x.meta16 += static_cast<int>(metaAt / 16);
             x.val16 += static_cast<int>(valAt * vb / 16);
-            F.rec.push_back(x);
+            *to++ = x;
         }
-        F.chunkStart[r + 1] = static_cast<int>(F.rec.size());
+        chunkAt += P.rec.size();
+        reinterpret_cast<int*>(F.head.data())[r + 1] = static_cast<int>(chunkAt);
         metaAt += P.meta.size();
         valAt += P.nVal;
     }
     return true;
+}
+
+}  // namespace
+
+bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb, FlowProgram& F)
+{
+    if (!startFlowProgram(H, S, R, F)) return false;
+    std::vector<RankScratch> scratch(kFlowThreads);
+    flowParallel(R, [&](int r, int w) {
+        buildRank(H, T, S, nSteps, flowBegin(r, H.n, R), flowBegin(r + 1, H.n, R), vb, scratch[w], F.prog[r]);
+    });
+    return finishFlowProgram(R, vb, F);
+}
+
+void buildFlowPrograms(std::vector<FlowBuild>& all)
+{
+    const int n = static_cast<int>(all.size());
+    // the largest first; then all their ranks, one list, so that a large level's ranks are shared out too
+    std::vector<int> order(n);
+    for (int i = 0; i < n; ++i) order[i] = i;
+    std::sort(order.begin(), order.end(), [&](int x, int y) {
+        return static_cast<long long>(all[x].H.n) * all[x].S > static_cast<long long>(all[y].H.n) * all[y].S;
+    });
+    flowParallel(n, [&](int i, int) {
+        FlowBuild& b = all[order[i]];
+        b.ok = attempt([&] {
+            b.H.prepare();
+            b.T = flowSteps(b.H, b.S, false, b.R, b.weight, b.nSteps);
+        }) && startFlowProgram(b.H, b.S, b.R, b.G);
+    });
+    std::vector<std::pair<int, int>> ranks;
+    for (int i : order)
+        if (all[i].ok)
+            for (int r = 0; r < all[i].R; ++r) ranks.push_back({i, r});
+    std::vector<RankScratch> scratch(kFlowThreads);
+    flowParallel(static_cast<int>(ranks.size()), [&](int i, int w) {
+        FlowBuild& b = all[ranks[i].first];
+        RankProgram& P = b.G.prog[ranks[i].second];
+        const int r = ranks[i].second;
+        if (!attempt([&] {
+                buildRank(b.H, b.T, b.S, b.nSteps, flowBegin(r, b.H.n, b.R), flowBegin(r + 1, b.H.n, b.R), b.vb, scratch[w], P);
+            }))
+        {
+            P.ok = false;
+            scratch[w].localOf.clear();
+        }
+    });
+    flowParallel(n, [&](int i, int) {
+        FlowBuild& b = all[i];
+        if (b.ok) b.ok = attempt([&] { b.ok = finishFlowProgram(b.R, b.vb, b.G); }) && b.ok;
+        b.T = std::vector<int>();
+        b.H = FlowLevel();
+    });
 }
 
 // Every hand-over of a program, replayed in step order.

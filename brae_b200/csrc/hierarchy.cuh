@@ -104,15 +104,17 @@ struct FlowSchedule
 {
     long long id = 0;             // names the schedule in the matrices' value buffers
     std::shared_ptr<char> held = std::make_shared<char>();  // copies of it: batches whose launches read the schedule
-    size_t bytes() const { return chunkStart.bytes() + rec.bytes() + meta.bytes(); }
+    size_t bytes() const { return blob.bytes(); }
     int ranks = 0;
     int nSteps = 0;
     int slots = 0;                // value slots of a CTA
     int nChunks = 0;
     long long nVal = 0;           // values (k::flowValues fills them)
-    DBuf<int> chunkStart;         // [ranks + 1]
-    DBuf<int4> rec;               // [chunks][3] k::FlowRec
-    DBuf<unsigned char> meta;     // the chunks' meta blobs
+    DBuf<unsigned char> blob;     // [chunk starts: ranks + 1][records: chunks x 3 int4 (k::FlowRec)][the chunks' meta blobs]
+    size_t recAt = 0, metaAt = 0;
+    const int* chunkStart() const { return reinterpret_cast<const int*>(blob.p); }
+    const int4* rec() const { return reinterpret_cast<const int4*>(blob.p + recAt); }
+    const unsigned char* meta() const { return blob.p + metaAt; }
 };
 
 // The dynamic shared memory of a pipelined launch in values of valueBytes (pipe.cu): the rank's

@@ -75,6 +75,7 @@ struct VCycleData
         DBuf<unsigned char> mail;   // {value, tag} by position, and the launch counter with the ranks that
         DBuf<unsigned> ctl;         // have finished (more than one rank)
         long long gen = -1;
+        std::weak_ptr<char> of;     // the schedule's FlowSchedule::held: gone with the schedule
         long long refused = -1;     // the generation whose values found no memory (flowReady)
     };
     std::map<long long, FlowBuffers> flows;
@@ -208,7 +209,8 @@ struct Matrix
     template <class T> void refreshItems();
     // the data-flow launch of a smoothing call (flow.cu)
     template <class T> const T* flowValuesOf(int level, const FlowSchedule& F);
-    template <class T> bool flowReady(int level, const FlowSchedule& F);
+    template <class T> bool flowReady(int level, const FlowSchedule& F, bool room = false);
+    void forgetFlows();                       // the values of schedules that are gone
     template <class T> k::FlowArgs<T> flowArgs(int level, const FlowSchedule& F, T* psi, const T* source);
     template <class T> void flowLaunch(int level, const FlowSchedule& F, T* psi, const T* source, bool fma = false);
     template <class T> bool flowForced(int level, T* psi, const T* source, int nSweeps, bool symmetric, int ranks, int weight, float* ms);

@@ -224,3 +224,30 @@ def test_batched_wait_gives_up(b2g, precision):
     assert batch.solve(srcs, again, ctl) == perfs
     for a, b in zip(first, again):
         assert np.array_equal(a, b)
+
+
+def test_batches_of_other_compositions(b2g):
+    # a mesh's levels get their CTA counts from the batch it is in: alone, among a few and among all, in turn, each
+    # with schedules of its own, of which those that no batch holds any more go; every result the same bits
+    built, meshes, mats = _build(b2g, BOXES)
+    for precision in ("fp64", "fp32_precond"):
+        ctl = b2g.controls_default(tolerance=1e-8, relTol=0.0, precision=precision)
+        want = None
+        kept = []
+        for members in (range(6), [4], [2, 4], range(6), [0, 2, 4, 5], [4]):
+            members = list(members)
+            batch = b2g.Batch([mats[k] for k in members])
+            kept.append(batch)  # some batches stay, with their schedules
+            if len(kept) > 2:
+                kept.pop(0)
+            psis = [np.zeros(built[k].n_cells) for k in members]
+            perfs = batch.solve([built[k].source for k in members], psis, ctl)
+            if want is None:
+                want = dict(zip(members, zip(psis, perfs)))
+            for k, psi, perf in zip(members, psis, perfs):
+                assert tuple(perf) == tuple(want[k][1]) and np.array_equal(psi, want[k][0]), (precision, members, k)
+        # a batch solved again after others have come and gone
+        psis = [np.zeros(built[k].n_cells) for k in (0, 2, 4, 5)]
+        kept[0].solve([built[k].source for k in (0, 2, 4, 5)], psis, ctl)
+        for k, psi in zip((0, 2, 4, 5), psis):
+            assert np.array_equal(psi, want[k][0])
