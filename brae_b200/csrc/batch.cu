@@ -26,7 +26,12 @@ constexpr int kTile = 2048;   // cells per tile
 // smoothing call, data flow against the sweep-by-sweep launch): 0.53 M cells 0.64 and 2.16, 1.07 M 0.84 and 2.00, 2.14 M
 // 1.02 and 2.07, 4.28 M 1.52 and 1.71, 8.56 M 2.42 and 1.53. Many cases fill the SMs by themselves.
 constexpr long long kFlowBatchCells = 3000000;
-constexpr int kFlowBatchShare = 1600;     // its cells per CTA, while the CTAs fit the SMs
+// Cells per CTA: the fine share where every CTA of a level then fits the SMs, else the coarse one. Two, and no share
+// by the batch's company, so that a mesh has two schedules of a level however many batches it passes through (a
+// server's groups are all different). Coarse shares of 2,500, 4,000, 5,600, 8,000 and 11,000 measured, ms a solve: 24 cases
+// of 1.1 M cells 41.3, 40.0, 39.6, 40.7, 45.0; 40 of 8.6 M cells 116.3, 110.3, 112.8, 113.1, 117.7; by the company, to fill
+// the SMs in one launch, 38.4 and 109.8.
+constexpr int kFlowBatchShares[2] = {1600, 4000};
 constexpr int kWarpsPerBlock = BT / 32;
 
 int warpGrid(int n) { return std::max(1, ceilDiv(n, kWarpsPerBlock)); }
@@ -1202,8 +1207,7 @@ void Batch::smooth(int lv, int nSweeps)
     auto pit = B.pipe.find(nSweeps * 16 + static_cast<int>(sizeof(T)));
     if (pipeOn && pit != B.pipe.end() && pit->second.use)
     {
-        // every sweep of the cases with a data-flow schedule in one launch (two when the cases with one CTA
-        // each do not fit beside the others); the rest below
+        // every sweep of the cases with a data-flow schedule in one launch each; the rest below
         const BatchLevel::Pipe& P = pit->second;
         for (const BatchLevel::FlowBlocks& F : P.flow)
             if (F.n)
@@ -1226,10 +1230,9 @@ void Batch::smooth(int lv, int nSweeps)
 }
 
 // The batched sweeps of level lv for nSweeps sweeps as data-flow launches (flow_kernels.cuh): each case's
-// level on a share of the SMs by its size, a power of two of CTAs (so a mesh keeps few schedules). All in one
-// cooperative launch while the CTAs fit the SMs; the cases with one CTA, which wait for nobody, in a launch of
-// their own when not. None when the cases' levels together have more than kFlowBatchCells cells. The level's
-// jobs, case by case.
+// level on a power of two of CTAs by its size. Cooperative launches of whole cases, each as many as fit the SMs;
+// the cases with one CTA, which wait for nobody, in a launch of their own where they do not fit the last one.
+// None when the cases' levels together have more than kFlowBatchCells cells. The level's jobs, case by case.
 void Batch::flowJobs(int lv, int nSweeps, size_t vb, std::vector<FlowJob>& jobs, std::vector<int>& jobCase) const
 {
     const int K = static_cast<int>(cases.size());
@@ -1239,9 +1242,7 @@ void Batch::flowJobs(int lv, int nSweeps, size_t vb, std::vector<FlowJob>& jobs,
     for (int c = 0; c < K; ++c)
         if (nLevelsOf[c] >= lv + 1) cells += cases[c]->mesh->lev[lv].nCells;
     if (cells > kFlowBatchCells) return;
-    // a CTA per kFlowBatchShare cells, fewer for all when that is more than the SMs
-    double share = kFlowBatchShare;
-    for (bool fits = false; !fits; share *= 1.1)
+    for (int share : kFlowBatchShares)
     {
         int remote = 0, single = 0;
         for (int c = 0; c < K; ++c)
@@ -1250,12 +1251,12 @@ void Batch::flowJobs(int lv, int nSweeps, size_t vb, std::vector<FlowJob>& jobs,
             const int n = cases[c]->mesh->lev[lv].nCells;
             if (n == 0) continue;
             int r = 1;
-            while (2 * r * share <= n && 2 * r <= sms) r *= 2;
+            while (2LL * r * share <= n && 2 * r <= sms) r *= 2;
             ranks[c] = r;
             if (r > 1) remote += r;
             else ++single;
         }
-        fits = remote == 0 || remote + std::min(single, sms / 2) <= sms;
+        if (remote + std::min(single, sms / 2) <= sms) break;
     }
     for (int c = 0; c < K; ++c)
     {
@@ -1333,25 +1334,39 @@ void Batch::preparePipe(int lv, int nSweeps)
     P.nPartsBig = static_cast<int>(big.size());
     if (P.nSmall)
     {
-        std::vector<int2> many, one;
-        for (int i = 0; i < P.nSmall; ++i)
-            for (int r = 0; r < table[i].ranks; ++r) (table[i].ranks > 1 ? many : one).push_back(make_int2(i, r));
-        // (one launch when every CTA fits; the one-CTA cases first else, the largest first)
-        if (!many.empty() && many.size() + one.size() <= static_cast<size_t>(sms))
+        // whole cases into launches of at most the SMs' CTAs, the largest first; the one-CTA cases beside the last
+        std::vector<int> order(P.nSmall);
+        for (int i = 0; i < P.nSmall; ++i) order[i] = i;
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+            return cases[caseOf[x]]->mesh->lev[lv].nCells > cases[caseOf[y]]->mesh->lev[lv].nCells;
+        });
+        std::vector<std::vector<int2>> many;
+        std::vector<int2> one;
+        for (int i : order)
         {
-            many.insert(many.end(), one.begin(), one.end());
+            if (table[i].ranks == 1)
+            {
+                one.push_back(make_int2(i, 0));
+                continue;
+            }
+            size_t at = 0;
+            while (at < many.size() && many[at].size() + table[i].ranks > static_cast<size_t>(sms)) ++at;
+            if (at == many.size()) many.emplace_back();
+            for (int r = 0; r < table[i].ranks; ++r) many[at].push_back(make_int2(i, r));
+        }
+        if (!many.empty() && many.back().size() + one.size() <= static_cast<size_t>(sms))
+        {
+            many.back().insert(many.back().end(), one.begin(), one.end());
             one.clear();
         }
-        std::stable_sort(one.begin(), one.end(), [&](const int2& x, const int2& y) {
-            return cases[caseOf[x.x]]->mesh->lev[lv].nCells > cases[caseOf[y.x]]->mesh->lev[lv].nCells;
-        });
-        for (int i = 0; i < 2; ++i)
-        {
-            const std::vector<int2>& v = i == 0 ? many : one;
-            P.flow[i].n = static_cast<int>(v.size());
-            P.flow[i].remote = i == 0;
-            if (!v.empty()) P.flow[i].blocks.upload(v.data(), v.size(), stream);
-        }
+        auto launch = [&](const std::vector<int2>& v, bool remote) {
+            P.flow.emplace_back();
+            P.flow.back().n = static_cast<int>(v.size());
+            P.flow.back().remote = remote;
+            P.flow.back().blocks.upload(v.data(), v.size(), stream);
+        };
+        for (const auto& v : many) launch(v, true);
+        if (!one.empty()) launch(one, false);
         const auto* bytes = reinterpret_cast<const unsigned char*>(table.data());
         P.hostTable.assign(bytes, bytes + sizeof(k::FlowArgs<T>) * table.size());
         P.table.upload(P.hostTable.data(), P.hostTable.size(), stream);
@@ -1385,12 +1400,18 @@ void Batch::preparePipe(int lv, int nSweeps)
     P.use = !gaveUp && P.msPipe < P.msSweeps;
     if (!P.use)
     {
-        // not kept: their memory goes, schedules and values
-        for (const BatchLevel::Pipe::Held& f : P.flows)
+        // not kept: their memory goes, schedules and values, where no other batch holds them
+        for (BatchLevel::Pipe::Held& f : P.flows)
         {
-            cases[f.first]->data<T>().flows.erase(f.second->id);
-            for (auto& kv : cases[f.first]->mesh->lev[lv].flowBatch)
-                if (kv.second.get() == f.second) kv.second.reset();
+            f.held.reset();
+            auto& have = cases[f.first]->mesh->lev[lv].flowBatch;
+            for (auto it = have.begin(); it != have.end(); ++it)
+                if (it->second.get() == f.second && f.second->held.use_count() == 1)
+                {
+                    cases[f.first]->data<T>().flows.erase(f.second->id);
+                    have.erase(it);
+                    break;
+                }
         }
         P.flows.clear();
         P.nSmall = 0;

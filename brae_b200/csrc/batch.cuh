@@ -114,7 +114,7 @@ struct BatchLevel
         int nSmall = 0;
         DBuf<unsigned char> table;   // k::FlowArgs<T>[nSmall]
         std::vector<unsigned char> hostTable;  // and on the host
-        FlowBlocks flow[2];          // the launches: with more than one rank, and one CTA each
+        std::vector<FlowBlocks> flow;  // the launches
         struct Held
         {
             int first;                    // the case

@@ -1082,6 +1082,15 @@ b2g_status b2g_level_sweep_shape(const b2g_mesh* mesh, int level, int* wholeLeve
     });
 }
 
+b2g_status b2g_mesh_schedule_bytes(const b2g_mesh* mesh, unsigned long long* bytes)
+{
+    return guarded([&] {
+        need(mesh && bytes, "b2g_mesh_schedule_bytes: null argument");
+        const std::shared_lock<std::shared_mutex> use(mesh->m.use);
+        *bytes = b2g::flowBytes(mesh->m);
+    });
+}
+
 b2g_status b2g_level_mc_pipe(const b2g_mesh* mesh, int level, int nSweeps, int symmetric, int* ranks,
                              float* msPipe, float* msColours)
 {

@@ -521,12 +521,6 @@ void flowsForBatch(std::vector<FlowJob>& jobs, cudaStream_t s)
     {
         auto& have = jobs[i].level->flowBatch;
         if (have.count(keyOf(jobs[i]))) continue;
-        // the level's schedules of this call for other CTA counts that no batch holds any more make room
-        for (auto it = have.begin(); it != have.end();)
-        {
-            const bool old = it->first.first == keyOf(jobs[i]).first && it->second && it->second->held.use_count() == 1;
-            it = old ? have.erase(it) : std::next(it);
-        }
         have[keyOf(jobs[i])];  // (a level listed twice is built once)
         missing.push_back(i);
     }

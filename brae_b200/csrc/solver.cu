@@ -1444,7 +1444,7 @@ void Matrix::ensureMulticolour()
 
 // The prolonged and scaled correction of a small level in one launch (scaleProlongCluster): as many CTAs as
 // give each thread one cell, up to a cluster of 16 (8 where that cannot be resident) with two. false when the
-// level is larger, or the sums run in serial order. Measured per V-cycle on a 46 x 23 x 23 box: see there.
+// level is larger, or the sums run in serial order.
 template <class T>
 bool Matrix::scaleProlonged(int level, const T* coarse, T* field, const T* src)
 {

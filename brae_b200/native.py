@@ -78,6 +78,7 @@ def _load():
         "b2g_level_grid_stall": (ip, [vp, ip, vp, vp, ip, ip, C.c_longlong]),
         "b2g_level_smooth_pipelined": (ip, [vp, ip, vp, vp, ip, ip]),
         "b2g_level_smooth_flow": (ip, [vp, ip, vp, vp, ip, ip, ip, ip, C.c_longlong, C.POINTER(C.c_float)]),
+        "b2g_mesh_schedule_bytes": (ip, [vp, C.POINTER(C.c_ulonglong)]),
         "b2g_flow_handovers": (ip, [ip, ip, vp, vp, vp, ip, ip, ip, ip, ip, C.POINTER(C.c_longlong)]),
         "b2g_level_pipe_shape": (ip, [vp, ip, ip, ip, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_float),
                                       C.POINTER(C.c_float), C.POINTER(C.c_float), C.POINTER(C.c_float),
@@ -161,7 +162,7 @@ EXPORTED = [
     "b2g_batch_launches", "b2g_batch_stall", "b2g_batch_destroy", "b2g_mesh_set_pair", "b2g_mesh_level_pair",
     "b2g_gamg_solve_coupled", "b2g_matrix_create_coupled", "b2g_matrix_level_pair_coeffs", "b2g_matrix_gamg_solve",
     "b2g_matrix_set_coeffs", "b2g_matrix_level_timings", "b2g_level_smooth_stall", "b2g_set_sweep_pipeline",
-    "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_flow_handovers", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
+    "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_flow_handovers", "b2g_mesh_schedule_bytes", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
 ]
 
 
@@ -303,6 +304,13 @@ class Mesh(_Owner):
         nc, nf = C.c_int(), C.c_int()
         _check(lib.b2g_mesh_level_size(self.handle, level, C.byref(nc), C.byref(nf)))
         return nc.value, nf.value
+
+    @property
+    def schedule_bytes(self) -> int:
+        """Device bytes of the smoothing schedules, the matrices' values included (b2g_mesh_schedule_bytes)."""
+        v = C.c_ulonglong()
+        _check(lib.b2g_mesh_schedule_bytes(self.handle, C.byref(v)))
+        return v.value
 
     @property
     def build_ms(self) -> float:

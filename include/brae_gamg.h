@@ -410,6 +410,9 @@ B2G_API b2g_status b2g_level_smooth_pipelined(b2g_matrix* m, int level, double* 
  * (psi then holds 5 * nSweeps sweeps). B2G_ERR_ARGUMENT when the level has no such schedule. For tests and tuning. */
 B2G_API b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const double* source, int nSweeps,
                                          int symmetric, int ranks, int weight, long long stallLimit, float* ms);
+/* The device bytes of the mesh's smoothing schedules, its live matrices' values of them included (0 when they have
+ * been dropped). Diagnostic. */
+B2G_API b2g_status b2g_mesh_schedule_bytes(const b2g_mesh* mesh, unsigned long long* bytes);
 /* The hand-overs between CTAs of the data-flow launch that nSweeps sweeps of this addressing take on `ranks` CTAs
  * (host arrays; no device needed): the exact Gauss-Seidel order, or with `colours` (a colour per cell from 0; no
  * two cells of a colour share a face) the multicolour one. counts: values stored for another CTA, values another

@@ -251,3 +251,21 @@ def test_batches_of_other_compositions(b2g):
         kept[0].solve([built[k].source for k in (0, 2, 4, 5)], psis, ctl)
         for k, psi in zip((0, 2, 4, 5), psis):
             assert np.array_equal(psi, want[k][0])
+
+
+def test_schedules_do_not_grow_with_the_compositions(b2g):
+    # cases that pass through batches of every size, as a server's groups do: two CTA counts a level at the most,
+    # whatever the company, so that from the second count on nothing is built any more
+    c = cases.box_case(nx=40, ny=40, nz=40, seed=27)
+    meshes = [b2g.Mesh(c.lower, c.upper, c.Sf, c.magSf, c.n_cells, 10, True) for _ in range(8)]
+    mats = [b2g.Matrix(m, c.diag, c.coef) for m in meshes]
+    ctl = b2g.controls_default(tolerance=1e-6, relTol=0.0)
+    want, grown = None, []
+    for size in (1, 8, 2, 5, 3, 7, 4, 6, 8, 1):
+        psis = [np.zeros(c.n_cells) for _ in range(size)]
+        b2g.Batch(mats[:size]).solve([c.source] * size, psis, ctl)
+        want = psis[0] if want is None else want
+        assert all(np.array_equal(p, want) for p in psis)
+        grown.append(meshes[0].schedule_bytes)
+    assert 0 < grown[0] < grown[1]  # alone on the fine share, among all on the coarse one
+    assert grown[2:] == grown[1:2] * (len(grown) - 2), grown

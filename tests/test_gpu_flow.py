@@ -286,6 +286,7 @@ def solve_batch():
 
 
 want, want_batch = solve(A), solve_batch()
+assert mesh.schedule_bytes > 100 * c.n_cells
 before = mesh.pipe_shape(0, 2, 8)
 assert before["ranks"] > 0 and not before["grid"], before
 # leave a few GB (and the room rule's eighth is gone): the next matrices, without pipelined launches, take it all
@@ -305,6 +306,7 @@ else:
 b.set_sweep_pipeline(True)
 after = mesh.pipe_shape(0, 2, 8)
 assert after["ms_sweep_by_sweep"] == 0.0, after   # the mesh's schedules went before the call failed
+assert mesh.schedule_bytes == 0 and batch_mesh.schedule_bytes == 0
 assert np.array_equal(solve(A), want)
 assert np.array_equal(solve_batch(), want_batch)
 print("SAME", len(kept))
