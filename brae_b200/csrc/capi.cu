@@ -940,6 +940,40 @@ b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const do
     });
 }
 
+b2g_status b2g_level_smooth_flow32(b2g_matrix* m, int level, float* psi, const float* source, int nSweeps, int symmetric,
+                                   int ranks, int weight)
+{
+    return guarded([&] {
+        need(m && psi && source, "b2g_level_smooth_flow32: null argument");
+        need(level >= 0 && level <= m->mat->nLevels(), "b2g_level_smooth_flow32: level out of range");
+        need(nSweeps >= 1, "b2g_level_smooth_flow32: nSweeps must be positive");
+        need(ranks >= 0 && weight >= 1 && weight <= 64, "b2g_level_smooth_flow32: ranks or weight out of range");
+        b2g::Matrix& A = *m->mat;
+        need(!A.coupled, "b2g_level_smooth_flow32: not for a coupled matrix");
+        const std::shared_lock<std::shared_mutex> use(A.mesh->use);
+        A.ensureFp32();
+        b2g::DBuf<float> x, b;
+        for (b2g::DBuf<float>* v : {&x, &b})
+        {
+            v->alloc(A.nAlloc(level), A.stream);
+            v->zero(A.stream);
+        }
+        A.toPos(level, static_cast<const float*>(psi), x.p);
+        A.toPos(level, source, b.p);
+        if (ranks == 0)
+        {
+            if (symmetric) A.symSmooth<float>(level, x.p, b.p, nSweeps);
+            else
+                for (int sw = 0; sw < nSweeps; ++sw)
+                    A.gsLaunch<float>(A.mesh->lev[level], A.v32.coef[level], x.p, b.p, nullptr, false);
+        }
+        else if (!A.flowForced<float>(level, x.p, b.p, nSweeps, symmetric != 0, ranks, weight, nullptr))
+            b2g::fail(B2G_ERR_ARGUMENT, "b2g_level_smooth_flow32: the level does not fit that many CTAs");
+        A.fromPos(level, static_cast<const float*>(x.p), psi);
+        A.checkDeviceError();
+    });
+}
+
 b2g_status b2g_flow_handovers(int nCells, int nFaces, const int32_t* lower, const int32_t* upper, const int32_t* colours,
                               int nSweeps, int symmetric, int ranks, int weight, int valueBytes, long long counts[4])
 {

@@ -2101,6 +2101,9 @@ b2g_perf Matrix::gamg(const b2g_controls& c, b2g_solve_log* log)
 }
 
 template void Matrix::toPos<double>(int, const double*, double*);
+template void Matrix::toPos<float>(int, const float*, float*);
+template void Matrix::fromPos<float>(int, const float*, float*);
+template void Matrix::symSmooth<float>(int, float*, const float*, int);
 template void Matrix::fromPos<double>(int, const double*, double*);
 template void Matrix::amul<double>(int, const double*, double*);
 template void Matrix::amul<float>(int, const float*, float*);

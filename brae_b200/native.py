@@ -78,6 +78,7 @@ def _load():
         "b2g_level_grid_stall": (ip, [vp, ip, vp, vp, ip, ip, C.c_longlong]),
         "b2g_level_smooth_pipelined": (ip, [vp, ip, vp, vp, ip, ip]),
         "b2g_level_smooth_flow": (ip, [vp, ip, vp, vp, ip, ip, ip, ip, C.c_longlong, C.POINTER(C.c_float)]),
+        "b2g_level_smooth_flow32": (ip, [vp, ip, vp, vp, ip, ip, ip, ip]),
         "b2g_mesh_schedule_bytes": (ip, [vp, C.POINTER(C.c_ulonglong)]),
         "b2g_flow_handovers": (ip, [ip, ip, vp, vp, vp, ip, ip, ip, ip, ip, C.POINTER(C.c_longlong)]),
         "b2g_level_pipe_shape": (ip, [vp, ip, ip, ip, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_float),
@@ -162,7 +163,7 @@ EXPORTED = [
     "b2g_batch_launches", "b2g_batch_stall", "b2g_batch_destroy", "b2g_mesh_set_pair", "b2g_mesh_level_pair",
     "b2g_gamg_solve_coupled", "b2g_matrix_create_coupled", "b2g_matrix_level_pair_coeffs", "b2g_matrix_gamg_solve",
     "b2g_matrix_set_coeffs", "b2g_matrix_level_timings", "b2g_level_smooth_stall", "b2g_set_sweep_pipeline",
-    "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_flow_handovers", "b2g_mesh_schedule_bytes", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
+    "b2g_level_smooth_pipelined", "b2g_level_smooth_flow", "b2g_level_smooth_flow32", "b2g_flow_handovers", "b2g_mesh_schedule_bytes", "b2g_level_grid_stall", "b2g_set_part_cells", "b2g_level_pipe_shape", "b2g_coarsest_dense_solve", "b2g_assemble_pressure",
 ]
 
 
@@ -483,6 +484,10 @@ class Matrix(_Owner):
         _check(lib.b2g_level_smooth_flow(self.handle, level, _ptr(psi), _ptr(source), n_sweeps, int(symmetric), ranks, weight,
                                          int(stall_limit), C.byref(ms) if timed else None))
         return ms.value
+
+    def smooth_flow32(self, level, psi, source, n_sweeps, ranks, weight=1, symmetric=False):
+        """smooth_flow on float32 CUDA tensors; ranks 0: the sweeps as launches of their own."""
+        _check(lib.b2g_level_smooth_flow32(self.handle, level, _ptr(psi), _ptr(source), n_sweeps, int(symmetric), ranks, weight))
 
     def grid_stall(self, level, psi, source, n_sweeps, ranks, spin_limit):
         """The grid form with no rank publishing its progress (b2g_level_grid_stall): the status name."""

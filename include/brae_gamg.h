@@ -410,6 +410,10 @@ B2G_API b2g_status b2g_level_smooth_pipelined(b2g_matrix* m, int level, double* 
  * (psi then holds 5 * nSweeps sweeps). B2G_ERR_ARGUMENT when the level has no such schedule. For tests and tuning. */
 B2G_API b2g_status b2g_level_smooth_flow(b2g_matrix* m, int level, double* psi, const double* source, int nSweeps,
                                          int symmetric, int ranks, int weight, long long stallLimit, float* ms);
+/* The same in FP32, as the FP32-preconditioned form sweeps (device pointers to float, natural cell order):
+ * `ranks` CTAs, or with ranks 0 the sweeps as launches of their own. For tests. */
+B2G_API b2g_status b2g_level_smooth_flow32(b2g_matrix* m, int level, float* psi, const float* source, int nSweeps,
+                                           int symmetric, int ranks, int weight);
 /* The device bytes of the mesh's smoothing schedules, its live matrices' values of them included (0 when they have
  * been dropped). Diagnostic. */
 B2G_API b2g_status b2g_mesh_schedule_bytes(const b2g_mesh* mesh, unsigned long long* bytes);
