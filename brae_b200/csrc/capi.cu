@@ -383,8 +383,21 @@ std::unique_ptr<b2g_mesh> createMesh(int nCells, int nFaces, const int32_t* lowe
     need(nFaces == 0 || (lower && upper && Sf && magSf), "b2g_mesh_create: null array");
     need(forwardInOut != nullptr, "b2g_mesh_create: null direction flag");
     need(memspace == B2G_MEM_HOST || memspace == B2G_MEM_DEVICE, "b2g_mesh_create: bad memspace");
+    // (a build that fails leaves the caller's flag as it was: the call may run once more)
+    struct Given
+    {
+        int* p;
+        int value;
+        bool keep = true;
+        ~Given()
+        {
+            if (keep) *p = value;
+        }
+    } given{forwardInOut, *forwardInOut};
     std::unique_ptr<b2g_mesh> h(new b2g_mesh);
     b2g::Mesh& M = h->m;
+    // (another thread's call that runs out of memory looks the registered meshes over: not this one yet)
+    const std::shared_lock<std::shared_mutex> building(M.use);
     M.stream = stream;
     cudaGetDevice(&M.device);
     cudaEvent_t e0, e1;
@@ -435,6 +448,7 @@ std::unique_ptr<b2g_mesh> createMesh(int nCells, int nFaces, const int32_t* lowe
     B2G_CUDA(cudaEventElapsedTime(&M.buildMs, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    given.keep = false;
     return h;
 }
 
