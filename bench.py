@@ -381,7 +381,7 @@ def run_ours(args, world, rank, local):
     gs_bytes = 32 * n + 16 * nf       # one sweep: diag, b, psi read + write; upper; two labels
     amul_bytes = 24 * n + 16 * nf     # diag, x, y; upper; two labels
     gs_gbs = fin["smooth_gbs"]
-    traffic = traffic_per_launch("gsSweep", f"graded_channel_{args.n}")
+    traffic = traffic_per_launch("gsFlow", f"graded_channel_{args.n}")
     all_sweep_gbs = tot["smooth_bytes"] / max(tot["smooth_ms"] * 1e-3, 1e-12) / 1e9
     all_amul_gbs = tot["amul_bytes"] / max(tot["amul_ms"] * 1e-3, 1e-12) / 1e9
 
@@ -484,7 +484,7 @@ def run_ours(args, world, rank, local):
             "fused_amul_all_levels_share": tot["fused_ms"] / ms4[3],
             "levels": levels,
         },
-        "roofline": {"kernel": "gsSweep, finest level (exact Gauss-Seidel; per sweep)", "bound": "hbm",
+        "roofline": {"kernel": "gsFlow, finest level (exact Gauss-Seidel, two sweeps a launch; per sweep)", "bound": "hbm",
                      "achieved": gs_gbs, "peak": peak, "unit": "GB/s", "frac": gs_gbs / peak,
                      "traffic": traffic, "peak_source": peak_kind, "algorithmic_bytes_per_sweep": gs_bytes,
                      "all_levels": {"sweep_gbs": all_sweep_gbs, "sweep_frac": all_sweep_gbs / peak,
