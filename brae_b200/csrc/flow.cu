@@ -201,7 +201,7 @@ bool flowRoom(size_t bytes)
     return freeB + (reserved - used) >= bytes + total / 8;
 }
 
-FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s)
+FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s, bool prepared)
 {
     FlowLevel H;
     H.n = L.nCells;
@@ -213,7 +213,7 @@ FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s)
     get(L.gs.posRow, H.posRow, static_cast<size_t>(H.n) + 1);
     get(L.gs.entColPos, H.col, 2 * static_cast<size_t>(L.nFaces));
     B2G_CUDA(cudaStreamSynchronize(s));
-    H.prepare();
+    if (prepared) H.prepare();
     return H;
 }
 
@@ -331,6 +331,8 @@ void Matrix::forgetFlows()
     sweep(v32.flows);
 }
 
+static int symRanks(int n) { return std::max(1, flowShapes(n).front().ranks / 2); }
+
 // Whether this matrix has the schedule's values, filled here outside a capture; false when there is no memory
 // for them, and the level then runs its other form (tried again with the next solve).
 template <class T>
@@ -432,14 +434,14 @@ bool Matrix::flowForced(int level, T* psiL, const T* src, int nSweeps, bool symm
 }
 
 // The symmetric sweeps' launch of `level`, kept where it beats the sweeps' own launches (null else, or when the
-// level has no such schedule). Those are two walks a sweep and two vector moves; the two walks are timed, both
+// level has no such schedule). Those are two walks a sweep and two vector moves; one walk is timed, for all,
 // by the forward layout (the reversed one has the same depth), so that a level that takes the data flow never
 // needs the reversed one. On half the CTAs of a forward call, where they hold the level: the walks of a
 // symmetric call follow one another, so a step has a share of the items. Measured per call, half against as many
 // (FP64, boxes of 151 k and 1 M cells, their levels): 0.37 and 0.50 ms on 152 k cells, 0.34 and 0.40 on 76 k, 0.84
 // and 0.96 on 512 k, 0.67 and 0.72 on 64 k; 0.16 and 0.12 on 10 k. Outside any capture.
 template <class T>
-void Matrix::ensureSymFlow(int level, int nSweeps)
+void Matrix::ensureSymFlow(int level, int nSweeps, FlowBuild* made)
 {
     LevelAddr& L = mesh->lev[level];
     const int key = nSweeps * 16 + static_cast<int>(sizeof(T));
@@ -455,19 +457,27 @@ void Matrix::ensureSymFlow(int level, int nSweeps)
     x.zero(stream);
     b.zero(stream);
     const long long l0 = launches;
-    const float msSweeps = callTime([&] {
-        for (int w = 0; w < 2 * nSweeps; ++w) gsLaunch<T>(L, data<T>().coef[level], x.p, b.p, nullptr, false);
-    });
-    FlowLevel H = flowDownload(L, stream);
+    const float msSweeps =
+        2 * nSweeps * callTime([&] { gsLaunch<T>(L, data<T>().coef[level], x.p, b.p, nullptr, false); }, 1);
+    FlowLevel H;
     const int forward = flowShapes(L.nCells).front().ranks;
-    for (int ranks : {std::max(1, forward / 2), forward})
+    for (int ranks : {symRanks(L.nCells), forward})
     {
         std::unique_ptr<FlowSchedule> F;
         float ms = 0.f;
         const bool ran = attempt([&] {
             int nSteps = 0;
-            const std::vector<int> steps = flowSteps(H, nSweeps, true, ranks, 4, nSteps);
-            F = buildFlow(H, steps, 2 * nSweeps, nSteps, ranks, sizeof(T), stream);
+            if (made && ranks == made->R)
+            {
+                if (made->ok && flowRoom(made->G.deviceBytes(sizeof(T)))) F = uploadFlow(made->G, made->nSteps, ranks, stream);
+                B2G_CUDA(cudaStreamSynchronize(stream));
+            }
+            else
+            {
+                if (H.n == 0) H = flowDownload(L, stream);
+                const std::vector<int> steps = flowSteps(H, nSweeps, true, ranks, 4, nSteps);
+                F = buildFlow(H, steps, 2 * nSweeps, nSteps, ranks, sizeof(T), stream);
+            }
             if (F) ms = flowTime<T>(level, *F, x.p, b.p);
         });
         if (!F) continue;
@@ -479,6 +489,37 @@ void Matrix::ensureSymFlow(int level, int nSweeps)
     }
     launches = l0;
     B2G_CUDA(cudaStreamSynchronize(stream));
+}
+
+// The symmetric sweeps' launches of {level, sweeps}, the missing schedules built side by side: a level's steps are one
+// serial walk, which the other levels' work then hides.
+template <class T>
+void Matrix::ensureSymFlows(const std::vector<std::pair<int, int>>& wanted)
+{
+    std::vector<std::pair<int, int>> missing;
+    for (const auto& w : wanted)
+        if (!mesh->lev[w.first].flowSym.count(w.second * 16 + static_cast<int>(sizeof(T))) && mesh->lev[w.first].nCells &&
+            std::find(missing.begin(), missing.end(), w) == missing.end())
+            missing.push_back(w);
+    std::vector<FlowBuild> made(missing.size());
+    const bool side = !mesh->flowOff && attempt([&] {
+        if (!flowRoom(0)) throw std::bad_alloc();
+        for (size_t i = 0; i < missing.size(); ++i)
+        {
+            FlowBuild& b = made[i];
+            b.H = flowDownload(mesh->lev[missing[i].first], stream, false);
+            b.S = 2 * missing[i].second;
+            b.symmetric = true;
+            b.R = symRanks(b.H.n);
+            b.vb = sizeof(T);
+        }
+        buildFlowPrograms(made);
+    });
+    for (size_t i = 0; i < missing.size(); ++i)
+    {
+        ensureSymFlow<T>(missing[i].first, missing[i].second, side ? &made[i] : nullptr);
+        made[i] = FlowBuild();
+    }
 }
 
 // nSweeps symmetric sweeps of `level` in one launch; false when they run as launches of their own
@@ -655,8 +696,10 @@ template k::FlowArgs<float> Matrix::flowArgs<float>(int, const FlowSchedule&, fl
 
 template bool Matrix::flowForced<double>(int, double*, const double*, int, bool, int, int, float*);
 template bool Matrix::flowForced<float>(int, float*, const float*, int, bool, int, int, float*);
-template void Matrix::ensureSymFlow<double>(int, int);
-template void Matrix::ensureSymFlow<float>(int, int);
+template void Matrix::ensureSymFlow<double>(int, int, FlowBuild*);
+template void Matrix::ensureSymFlow<float>(int, int, FlowBuild*);
+template void Matrix::ensureSymFlows<double>(const std::vector<std::pair<int, int>>&);
+template void Matrix::ensureSymFlows<float>(const std::vector<std::pair<int, int>>&);
 template bool Matrix::symFlowSweeps<double>(int, double*, const double*, int);
 template bool Matrix::symFlowSweeps<float>(int, float*, const float*, int);
 template void Matrix::refreshSymFlows<double>();

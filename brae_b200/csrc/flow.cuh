@@ -60,7 +60,8 @@ struct FlowProgram
     size_t deviceBytes(size_t vb) const { return blobBytes + vb * nVal; }
 };
 
-FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s);
+// (`prepared` false: H.prepare() is left to the caller)
+FlowLevel flowDownload(const LevelAddr& L, cudaStream_t s, bool prepared = true);
 // (both set the level's order)
 std::vector<int> flowSteps(FlowLevel& H, int nSweeps, bool symmetric, int R, int weight, int& nSteps);
 std::vector<int> colourSteps(FlowLevel& H, const std::vector<int>& colourOf, int nColours, int nSweeps, bool symmetric,
@@ -78,12 +79,13 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
 // The same on the device, or null.
 std::unique_ptr<FlowSchedule> buildFlow(FlowLevel& H, const std::vector<int>& T, int S, int nSteps, int R, size_t vb,
                                         cudaStream_t s);
-// Programs of many levels (forward sweeps) side by side on the host's cores; ok is false where the level has
+// Programs of many levels side by side on the host's cores; ok is false where the level has
 // none. The levels' addressing is freed on the way.
 struct FlowBuild
 {
     FlowLevel H;
-    int S = 0, R = 0, weight = 4;
+    int S = 0, R = 0, weight = 4;  // S: visits of a cell, two a sweep when symmetric
+    bool symmetric = false;
     size_t vb = 0;
     std::vector<int> T;
     int nSteps = 0;
@@ -106,10 +108,10 @@ void flowsForBatch(std::vector<FlowJob>& jobs, cudaStream_t s);
 template <class T>
 void launchFlowBatch(const void* table, const int2* blocks, int nBlocks, bool remote, const int* caseOf, const int* active,
                      cudaStream_t s);
-// Runs body(i, worker) for i in [0, n) on the host's cores, worker < kFlowThreads; the first exception is
+// Runs body(i, worker) for i in [0, n) on the host's cores, `threads` at most, worker < kFlowThreads; the first exception is
 // rethrown. Nested calls run on the calling thread.
 constexpr int kFlowThreads = 16;
-void flowParallel(int n, const std::function<void(int, int)>& body);
+void flowParallel(int n, const std::function<void(int, int)>& body, int threads = kFlowThreads);
 // The launches worth timing on a level of n cells.
 struct FlowShape
 {

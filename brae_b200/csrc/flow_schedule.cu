@@ -358,12 +358,12 @@ void FlowLevel::prepare()
     });
 }
 
-void flowParallel(int n, const std::function<void(int, int)>& body)
+void flowParallel(int n, const std::function<void(int, int)>& body, int threads)
 {
     // a loop within a loop runs on its own thread: the outer one has the cores
     static thread_local bool inside = false;
     const int hw = static_cast<int>(std::max(1u, std::thread::hardware_concurrency()));
-    const int nt = inside ? 1 : std::min(n, std::min(hw, kFlowThreads));
+    const int nt = inside ? 1 : std::min({n, hw, kFlowThreads, threads});
     std::atomic<int> next{0};
     std::vector<std::exception_ptr> bad(std::max(nt, 1));
     auto work = [&](int w) {
@@ -564,9 +564,11 @@ bool buildFlowProgram(FlowLevel& H, const std::vector<int>& T, int S, int nSteps
 {
     if (!startFlowProgram(H, S, R, F)) return false;
     std::vector<RankScratch> scratch(kFlowThreads);
+    // (a thread takes some 30 us to start, an item 0.2 us to place)
+    const int threads = 1 + static_cast<int>(static_cast<long long>(H.n) * S / 8192);
     flowParallel(R, [&](int r, int w) {
         buildRank(H, T, S, nSteps, flowBegin(r, H.n, R), flowBegin(r + 1, H.n, R), vb, scratch[w], F.prog[r]);
-    });
+    }, threads);
     return finishFlowProgram(R, vb, F);
 }
 
@@ -583,7 +585,7 @@ void buildFlowPrograms(std::vector<FlowBuild>& all)
         FlowBuild& b = all[order[i]];
         b.ok = attempt([&] {
             b.H.prepare();
-            b.T = flowSteps(b.H, b.S, false, b.R, b.weight, b.nSteps);
+            b.T = flowSteps(b.H, b.symmetric ? b.S / 2 : b.S, b.symmetric, b.R, b.weight, b.nSteps);
         }) && startFlowProgram(b.H, b.S, b.R, b.G);
     });
     std::vector<std::pair<int, int>> ranks;

@@ -1100,10 +1100,9 @@ void Matrix::prepareSmoother(const b2g_controls& c)
     // the symmetric smoothing calls as one launch each
     if (g_pipeline && sym && (fp64 || c.precision == B2G_PRECISION_FP32_PRECOND))
     {
+        std::vector<std::pair<int, int>> wanted;
         auto want = [&](int level, int nSweeps) {
-            if (nSweeps <= 0 || level > nLevels()) return;
-            if (fp64) ensureSymFlow<double>(level, nSweeps);
-            else ensureSymFlow<float>(level, nSweeps);
+            if (nSweeps > 0 && level <= nLevels()) wanted.push_back({level, nSweeps});
         };
         want(0, c.nFinestSweeps);
         for (int li = 0; li + 1 < nLevels(); ++li)
@@ -1111,6 +1110,8 @@ void Matrix::prepareSmoother(const b2g_controls& c)
             want(li + 1, std::min(c.nPostSweeps + c.postSweepsLevelMultiplier * li, c.maxPostSweeps));
             if (c.nPreSweeps) want(li + 1, std::min(c.nPreSweeps + c.preSweepsLevelMultiplier * li, c.maxPreSweeps));
         }
+        if (fp64) ensureSymFlows<double>(wanted);
+        else ensureSymFlows<float>(wanted);
         if (fp64) refreshSymFlows<double>();
         else refreshSymFlows<float>();
     }

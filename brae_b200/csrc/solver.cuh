@@ -216,15 +216,14 @@ struct Matrix
     template <class T> bool flowForced(int level, T* psi, const T* source, int nSweeps, bool symmetric, int ranks, int weight, float* ms);
     // the mean milliseconds of a few calls, after one that fills what is filled on first use
     template <class Call>
-    float callTime(Call&& call)
+    float callTime(Call&& call, int calls = 3)
     {
-        constexpr int kCalls = 3;
         call();
         cudaEvent_t e0, e1;
         B2G_CUDA(cudaEventCreate(&e0));
         B2G_CUDA(cudaEventCreate(&e1));
         B2G_CUDA(cudaEventRecord(e0, stream));
-        for (int i = 0; i < kCalls; ++i) call();
+        for (int i = 0; i < calls; ++i) call();
         B2G_CUDA(cudaEventRecord(e1, stream));
         B2G_CUDA(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -232,10 +231,11 @@ struct Matrix
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         checkDeviceError();
-        return ms / kCalls;
+        return ms / static_cast<float>(calls);
     }
     template <class T> float flowTime(int level, const FlowSchedule& F, T* psi, const T* source, bool fma = false);
-    template <class T> void ensureSymFlow(int level, int nSweeps);
+    template <class T> void ensureSymFlow(int level, int nSweeps, struct FlowBuild* made = nullptr);
+    template <class T> void ensureSymFlows(const std::vector<std::pair<int, int>>& wanted);
     template <class T> bool symFlowSweeps(int level, T* psi, const T* source, int nSweeps);
     template <class T> void refreshSymFlows();
     // the coarsest level's dense Cholesky factor (FP32-preconditioned forms, coarsestDirect), made for
